@@ -13,6 +13,7 @@ from . import _lib
 # while `python -m graphcuda_b200.build` is (re)building it.
 if "graphcuda_b200.build" not in getattr(_sys, "orig_argv", []):
     _lib.lib()
+    _lib.load_host()
 
 from . import _graphcuda  # noqa: E402
 from ._graphcuda import (gemm_cublas, matmul1, matmul2, matmul3, matmul4,  # noqa: E402

@@ -27,7 +27,7 @@ def gcn_conv_forward(X, adjm, weights, apply_relu):
     > 0) as float32; without ReLU the mask is an uninitialised 0-dim CPU tensor
     (src/graphcuda/cuda/gcn.cu:5-25)."""
     adj = as_adjacency(adjm)
-    Y, mask, _ = layer_forward(X, adj, weights, None, bool(apply_relu), want_mask=bool(apply_relu))
+    Y, mask = layer_forward(X, adj, weights, None, bool(apply_relu), want_mask=bool(apply_relu))
     if not apply_relu:
         mask = torch.empty(())
     return Y, mask

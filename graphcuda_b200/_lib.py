@@ -122,6 +122,29 @@ def lib() -> C.CDLL:
     return handle
 
 
+host = None  # the native host module (csrc/host), set by load_host()
+
+
+def load_host():
+    """Loads lib/_gc_host.so (once) and binds it to the C-ABI library."""
+    global host
+    if host is not None:
+        return host
+    import importlib.machinery
+    import importlib.util
+
+    import torch  # noqa: F401  (its libraries must be in the process first)
+    path = _build.host_path()
+    if not os.path.exists(path):
+        raise LibraryMissing(f"{path} not found: run `python -m graphcuda_b200.build` (needs nvcc and g++).")
+    loader = importlib.machinery.ExtensionFileLoader(_build.HOSTNAME, path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader(_build.HOSTNAME, loader))
+    loader.exec_module(module)
+    module.load_abi(os.environ.get("GRAPHCUDA_B200_LIB", _build.lib_path()))
+    host = module
+    return host
+
+
 def check(status: int, what: str) -> None:
     """Maps a non-zero status to RuntimeError (what TORCH_CHECK raises in the
     reference: src/graphcuda/cuda/gemm_cublas.cu:4-7)."""

@@ -18,91 +18,51 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .ops import _require, _stream, arena, EPI_RELU, EPI_ACCUMULATE
-
-
-class SpmmPlan:
-    """A built processing plan: device buffer and the counts it was built with."""
-
-    __slots__ = ("buf", "n_pieces", "n_slots", "n_cut", "panel_cols")
-
-    def __init__(self, buf, n_pieces, n_slots, n_cut, panel_cols):
-        self.buf, self.n_pieces, self.n_slots, self.n_cut, self.panel_cols = buf, n_pieces, n_slots, n_cut, panel_cols
+from .ops import _require, _stream, arena, EPI_RELU
 
 
 class CSRAdjacency:
-    """int32 CSR on one device, with the SpMM plan and the symmetry verdict."""
+    """int32 CSR on one device, with the SpMM plans and the symmetry verdict (held by the native host side)."""
 
     def __init__(self, rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor, shape, *,
                  symmetric: Optional[bool] = None, build_plan: bool = True):
-        _require(rowptr.is_cuda and col.is_cuda and val.is_cuda, "CSR arrays must be CUDA tensors")
-        _require(rowptr.dtype == torch.int32 and col.dtype == torch.int32, "rowptr/col must be int32")
-        _require(val.dtype == torch.float32, "CSR values must be float32")
-        _require(rowptr.numel() == shape[0] + 1, "rowptr must have M+1 entries")
-        _require(col.numel() == val.numel(), "col and val must have the same length")
-        self.rowptr = rowptr.contiguous()
-        self.col = col.contiguous()
-        self.val = val.contiguous()
         self.shape = (int(shape[0]), int(shape[1]))
-        self.nnz = int(col.numel())
-        self.device = rowptr.device
-        self._symmetric = symmetric
-        self.use_plan = bool(build_plan)
-        self.segment = None  # longest piece in non-zeros; None: gc_spmm_default_segment(nnz)
+        self._h = _lib.host.csr(rowptr, col, val, self.shape[0], self.shape[1],
+                                -1 if symmetric is None else int(bool(symmetric)), bool(build_plan))
+        self.rowptr, self.col, self.val = self._h.rowptr, self._h.col, self._h.val
+        self.nnz = int(self._h.nnz)
+        self.device = self.rowptr.device
         self.perm = None  # set by normalized_adjacency(reorder=...): perm[new] = old vertex id
         self.inv_perm = None
-        self._plans = {}  # panel_cols -> SpmmPlan
+
+    @property
+    def use_plan(self) -> bool:
+        return self._h.use_plan
+
+    @use_plan.setter
+    def use_plan(self, value: bool) -> None:
+        self._h.use_plan = bool(value)
+
+    @property
+    def segment(self) -> Optional[int]:
+        """Longest piece of plans built from now on, in non-zeros; None: gc_spmm_default_segment(nnz)."""
+        return self._h.segment or None
+
+    @segment.setter
+    def segment(self, value: Optional[int]) -> None:
+        self._h.segment = int(value or 0)
 
     def plan_for(self, F: int, panel_cols: Optional[int] = None):
-        """The processing plan for feature width F (built on first use and kept):
-        (plan buffer, n_pieces, n_slots, n_cut)."""
-        L = _lib.lib()
-        M, K = self.shape
-        if panel_cols is None:
-            panel_cols = int(L.gc_spmm_default_panel_cols(K, max(F, 1)))
-        hit = self._plans.get(panel_cols)
-        if hit is not None:
-            return hit
-        seg = int(L.gc_spmm_default_segment(self.nnz)) if self.segment is None else int(self.segment)
-        dev = self.device
-        with torch.cuda.device(dev):
-            s = _stream(dev)
-            counts = torch.zeros(3, dtype=torch.int64, device=dev)
-            wsb = L.gc_spmm_plan_workspace_bytes(M, 0)
-            ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-            _lib.check(L.gc_spmm_plan_count(self.rowptr.data_ptr(), self.col.data_ptr(), M, K, panel_cols, seg,
-                                            counts.data_ptr(), ws.data_ptr(), wsb, s), "gc_spmm_plan_count")
-            n_pieces, n_slots, n_cut = (int(x) for x in counts.tolist())  # the one host read of plan building
-            del ws
-            pbytes = L.gc_spmm_plan_bytes(n_pieces, n_cut)
-            plan = torch.empty(pbytes, dtype=torch.uint8, device=dev)
-            wsb = L.gc_spmm_plan_workspace_bytes(M, n_pieces)
-            ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-            _lib.check(L.gc_spmm_plan_build(self.rowptr.data_ptr(), self.col.data_ptr(), M, K, panel_cols, seg,
-                                            n_pieces, n_slots, n_cut, plan.data_ptr(), pbytes, ws.data_ptr(), wsb,
-                                            s), "gc_spmm_plan_build")
-            torch.cuda.current_stream(dev).synchronize()  # ws is released below
-        entry = SpmmPlan(plan, n_pieces, n_slots, n_cut, panel_cols)
-        self._plans[panel_cols] = entry
-        return entry
+        """The processing plan for feature width F (built on first use and kept): buf, n_pieces, n_slots, n_cut,
+        panel_cols."""
+        return self._h.plan_for(F, int(panel_cols or 0))
 
     @property
     def symmetric(self) -> bool:
         """Whether A == A^T bit for bit (decides if the layer may aggregate on
         the output side; the reference multiplies by A in the backward pass,
         never A^T: src/graphcuda/cuda/gcn.cu:49)."""
-        if self._symmetric is None:
-            if self.shape[0] != self.shape[1]:
-                self._symmetric = False
-            else:
-                out = torch.empty(1, dtype=torch.int32, device=self.device)
-                with torch.cuda.device(self.device):
-                    st = _lib.lib().gc_csr_is_symmetric(self.rowptr.data_ptr(), self.col.data_ptr(),
-                                                        self.val.data_ptr(), self.shape[0], out.data_ptr(),
-                                                        _stream(self.device))
-                _lib.check(st, "gc_csr_is_symmetric")
-                self._symmetric = bool(out.item())
-        return self._symmetric
+        return self._h.is_symmetric()
 
     def plan_counts(self, F: int = 256, panel_cols: Optional[int] = None):
         """(pieces, scratch slots, cut rows) of the plan for width F -- for tests and reports."""
@@ -117,58 +77,7 @@ class CSRAdjacency:
         """Y = A @ H (+bias)(ReLU).  Returns Y or (Y, mask).  gate (contiguous,
         shape of Y): Y is multiplied by (gate > 0) in the store.  H may be a bfloat16 matrix as ops.to_bf16 lays
         it out (the reduced-precision tier: half the gathered bytes, fp32 sums and output)."""
-        _require(H.dim() == 2, "B must be 2D")
-        _require(H.size(0) == self.shape[1], "A.cols must match B.rows")
-        _require(H.is_cuda and H.device == self.device, "A and B must be CUDA tensors on the same device")
-        h16 = H.dtype == torch.bfloat16
-        _require(H.dtype == torch.float32 or h16, "B must be float32 (or bfloat16 for the reduced-precision tier)")
-        if h16:
-            _require(H.stride(1) == 1 and H.size(1) % 8 == 0 and (H.size(0) <= 1 or H.stride(0) % 8 == 0)
-                     and H.data_ptr() % 16 == 0, "a bfloat16 B needs a width and row pitch that are multiples of 8")
-        elif H.stride(1) != 1 or (H.size(0) > 1 and H.stride(0) < H.size(1)):
-            H = H.contiguous()
-        M, K = self.shape
-        F = H.size(1)
-        dev = self.device
-        epi = EPI_RELU if relu else 0
-        if accumulate_into is not None:
-            out = accumulate_into
-            epi |= EPI_ACCUMULATE
-        if out is None:
-            out = torch.empty((M, F), dtype=torch.float32, device=dev)
-        # `out` may be a column slice of a wider row-major matrix (unit column stride)
-        _require(tuple(out.shape) == (M, F) and out.dtype == torch.float32 and out.stride(1) == 1
-                 and (M <= 1 or out.stride(0) >= F), "out has the wrong shape, dtype or layout")
-        ldy = out.stride(0) if M > 1 else max(F, 1)
-        _require(not want_mask or ldy == F, "a mask needs a contiguous output")
-        mask = torch.empty((M, F), dtype=torch.float32, device=dev) if want_mask else None
-        if bias is not None:
-            _require(bias.is_cuda and bias.dtype == torch.float32 and bias.numel() == F, "bias must be float32 [F]")
-            bias = bias.contiguous()
-        if gate is not None:
-            _require(gate.is_cuda and gate.dtype == torch.float32 and tuple(gate.shape) == (M, F)
-                     and gate.is_contiguous() and ldy == F, "gate must be a contiguous float32 tensor of Y's shape")
-        if M == 0 or F == 0:
-            return (out, mask) if want_mask else out
-        L = _lib.lib()
-        with torch.cuda.device(dev):
-            plan = self.plan_for(F, panel_cols) if self.use_plan else None
-            scratch = None
-            if plan is not None and plan.n_cut > 0:
-                scratch = arena.get("spmm", L.gc_spmm_scratch_bytes(plan.n_slots, F), dev)
-            ldh = H.stride(0) if H.size(0) > 1 else max(F, 1)
-            fn = L.gc_spmm_csr_bf16h_f32 if h16 else L.gc_spmm_csr_f32
-            st = fn(self.rowptr.data_ptr(), self.col.data_ptr(), self.val.data_ptr(), M, K, F,
-                                   H.data_ptr(), ldh, bias.data_ptr() if bias is not None else None, epi,
-                                   out.data_ptr(), ldy, mask.data_ptr() if mask is not None else None,
-                                   gate.data_ptr() if gate is not None else None,
-                                   plan.buf.data_ptr() if plan is not None else None,
-                                   plan.n_pieces if plan is not None else 0, plan.n_slots if plan is not None else 0,
-                                   plan.n_cut if plan is not None else 0,
-                                   scratch.data_ptr() if scratch is not None else None,
-                                   scratch.numel() if scratch is not None else 0, _stream(dev))
-        _lib.check(st, "gc_spmm_csr_f32")
-        return (out, mask) if want_mask else out
+        return _lib.host.spmm(self._h, H, bias, relu, want_mask, accumulate_into, out, int(panel_cols or 0), gate)
 
     def matmul_into_blocks(self, H: torch.Tensor, blocks, block_rows: int, *, bias: Optional[torch.Tensor] = None,
                            relu: bool = False, panel_cols: Optional[int] = None) -> None:
@@ -229,44 +138,59 @@ class DenseAdjacency:
     src/graphcuda/cpp/gcn.cpp:10).  Products run on the dense GEMM path."""
 
     def __init__(self, A: torch.Tensor, symmetric: Optional[bool] = None):
-        _require(A.dim() == 2 and A.is_cuda and A.dtype == torch.float32, "dense adjacency must be a float32 CUDA matrix")
+        self._h = _lib.host.dense(A, -1 if symmetric is None else int(bool(symmetric)))
         self.A = A
         self.shape = tuple(A.shape)
         self.device = A.device
-        self._symmetric = symmetric
 
     @property
     def symmetric(self) -> bool:
         """A == A^T bit for bit.  The verdict is remembered on the tensor itself (with the version it was taken
         at), so wrapping the same matrix again -- every layer call does -- does not repeat the comparison."""
-        if self._symmetric is None:
+        h = self._h
+        if h.symmetric < 0:
             memo = getattr(self.A, "_gc_symmetric", None)
             if memo is not None and memo[0] == self.A._version:
-                self._symmetric = memo[1]
+                h.symmetric = int(memo[1])
             else:
-                self._symmetric = self.shape[0] == self.shape[1] and bool(torch.equal(self.A, self.A.t()))
+                verdict = h.is_symmetric()
                 try:
-                    self.A._gc_symmetric = (self.A._version, self._symmetric)
+                    self.A._gc_symmetric = (self.A._version, verdict)
                 except Exception:
                     pass
-        return self._symmetric
+        return bool(h.symmetric)
+
+    def _bf16(self) -> torch.Tensor:
+        """The adjacency does not change between calls: its bf16 copy is made once per version of the tensor and
+        remembered on the tensor itself, like the symmetry verdict, so that it lives exactly as long as A."""
+        memo = getattr(self.A, "_gc_bf16", None)
+        if memo is None or memo[0] != self.A._version:
+            memo = (self.A._version, _lib.host.to_bf16(self.A, False))
+            try:
+                self.A._gc_bf16 = memo
+            except Exception:
+                pass
+        return memo[1]
 
     def matmul(self, H: torch.Tensor, *, bias=None, relu=False, want_mask=False, accumulate_into=None, out=None,
                precision=None, gate=None):
         from .ops import gemm, gemm_bf16_operands, get_default_precision, to_bf16
         _require(accumulate_into is None, "accumulate is not available on the dense path")
         if (precision or get_default_precision()) == "bf16" and not want_mask:
-            # the adjacency does not change between calls: its bf16 copy is made once (per version of the tensor)
-            # (remembered on the tensor itself, like the symmetry verdict, so that it lives exactly as long as A)
-            memo = getattr(self.A, "_gc_bf16", None)
-            if memo is None or memo[0] != self.A._version:
-                memo = (self.A._version, to_bf16(self.A))
-                try:
-                    self.A._gc_bf16 = memo
-                except Exception:
-                    pass
-            return gemm_bf16_operands(memo[1], to_bf16(H, transpose=True), bias=bias, relu=relu, out=out, gate=gate)
+            return gemm_bf16_operands(self._bf16(), to_bf16(H, transpose=True), bias=bias, relu=relu, out=out, gate=gate)
         return gemm(self.A, H, bias=bias, relu=relu, want_mask=want_mask, precision=precision, out=out, gate=gate)
+
+
+def native_handle(adj, prec: int, *, needs_symmetry: bool):
+    """The native object behind an adjacency, with what the layer will ask of it already settled: the symmetry verdict
+    and, in the bf16 tier, the converted copy of a dense matrix are remembered on the Python side."""
+    h = adj._h
+    if isinstance(adj, DenseAdjacency):
+        if needs_symmetry:
+            adj.symmetric
+        if prec == _lib.PREC_BF16:
+            h.A16 = adj._bf16()
+    return h
 
 
 # ---------------------------------------------------------------- conversion

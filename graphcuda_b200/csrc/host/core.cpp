@@ -1,0 +1,228 @@
+// Library binding, scratch buffers and the single products (see host.h).
+#include "host.h"
+
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <dlfcn.h>
+
+#include <unordered_map>
+
+namespace gch {
+
+void raise(const std::string& msg) { throw std::runtime_error(msg); }
+
+Abi abi;
+
+void load_abi(const std::string& path) {
+  void* h = dlopen(path.c_str(), RTLD_NOW | RTLD_LOCAL);
+  if (!h) raise(std::string("cannot load ") + path + ": " + dlerror());
+#define X(name)                                                                   \
+  abi.name = reinterpret_cast<decltype(abi.name)>(dlsym(h, #name));               \
+  if (!abi.name) raise(std::string(#name) + " is missing from " + path);
+  GC_HOST_FUNCTIONS(X)
+#undef X
+}
+
+void check(int status, const char* what) {
+  if (__builtin_expect(status == 0, 1)) return;
+  std::string msg = abi.gc_last_error();
+  if (msg.empty()) msg = abi.gc_status_string(status);
+  raise(std::string(what) + ": " + msg + " (status " + std::to_string(status) + ")");
+}
+
+// ------------------------------------------------------------------ scratch
+namespace {
+struct Key {
+  int device;
+  void* stream;
+  bool operator==(const Key& o) const { return device == o.device && stream == o.stream; }
+};
+struct KeyHash {
+  size_t operator()(const Key& k) const { return std::hash<void*>()(k.stream) * 31 + size_t(k.device); }
+};
+struct Buffers {
+  Tensor buf[kTags];
+};
+std::mutex scratch_mutex;
+// Never destroyed: the tensors must not outlive torch's allocator at process exit.
+std::unordered_map<Key, Buffers, KeyHash>& buffers() {
+  static auto* m = new std::unordered_map<Key, Buffers, KeyHash>();
+  return *m;
+}
+Tensor bytes_on(size_t n, const at::Device& dev) {
+  return at::empty({int64_t(n)}, at::TensorOptions().dtype(at::kByte).device(dev));
+}
+}  // namespace
+
+Tensor scratch_buffer(Tag tag, size_t bytes, const at::Device& dev) {
+  const auto stream = at::cuda::getCurrentCUDAStream(dev.index());
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+    return bytes_on(std::max<size_t>(256, bytes), dev);
+  std::lock_guard<std::mutex> lock(scratch_mutex);
+  Tensor& b = buffers()[Key{dev.index(), stream.stream()}].buf[tag];
+  if (!b.defined() || size_t(b.numel()) < bytes) {
+    const size_t size = std::max<size_t>(256, (bytes + bytes / 4 + 255) & ~size_t(255));  // growth is rare
+    Tensor n = bytes_on(size, dev).zero_();
+    if (b.defined()) n.narrow(0, 0, 256).copy_(b.narrow(0, 0, 256));
+    b = n;
+  }
+  return b;
+}
+
+Scratch scratch(Tag tag, size_t bytes, const at::Device& dev) {
+  Tensor t = scratch_buffer(tag, bytes, dev);
+  return Scratch{t.data_ptr(), size_t(t.numel()), t};
+}
+
+void scratch_clear() {
+  std::lock_guard<std::mutex> lock(scratch_mutex);
+  buffers().clear();
+}
+
+// ------------------------------------------------------------------ layouts
+Tensor empty_f32(int64_t rows, int64_t cols, const at::Device& dev) {
+  return at::empty({rows, cols}, at::TensorOptions().dtype(at::kFloat).device(dev));
+}
+
+Tensor row_major(const Tensor& t) {
+  if (t.stride(1) == 1 && t.stride(0) >= std::max<int64_t>(1, t.size(1))) return t;
+  if (t.size(1) == 1 && t.stride(0) >= 1) return t;
+  return t.contiguous();
+}
+
+Mat as_operand(Tensor& t) {
+  if (t.stride(1) == 1 && (t.size(0) <= 1 || t.stride(0) >= t.size(1)))
+    return Mat{t.const_data_ptr<float>(), t.size(0), t.size(1), ld_of(t), 0};
+  if (t.stride(0) == 1 && (t.size(1) <= 1 || t.stride(1) >= t.size(0))) {
+    const int64_t ld = t.size(1) > 1 ? t.stride(1) : std::max<int64_t>({t.size(0), t.stride(1), 1});
+    return Mat{t.const_data_ptr<float>(), t.size(0), t.size(1), ld, 1};
+  }
+  t = t.contiguous();
+  return Mat{t.const_data_ptr<float>(), t.size(0), t.size(1), ld_of(t), 0};
+}
+
+// ------------------------------------------------------------------ products
+void gemm_into(const Mat& A, const Mat& B, float* C, int64_t ldc, const Epi& ep, bool transposed_out, int prec,
+               const at::Device& dev) {
+  const int64_t M = A.rows, K = A.cols, N = B.cols;
+  if (M == 0 || N == 0) return;
+  const size_t need = abi.gc_gemm_workspace_bytes(A.trans, B.trans, M, N, K, prec);
+  const Scratch ws = scratch(kGemm, need, dev);
+  const int epi = (ep.relu ? GC_EPI_RELU : 0) | (transposed_out ? GC_EPI_TRANSPOSED_OUT : 0);
+  check(abi.gc_gemm_f32(A.trans, B.trans, M, N, K, A.p, A.ld, B.p, B.ld, C, ldc, ep.bias, epi, ep.mask, ep.gate, prec,
+                        ws.ptr, ws.bytes, stream_of(dev)),
+        "gc_gemm_f32");
+}
+
+Tensor to_bf16(const Tensor& Xin, bool transpose) {
+  require(Xin.dim() == 2 && Xin.is_cuda() && Xin.scalar_type() == at::kFloat, "to_bf16: float32 CUDA matrix expected");
+  const Tensor X = row_major(Xin);
+  const int64_t rows = transpose ? X.size(1) : X.size(0), cols = transpose ? X.size(0) : X.size(1);
+  const int64_t ld = (cols + 7) / 8 * 8;
+  const c10::cuda::CUDAGuard guard(X.device());
+  Tensor out = at::empty({rows, ld}, at::TensorOptions().dtype(at::kBFloat16).device(X.device()));
+  check(abi.gc_convert_f32_bf16(X.const_data_ptr<float>(), ld_of(X), rows, cols,
+                                static_cast<uint16_t*>(out.data_ptr()), ld, transpose ? 1 : 0, stream_of(X.device())),
+        "gc_convert_f32_bf16");
+  return ld == cols ? out : out.narrow(1, 0, cols);
+}
+
+void gemm_bf16_into(const Tensor& A16, const Tensor& Bt16, float* C, int64_t ldc, const Epi& ep,
+                    const at::Device& dev) {
+  const int64_t M = A16.size(0), K = A16.size(1), N = Bt16.size(0);
+  if (M == 0 || N == 0) return;
+  const Scratch ws = scratch(kGemm, abi.gc_gemm_bf16_workspace_bytes(M, N, K), dev);
+  const int64_t k8 = (K + 7) / 8 * 8;
+  check(abi.gc_gemm_bf16_f32(M, N, K, static_cast<const uint16_t*>(A16.data_ptr()), M > 1 ? A16.stride(0) : k8,
+                             static_cast<const uint16_t*>(Bt16.data_ptr()), N > 1 ? Bt16.stride(0) : k8, C, ldc,
+                             ep.bias, ep.relu ? GC_EPI_RELU : 0, ep.mask, ep.gate, ws.ptr, ws.bytes, stream_of(dev)),
+        "gc_gemm_bf16_f32");
+}
+
+// ------------------------------------------------------------------ CSR
+std::shared_ptr<Plan> Adj::plan_for(int64_t F, int64_t panel_cols) {
+  std::lock_guard<std::mutex> lock(mutex_);
+  const bool standard = panel_cols <= 0;
+  if (standard) {
+    auto it = by_width_.find(F);
+    if (it != by_width_.end()) return it->second;
+    panel_cols = abi.gc_spmm_default_panel_cols(K, std::max<int64_t>(F, 1));
+  }
+  auto hit = plans_.find(panel_cols);
+  std::shared_ptr<Plan> p = hit != plans_.end() ? hit->second : nullptr;
+  if (!p) {
+    const at::Device dev = device();
+    const c10::cuda::CUDAGuard guard(dev);
+    void* st = stream_of(dev);
+    const int64_t seg = segment > 0 ? segment : abi.gc_spmm_default_segment(nnz);
+    const int32_t* rp = rowptr.const_data_ptr<int32_t>();
+    const int32_t* cp = col.const_data_ptr<int32_t>();
+    Tensor counts = at::empty({3}, at::TensorOptions().dtype(at::kLong).device(dev));
+    size_t wsb = abi.gc_spmm_plan_workspace_bytes(M, 0);
+    Tensor ws = bytes_on(wsb, dev);
+    check(abi.gc_spmm_plan_count(rp, cp, M, K, panel_cols, seg, counts.data_ptr<int64_t>(), ws.data_ptr(), wsb, st),
+          "gc_spmm_plan_count");
+    const Tensor host = counts.cpu();  // the one host read of plan building
+    const int64_t* c = host.const_data_ptr<int64_t>();
+    p = std::make_shared<Plan>();
+    p->n_pieces = c[0];
+    p->n_slots = c[1];
+    p->n_cut = c[2];
+    p->panel_cols = panel_cols;
+    const size_t pb = abi.gc_spmm_plan_bytes(p->n_pieces, p->n_cut);
+    p->buf = bytes_on(pb, dev);
+    wsb = abi.gc_spmm_plan_workspace_bytes(M, p->n_pieces);
+    ws = bytes_on(wsb, dev);
+    check(abi.gc_spmm_plan_build(rp, cp, M, K, panel_cols, seg, p->n_pieces, p->n_slots, p->n_cut, p->buf.data_ptr(),
+                                 pb, ws.data_ptr(), wsb, st),
+          "gc_spmm_plan_build");
+    // other streams may use the plan next
+    C10_CUDA_CHECK(cudaStreamSynchronize(static_cast<cudaStream_t>(st)));
+    plans_[panel_cols] = p;
+  }
+  if (standard) by_width_[F] = p;
+  return p;
+}
+
+bool Adj::is_symmetric() {
+  if (symmetric < 0) {
+    if (M != K) {
+      symmetric = 0;
+    } else if (dense) {
+      symmetric = A.equal(A.t()) ? 1 : 0;
+    } else {
+      const c10::cuda::CUDAGuard guard(device());
+      Tensor out = at::empty({1}, at::TensorOptions().dtype(at::kInt).device(device()));
+      check(abi.gc_csr_is_symmetric(rowptr.const_data_ptr<int32_t>(), col.const_data_ptr<int32_t>(),
+                                    val.const_data_ptr<float>(), M, out.data_ptr<int32_t>(), stream_of(device())),
+            "gc_csr_is_symmetric");
+      symmetric = out.item<int32_t>() ? 1 : 0;
+    }
+  }
+  return symmetric != 0;
+}
+
+void spmm_into(Adj& a, const void* H, int64_t ldh, bool h16, int64_t F, float* Y, int64_t ldy, const Epi& ep,
+               bool accumulate, int64_t panel_cols) {
+  const at::Device dev = a.device();
+  std::shared_ptr<Plan> plan = a.use_plan ? a.plan_for(F, panel_cols) : nullptr;
+  Scratch s{nullptr, 0, Tensor()};
+  if (plan && plan->n_cut > 0) s = scratch(kSpmm, abi.gc_spmm_scratch_bytes(plan->n_slots, F), dev);
+  const int epi = (ep.relu ? GC_EPI_RELU : 0) | (accumulate ? GC_EPI_ACCUMULATE : 0);
+  const int32_t* rp = a.rowptr.const_data_ptr<int32_t>();
+  const int32_t* cp = a.col.const_data_ptr<int32_t>();
+  const float* vp = a.val.const_data_ptr<float>();
+  const void* pb = plan ? plan->buf.data_ptr() : nullptr;
+  const int64_t np = plan ? plan->n_pieces : 0, ns = plan ? plan->n_slots : 0, nc = plan ? plan->n_cut : 0;
+  void* st = stream_of(dev);
+  if (h16)
+    check(abi.gc_spmm_csr_bf16h_f32(rp, cp, vp, a.M, a.K, F, static_cast<const uint16_t*>(H), ldh, ep.bias, epi, Y,
+                                    ldy, ep.mask, ep.gate, pb, np, ns, nc, s.ptr, s.bytes, st),
+          "gc_spmm_csr_f32");
+  else
+    check(abi.gc_spmm_csr_f32(rp, cp, vp, a.M, a.K, F, static_cast<const float*>(H), ldh, ep.bias, epi, Y, ldy,
+                              ep.mask, ep.gate, pb, np, ns, nc, s.ptr, s.bytes, st),
+          "gc_spmm_csr_f32");
+}
+
+}  // namespace gch

@@ -17,51 +17,25 @@ import torch
 import torch.nn as nn
 from torch.nn.parameter import Parameter
 
-from .adjacency import as_adjacency
-from .engine import layer_backward, layer_forward
+from . import _lib
+from .adjacency import as_adjacency, native_handle
+from .ops import _prec
 
 
-class GCNConvFunction(torch.autograd.Function):
-    """Y = relu((adjm @ X) @ weights [+ bias]).
+class GCNConvFunction:
+    """Y = relu((adjm @ X) @ weights [+ bias]) as one autograd node (csrc/host/layer.cpp).
 
     Unlike the reference (python/gcn.py:18) the fp32 mask is not materialised:
     the activation itself is saved and the mask re-derived as Y > 0; the
     aggregated features are saved instead of being recomputed (gcn.cu:40)."""
 
     @staticmethod
-    def forward(ctx, X, adjm, weights, apply_relu, bias=None, precision=None, fuse=0):
+    def apply(X, adjm, weights, apply_relu, bias=None, precision=None, fuse=0):
         # fuse: bit 0 = the incoming gradient is already multiplied by this layer's ReLU mask;
         #       bit 1 = X is the ReLU output of the layer below: gate dX by (X > 0) where it is produced
-        adj = as_adjacency(adjm)
-        Y, _, saved = layer_forward(X, adj, weights, bias, bool(apply_relu), precision=precision)
-        order, inter = saved
-        ctx.adj = adj
-        ctx.order = order
-        ctx.apply_relu = bool(apply_relu)
-        ctx.precision = precision
-        ctx.has_bias = bias is not None
-        ctx.has_inter = inter is not None
-        ctx.fuse = int(fuse)
-        tensors = [X, weights, Y]
-        if inter is not None:
-            tensors.append(inter)
-        ctx.save_for_backward(*tensors)
-        return Y
-
-    @staticmethod
-    def backward(ctx, grad_Y):
-        saved = ctx.saved_tensors
-        X, weights, Y = saved[:3]
-        inter = saved[3] if ctx.has_inter else None
-        need_dX, _, need_dW = ctx.needs_input_grad[:3]
-        need_db = ctx.has_bias and ctx.needs_input_grad[4]
-        if grad_Y.stride(-1) != 1:  # rows may keep a larger pitch (a padded gradient from the fused loss)
-            grad_Y = grad_Y.contiguous()
-        dX, dW, db = layer_backward(grad_Y, X, ctx.adj, weights, ctx.apply_relu, Y,
-                                    (ctx.order, inter), need_dX=need_dX, need_dW=need_dW, need_db=need_db,
-                                    precision=ctx.precision, grad_is_gated=bool(ctx.fuse & 1),
-                                    gate_dx_by_input=bool(ctx.fuse & 2))
-        return dX, None, dW, None, db, None, None
+        prec = _prec(precision)
+        h = native_handle(as_adjacency(adjm), prec, needs_symmetry=weights.size(1) < weights.size(0))
+        return _lib.host.conv(X, h, weights, bias, bool(apply_relu), prec, int(fuse))
 
 
 class GCNConv(nn.Module):

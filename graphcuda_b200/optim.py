@@ -11,33 +11,11 @@ issued -- or recorded -- so change it between captures, not between replays.
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
 from . import _lib
-from .ops import _stream
 
 _MAX = 32  # tensors per launch (kMaxTensors in csrc/optim.cu)
-
-
-def _ptr_array(tensors):
-    return (C.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
-
-
-def _check_param(p: torch.Tensor) -> None:
-    if not (p.is_cuda and p.dtype == torch.float32 and p.is_contiguous()):
-        raise RuntimeError("fused optimizers need contiguous float32 CUDA parameters")
-
-
-def _grads_of(params):
-    out = []
-    for p in params:
-        g = p.grad
-        if g.is_sparse or g.dtype != torch.float32 or g.device != p.device:
-            raise RuntimeError("fused optimizers need dense float32 gradients on the parameter's device")
-        out.append(g if g.is_contiguous() else g.contiguous())
-    return out
 
 
 class FusedAdam(torch.optim.Optimizer):
@@ -59,13 +37,11 @@ class FusedAdam(torch.optim.Optimizer):
         if closure is not None:
             with torch.enable_grad():
                 loss = closure()
-        L = _lib.lib()
         for group in self.param_groups:
             by_device = {}
             for p in group["params"]:
                 if p.grad is None:
                     continue
-                _check_param(p)
                 st = self.state[p]
                 if not st:
                     st["exp_avg"] = torch.zeros_like(p, memory_format=torch.contiguous_format)
@@ -75,16 +51,11 @@ class FusedAdam(torch.optim.Optimizer):
                 # one launch per 32 tensors; every launch keeps its own step count
                 for chunk, i in enumerate(range(0, len(all_ps), _MAX)):
                     ps = all_ps[i:i + _MAX]
-                    grads = _grads_of(ps)
-                    ms = [self.state[p]["exp_avg"] for p in ps]
-                    vs = [self.state[p]["exp_avg_sq"] for p in ps]
-                    sizes = (C.c_int64 * len(ps))(*[p.numel() for p in ps])
-                    with torch.cuda.device(dev):
-                        rc = L.gc_adam_step_f32(len(ps), _ptr_array(ps), _ptr_array(grads), _ptr_array(ms),
-                                                _ptr_array(vs), sizes, group["lr"], group["betas"][0],
-                                                group["betas"][1], group["eps"], group["weight_decay"],
-                                                self._group_state(group, dev, chunk).data_ptr(), _stream(dev))
-                    _lib.check(rc, "gc_adam_step_f32")
+                    st = [self.state[p] for p in ps]
+                    _lib.host.adam_step(ps, [p.grad for p in ps], [x["exp_avg"] for x in st],
+                                        [x["exp_avg_sq"] for x in st], group["lr"], group["betas"][0],
+                                        group["betas"][1], group["eps"], group["weight_decay"],
+                                        self._group_state(group, dev, chunk))
         return loss
 
     def steps_taken(self) -> int:
@@ -108,20 +79,13 @@ class FusedSGD(torch.optim.Optimizer):
         if closure is not None:
             with torch.enable_grad():
                 loss = closure()
-        L = _lib.lib()
         for group in self.param_groups:
             by_device = {}
             for p in group["params"]:
                 if p.grad is not None:
-                    _check_param(p)
                     by_device.setdefault(p.device, []).append(p)
-            for dev, ps in by_device.items():
+            for ps in by_device.values():
                 for i in range(0, len(ps), _MAX):
                     chunk = ps[i:i + _MAX]
-                    grads = _grads_of(chunk)
-                    sizes = (C.c_int64 * len(chunk))(*[p.numel() for p in chunk])
-                    with torch.cuda.device(dev):
-                        rc = L.gc_sgd_step_f32(len(chunk), _ptr_array(chunk), _ptr_array(grads), sizes, group["lr"],
-                                               group["weight_decay"], _stream(dev))
-                    _lib.check(rc, "gc_sgd_step_f32")
+                    _lib.host.sgd_step(chunk, [p.grad for p in chunk], group["lr"], group["weight_decay"])
         return loss
