@@ -32,6 +32,7 @@ SOURCES = [
     "gather_probe.cu",
     "gemm.cu",
     "gemm_simt.cu",
+    "gemm_narrow.cu",
     "gemm_tcgen05.cu",
     "elementwise.cu",
     "gcn_layer.cu",

@@ -50,7 +50,7 @@ int gc_gemm_resolve_precision(int transA, int transB, int64_t M, int64_t N, int6
 size_t gc_gemm_workspace_bytes(int transA, int transB, int64_t M, int64_t N, int64_t K, int precision) {
   if (M <= 0 || N <= 0 || K < 0) return 256;
   // AUTO may resolve either way depending on leading dimensions: report the larger.
-  size_t simt = gc::simt_workspace_bytes(M, N, K);
+  size_t simt = gc::simt_workspace_bytes(transA != 0, M, N, K);
   size_t tc3 = gc::tc_workspace_bytes(transA != 0, transB != 0, M, N, K, 3);
   size_t tc1 = gc::tc_workspace_bytes(transA != 0, transB != 0, M, N, K, 1);
   switch (precision) {

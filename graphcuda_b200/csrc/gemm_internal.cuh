@@ -28,12 +28,19 @@ __device__ __forceinline__ void epilogue_store(float v, int m, int n, float* C, 
   C[off] = v;
 }
 
-// CUDA-core path (gemm_simt.cu)
-int simt_splits(int64_t M, int64_t N, int64_t K);
-size_t simt_workspace_bytes(int64_t M, int64_t N, int64_t K);
+// CUDA-core path (gemm_simt.cu; gemm_narrow.cu for up to 16 columns)
+bool narrow_supported(bool ta, int64_t M, int64_t N, int64_t K);
+size_t narrow_partial_bytes(bool ta, int64_t M, int64_t N, int64_t K);
+int gemm_narrow(bool ta, bool tb, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B,
+                int64_t ldb, float* C, int64_t ldc, const GemmEpilogue& ep, float* partial, cudaStream_t st);
+size_t simt_workspace_bytes(bool ta, int64_t M, int64_t N, int64_t K);
 int gemm_simt(bool ta, bool tb, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B,
               int64_t ldb, float* C, int64_t ldc, const GemmEpilogue& ep, void* workspace, size_t workspace_bytes,
               cudaStream_t st);
+
+// C = sum of the partial tiles [splits][M][N] in a fixed order, then the epilogue (gemm_tcgen05.cu)
+int splitk_reduce(int M, int N, int splits, const float* partial, float* C, int64_t ldc, const GemmEpilogue& ep,
+                  cudaStream_t st);
 
 // Tensor-core path (gemm_tcgen05.cu)
 bool tc_supported(bool ta, bool tb, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc);

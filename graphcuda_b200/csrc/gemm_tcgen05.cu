@@ -568,7 +568,7 @@ transpose_kernel(const float* __restrict__ in, int64_t ldin, float* __restrict__
 // the result is the same run to run; the groups run side by side because a capped-chain product has a thousand
 // partial tiles and one thread per element walking them all was latency-bound (0.22 ms for a 100 x 256 result).
 __global__ void __launch_bounds__(256)
-tc_splitk_reduce_kernel(int M, int N, int splits, const float* __restrict__ partial, float* __restrict__ C,
+splitk_reduce_kernel(int M, int N, int splits, const float* __restrict__ partial, float* __restrict__ C,
                         int64_t ldc, gc::GemmEpilogue ep) {
   __shared__ float sm[8][32];
   const int e = threadIdx.x % 32, g = threadIdx.x / 32;
@@ -811,6 +811,13 @@ int launch_layout(const Plan& pl, const CUtensorMap& mA, const CUtensorMap& mB, 
 
 namespace gc {
 
+int splitk_reduce(int M, int N, int splits, const float* partial, float* C, int64_t ldc, const GemmEpilogue& ep,
+                  cudaStream_t st) {
+  const unsigned g = unsigned(std::min<int64_t>(ceil_div(int64_t(M) * N, 32), kNumSMs * 8));
+  splitk_reduce_kernel<<<g, 256, 0, st>>>(M, N, splits, partial, C, ldc, ep);
+  return check_launch("split-K reduce");
+}
+
 bool tc_supported(bool ta, bool tb, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc) {
   (void)ldc;
   if (M <= 0 || N <= 0 || K <= 0) return false;
@@ -923,10 +930,7 @@ int gemm_tc(bool ta, bool tb, int64_t M, int64_t N, int64_t K, const float* A, i
   }
   if (rc != GC_OK) return rc;
   if (pl.splits > 1) {
-    const int64_t total = M * N;
-    const unsigned g = unsigned(std::min<int64_t>(ceil_div(total, 32), kNumSMs * 8));
-    tc_splitk_reduce_kernel<<<g, 256, 0, st>>>(int(M), int(N), pl.splits, partial, C, ldc, ep);
-    rc = check_launch("gemm_tc split-K reduce");
+    rc = splitk_reduce(int(M), int(N), pl.splits, partial, C, ldc, ep, st);
   }
   return rc;
 }
@@ -1001,10 +1005,7 @@ int gemm_bf16_core(int64_t M, int64_t N, int64_t K, const uint16_t* A, int64_t l
   else rc = run(gemm_tf32_kernel<256, 1, false, false, false, true>, Cfg<256, 1>::kSmemBytes, 256);
   if (rc != GC_OK) return rc;
   if (p.splits > 1) {
-    const int64_t total = M * N;
-    const unsigned g = unsigned(std::min<int64_t>(ceil_div(total, 32), kNumSMs * 8));
-    tc_splitk_reduce_kernel<<<g, 256, 0, st>>>(int(M), int(N), p.splits, p.partial, C, ldc, ep);
-    rc = check_launch("bf16 GEMM split-K reduce");
+    rc = splitk_reduce(int(M), int(N), p.splits, p.partial, C, ldc, ep, st);
   }
   return rc;
 }
