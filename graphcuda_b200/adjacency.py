@@ -45,7 +45,7 @@ class CSRAdjacency:
 
     @property
     def segment(self) -> Optional[int]:
-        """Longest piece of plans built from now on, in non-zeros; None: gc_spmm_default_segment(nnz)."""
+        """Longest piece of plans built from now on, in non-zeros; None: gc_spmm_segment(nnz, F)."""
         return self._h.segment or None
 
     @segment.setter

@@ -148,13 +148,14 @@ std::shared_ptr<Plan> Adj::plan_for(int64_t F, int64_t panel_cols) {
     if (it != by_width_.end()) return it->second;
     panel_cols = abi.gc_spmm_default_panel_cols(K, std::max<int64_t>(F, 1));
   }
-  auto hit = plans_.find(panel_cols);
+  const int64_t seg = segment > 0 ? segment : abi.gc_spmm_segment(nnz, F);
+  const auto key = std::make_pair(panel_cols, seg);
+  auto hit = plans_.find(key);
   std::shared_ptr<Plan> p = hit != plans_.end() ? hit->second : nullptr;
   if (!p) {
     const at::Device dev = device();
     const c10::cuda::CUDAGuard guard(dev);
     void* st = stream_of(dev);
-    const int64_t seg = segment > 0 ? segment : abi.gc_spmm_default_segment(nnz);
     const int32_t* rp = rowptr.const_data_ptr<int32_t>();
     const int32_t* cp = col.const_data_ptr<int32_t>();
     Tensor counts = at::empty({3}, at::TensorOptions().dtype(at::kLong).device(dev));
@@ -178,7 +179,7 @@ std::shared_ptr<Plan> Adj::plan_for(int64_t F, int64_t panel_cols) {
           "gc_spmm_plan_build");
     // other streams may use the plan next
     C10_CUDA_CHECK(cudaStreamSynchronize(static_cast<cudaStream_t>(st)));
-    plans_[panel_cols] = p;
+    plans_[key] = p;
   }
   if (standard) by_width_[F] = p;
   return p;

@@ -32,7 +32,7 @@ inline void require(bool cond, const char* msg) {
 
 // ------------------------------------------------------------------ C ABI
 #define GC_HOST_FUNCTIONS(X)                                                                                        \
-  X(gc_last_error) X(gc_status_string) X(gc_spmm_default_panel_cols) X(gc_spmm_default_segment)                     \
+  X(gc_last_error) X(gc_status_string) X(gc_spmm_default_panel_cols) X(gc_spmm_segment)                     \
   X(gc_spmm_plan_workspace_bytes) X(gc_spmm_plan_count) X(gc_spmm_plan_bytes) X(gc_spmm_plan_build)                 \
   X(gc_spmm_scratch_bytes) X(gc_spmm_csr_f32) X(gc_spmm_csr_bf16h_f32) X(gc_gemm_workspace_bytes) X(gc_gemm_f32)    \
   X(gc_convert_f32_bf16) X(gc_gemm_bf16_workspace_bytes) X(gc_gemm_bf16_f32) X(gc_relu_backward_f32)                \
@@ -116,7 +116,7 @@ struct Adj : torch::CustomClassHolder {
 
  private:
   std::mutex mutex_;
-  std::map<int64_t, std::shared_ptr<Plan>> plans_;    // by panel width
+  std::map<std::pair<int64_t, int64_t>, std::shared_ptr<Plan>> plans_;  // by panel width and segment
   std::map<int64_t, std::shared_ptr<Plan>> by_width_;  // by F, default panel width
 };
 using AdjPtr = c10::intrusive_ptr<Adj>;

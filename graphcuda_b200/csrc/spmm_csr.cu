@@ -32,6 +32,7 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <mutex>
@@ -122,6 +123,10 @@ struct Vec<4> {
   static __device__ __forceinline__ T add(const T& a, const T& b) {
     return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
   }
+  static __device__ __forceinline__ T shfl_xor(const T& a, int o) {
+    return make_float4(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
+                       __shfl_xor_sync(0xffffffffu, a.z, o), __shfl_xor_sync(0xffffffffu, a.w, o));
+  }
   static __device__ __forceinline__ T gt0(const T& a) {
     return make_float4(a.x > 0.f ? 1.f : 0.f, a.y > 0.f ? 1.f : 0.f, a.z > 0.f ? 1.f : 0.f, a.w > 0.f ? 1.f : 0.f);
   }
@@ -143,6 +148,7 @@ struct Vec<1> {
   static __device__ __forceinline__ void store(float* p, T v) { *p = v; }
   static __device__ __forceinline__ void fma(T& a, float s, const T& h) { a = fmaf(s, h, a); }
   static __device__ __forceinline__ T add(const T& a, const T& b) { return a + b; }
+  static __device__ __forceinline__ T shfl_xor(const T& a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
   static __device__ __forceinline__ T gt0(const T& a) { return a > 0.f ? 1.f : 0.f; }
   static __device__ __forceinline__ T mul(const T& a, const T& b) { return a * b; }
 };
@@ -397,6 +403,65 @@ spmm_pieces_narrow_kernel(const int32_t* __restrict__ rowptr, const int32_t* __r
 #pragma unroll
   for (int a = 0; a < NV; ++a)
     if (lane_g == a && a < units) finish_store<4>(acc[a], yrow, mrow, a * 4, my_ep, grow);
+}
+
+// Matrices with too few pieces to fill the GPU (a Cora-sized graph): a warp per piece, S = 32 / UN non-zeros side by
+// side, each gathered by UN lanes of one vector, U rounds in flight; the S partial sums are folded by shuffles in a
+// fixed order.  With groups of 4 lanes walking a piece one non-zero at a time, the longest piece (128 non-zeros) took
+// 32 dependent gathers -- 10 us on a matrix whose average row has 5.
+template <int UN, int VW, bool PLANNED>
+__global__ void __launch_bounds__(256)
+spmm_short_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, const float* __restrict__ val,
+                  int n_pieces, const int32_t* __restrict__ p_start, const int32_t* __restrict__ p_len,
+                  const int32_t* __restrict__ p_target, int F, const float* __restrict__ H, int64_t ldH,
+                  float* __restrict__ Y, int64_t ldY, float* __restrict__ scratch, int64_t ldS, int slot_capacity,
+                  int32_t* __restrict__ overflow, Epilogue ep, const __grid_constant__ RowBlocks rb) {
+  using V = Vec<VW>;
+  constexpr int S = 32 / UN, U = 4;
+  const int lane = threadIdx.x % 32, slot = lane / UN, f = (lane % UN) * VW + int(blockIdx.y) * UN * VW;
+  const int v = blockIdx.x * 8 + threadIdx.x / 32;
+  if (v >= n_pieces) return;
+  int start, end, target;
+  if (PLANNED) {
+    start = __ldg(p_start + v);
+    end = start + __ldg(p_len + v);
+    target = __ldg(p_target + v);
+  } else {
+    start = __ldg(rowptr + v);
+    end = __ldg(rowptr + v + 1);
+    target = v;
+  }
+  const bool direct = target >= 0;
+  if (!direct && (~target) >= slot_capacity) {
+    if (lane == 0) *overflow = 1;
+    return;
+  }
+  const bool live = f < F;
+  typename V::T acc = V::zero();
+  for (int base = start + slot; base < end; base += S * U) {
+    int c[U];
+    float w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool ok = base + u * S < end;
+      c[u] = ok ? __ldg(col + base + u * S) : -1;
+      w[u] = ok ? __ldg(val + base + u * S) : 0.f;
+    }
+    typename V::G h[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) h[u] = (live && c[u] >= 0) ? V::gather(H + int64_t(c[u]) * ldH + f) : V::gzero();
+#pragma unroll
+    for (int u = 0; u < U; ++u) V::fma(acc, w[u], h[u]);
+  }
+#pragma unroll
+  for (int o = UN; o < 32; o <<= 1) acc = V::add(acc, V::shfl_xor(acc, o));
+  if (slot != 0 || !live) return;
+  float* yrow = direct ? out_row(rb, Y, ldY, target) : scratch + int64_t(~target) * ldS;
+  float* mrow = (direct && ep.mask) ? ep.mask + int64_t(target) * ldY : nullptr;
+  const float* grow = (direct && ep.gate) ? ep.gate + int64_t(target) * ldY : nullptr;
+  Epilogue my_ep = ep;
+  if (!direct) my_ep = Epilogue{nullptr, nullptr, nullptr, 0, 0};
+  finish_store<VW>(acc, yrow, mrow, f, my_ep, grow);
 }
 
 // One warp per cut row: adds that row's partial sums in slot order, then the
@@ -657,6 +722,28 @@ void launch_pieces(bool planned, const int32_t* rowptr, const int32_t* col, cons
   launch_pieces<G, A, VWID, UU>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, \
                                 cap, ovf, ep, rb, st)
 
+// Matrices that a warp per piece serves sooner than groups of lanes do.  Measured (us, groups / warp per piece): 20 K
+// pieces F = 16 19.5 / 11.2, F = 64 28.5 / 16.1; 61 K pieces F = 7 19.3 / 21.4, F = 16 24.5 / 23.9, F = 64 35 / 29; 77 K
+// longer pieces F = 32 54 / 47; 175 K pieces F = 16 39 / 55, F = 64 79 / 78.
+inline bool short_pieces(int n_pieces, int F) { return n_pieces <= gc::kNumSMs * (F <= 8 ? 256 : 512); }
+
+template <int UN, int VW>
+void launch_short(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
+                  const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const float* H, int64_t ldH, float* Y,
+                  int64_t ldY, float* scratch, int64_t ldS, int cap, int32_t* ovf, const Epilogue& ep,
+                  const RowBlocks& rb, cudaStream_t st) {
+  const dim3 grid(unsigned((n_pieces + 7) / 8), unsigned((F + UN * VW - 1) / (UN * VW)));
+  if (planned)
+    spmm_short_kernel<UN, VW, true><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY,
+                                                          scratch, ldS, cap, ovf, ep, rb);
+  else
+    spmm_short_kernel<UN, VW, false><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY,
+                                                           scratch, ldS, cap, ovf, ep, rb);
+}
+#define GC_SHORT(UN, VWID)                                                                                       \
+  launch_short<UN, VWID>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap,  \
+                         ovf, ep, rb, st)
+
 // GROUP x NACC 128-bit vectors cover a row of H; small groups keep several
 // pieces in flight per warp and four accumulators per lane amortise the
 // (col, val) broadcast.
@@ -665,6 +752,14 @@ void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, cons
                    float* Y, int64_t ldY, float* scratch, int64_t ldS, int cap, int32_t* ovf, const Epilogue& ep,
                    const RowBlocks& rb, cudaStream_t st) {
   const int units = F / 4;  // 128-bit vectors per row
+  if (short_pieces(n_pieces, F) && units <= 16) {
+    if (units <= 1) GC_SHORT(1, 4);
+    else if (units <= 2) GC_SHORT(2, 4);
+    else if (units <= 4) GC_SHORT(4, 4);
+    else if (units <= 8) GC_SHORT(8, 4);
+    else GC_SHORT(16, 4);
+    return;
+  }
   // Measured on the 126 M-non-zero graph: up to 8 floats the lane-per-non-zero kernel wins (F = 8: 0.99 ms
   // against 2.0 ms); from 12 to 32 floats groups of 4 lanes with one or two 128-bit vectors per lane and 4
   // non-zeros in flight do (F = 32: 1.5 ms against 1.7 ms for 8 lanes x 1 vector, 3.4 ms for 2 lanes x 4
@@ -698,6 +793,12 @@ void dispatch_scalar(bool planned, const int32_t* rowptr, const int32_t* col, co
                      const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const float* H, int64_t ldH,
                      float* Y, int64_t ldY, float* scratch, int64_t ldS, int cap, int32_t* ovf, const Epilogue& ep,
                      const RowBlocks& rb, cudaStream_t st) {
+  if (short_pieces(n_pieces, F) && F <= 32) {
+    if (F <= 4) GC_SHORT(4, 1);
+    else if (F <= 8) GC_SHORT(8, 1);
+    else GC_SHORT(16, 1);
+    return;
+  }
   if (F <= 8) GC_PIECES(8, 1, 1, 4);
   else if (F <= 16) GC_PIECES(16, 1, 1, 4);
   else if (F <= 32) GC_PIECES(32, 1, 1, 4);
@@ -746,6 +847,17 @@ int64_t gc_spmm_default_segment(int64_t nnz) {
   int64_t p2 = 128;
   while (p2 < want && p2 < GC_SPMM_SEGMENT_MAX) p2 *= 2;
   return p2;
+}
+
+int64_t gc_spmm_segment(int64_t nnz, int64_t F) {
+  // A piece is walked a few gathers per memory round trip: up to 64 columns by 4 lanes, wider rows by 8 to 32, so the
+  // longest piece is a floor under the time of the launch.  Cutting costs partial sums and shortens the average piece.
+  // Measured optima: 2.5 M non-zeros 128..256 (F <= 64) and 256..512 (wider), 10.5 M 512 and 512..1024, 24.5 M
+  // 512..1024 and 1024.  At nnz / 8192 (gc_spmm_default_segment: 512, 2048, 2048) F = 16 took 65 / 352 / 407 us
+  // against 39 / 116 / 226, F = 256 1207 us on the second against 806.
+  const double want = (F <= 64 ? 0.12 : 0.16) * std::sqrt(double(std::max<int64_t>(nnz, 0)));
+  const int64_t seg = (int64_t(want) + 31) / 32 * 32;
+  return std::min<int64_t>(GC_SPMM_SEGMENT_MAX, std::max<int64_t>(128, seg));
 }
 
 size_t gc_spmm_plan_workspace_bytes(int64_t M, int64_t n_pieces) {

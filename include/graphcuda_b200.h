@@ -75,6 +75,11 @@ int64_t gc_spmm_default_panel_cols(int64_t K, int64_t F);
 /* Default segment length for a matrix of nnz non-zeros: a power of two in
  * [128, GC_SPMM_SEGMENT_MAX], about nnz / 8192. */
 int64_t gc_spmm_default_segment(int64_t nnz);
+/* Segment length for a plan that serves products of feature width F: in
+ * [128, GC_SPMM_SEGMENT_MAX], growing with the square root of nnz.  Shorter than
+ * the default above on large matrices, where it bounds the time of the longest
+ * piece. */
+int64_t gc_spmm_segment(int64_t nnz, int64_t F);
 /* Scratch for plan construction; pass n_pieces = 0 for gc_spmm_plan_count. */
 size_t gc_spmm_plan_workspace_bytes(int64_t M, int64_t n_pieces);
 /* counts (device, int64[3]) <- {n_pieces, n_slots, n_cut}. */
