@@ -29,6 +29,7 @@ SIGNATURES = {
     "gc_spmm_plan_workspace_bytes": (_size, [_i64, _i64]),
     "gc_spmm_default_segment": (_i64, [_i64]),
     "gc_spmm_segment": (_i64, [_i64, _i64]),
+    "gc_pad_rows_f32": (_int, [_f32p, _i64, _f32p, _i64, _i64, _i64, _void]),
     "gc_spmm_plan_count": (_int, [_i32p, _i32p, _i64, _i64, _i64, _i64, _i64p, _void, _size, _void]),
     "gc_spmm_plan_bytes": (_size, [_i64, _i64]),
     "gc_spmm_plan_build": (_int, [_i32p, _i32p, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _void, _size, _void, _size,

@@ -57,6 +57,22 @@ transpose_kernel(const float* __restrict__ in, int64_t ldin, float* __restrict__
   }
 }
 
+// One 16-byte store per thread; the loads of a warp are one contiguous stretch of the source whatever its pitch.
+__global__ void __launch_bounds__(256)
+pad_rows_kernel(const float* __restrict__ src, int64_t lds, float* __restrict__ dst, int64_t ldd, int64_t rows, int cols) {
+  const int quads = int(ldd / 4);
+  const int64_t total = rows * quads;
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < total; i += int64_t(gridDim.x) * 256) {
+    const int64_t r = i / quads;
+    const int c = int(i - r * quads) * 4;
+    const float* p = src + r * lds + c;
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = c + j < cols ? __ldg(p + j) : 0.f;
+    *reinterpret_cast<float4*>(dst + r * ldd + c) = make_float4(v[0], v[1], v[2], v[3]);
+  }
+}
+
 template <bool FROM_ACT>
 int mask_mul(const float* dY, int64_t lddy, const float* S, int64_t lds, float* G, int64_t ldg, int64_t M, int64_t N,
              void* stream, const char* who) {
@@ -109,6 +125,18 @@ scatter_slabs_kernel(const float* __restrict__ src, int64_t ld, int64_t rows, in
 }  // namespace
 
 extern "C" {
+
+int gc_pad_rows_f32(const float* src, int64_t ld_src, float* dst, int64_t ld_dst, int64_t rows, int64_t cols,
+                    void* stream) {
+  GC_REQUIRE(rows >= 0 && cols >= 0 && cols < INT32_MAX, "gc_pad_rows_f32: bad size");
+  if (rows == 0 || cols == 0) return GC_OK;
+  GC_REQUIRE(src && dst, "gc_pad_rows_f32: null pointer");
+  GC_REQUIRE(ld_src >= cols && ld_dst >= cols && ld_dst % 4 == 0 && gc::aligned16(dst),
+             "gc_pad_rows_f32: ld_dst must be a multiple of 4 and dst 16-byte aligned");
+  const unsigned grid = unsigned(std::min<int64_t>(gc::ceil_div(rows * (ld_dst / 4), 256), gc::kNumSMs * 16));
+  pad_rows_kernel<<<grid, 256, 0, gc::as_stream(stream)>>>(src, ld_src, dst, ld_dst, rows, int(cols));
+  return gc::check_launch("gc_pad_rows_f32");
+}
 
 int gc_scatter_column_slabs_f32(const float* src, int64_t ld, int64_t rows, int64_t F, int64_t w, float* const* dst,
                                 int n_dst, int64_t dst_ld, void* stream) {

@@ -147,8 +147,7 @@ py::object spmm(const AdjPtr& adj, const Tensor& Hin, const OptTensor& bias_in, 
       ep.gate = gate->const_data_ptr<float>();
     }
     if (M != 0 && F != 0)
-      spmm_into(a, H.data_ptr(), H.size(0) > 1 ? H.stride(0) : std::max<int64_t>(F, 1), h16, F,
-                static_cast<float*>(out.data_ptr()), ldy, ep, accumulate, panel_cols);
+      spmm_into(a, H, static_cast<float*>(out.data_ptr()), ldy, ep, accumulate, panel_cols);
   }
   return want_mask ? py::object(py::make_tuple(out, mask)) : py::cast(out);
 }

@@ -203,13 +203,35 @@ bool Adj::is_symmetric() {
   return symmetric != 0;
 }
 
-void spmm_into(Adj& a, const void* H, int64_t ldh, bool h16, int64_t F, float* Y, int64_t ldy, const Epi& ep,
-               bool accumulate, int64_t panel_cols) {
+void spmm_into(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, bool accumulate, int64_t panel_cols) {
   const at::Device dev = a.device();
+  const int64_t F = Hin.size(1);
+  const bool h16 = Hin.scalar_type() == at::kBFloat16;
   std::shared_ptr<Plan> plan = a.use_plan ? a.plan_for(F, panel_cols) : nullptr;
   Scratch s{nullptr, 0, Tensor()};
   if (plan && plan->n_cut > 0) s = scratch(kSpmm, abi.gc_spmm_scratch_bytes(plan->n_slots, F), dev);
-  const int epi = (ep.relu ? GC_EPI_RELU : 0) | (accumulate ? GC_EPI_ACCUMULATE : 0);
+  int epi = (ep.relu ? GC_EPI_RELU : 0) | (accumulate ? GC_EPI_ACCUMULATE : 0);
+  const void* H = Hin.data_ptr();
+  int64_t ldh = Hin.size(0) > 1 ? Hin.stride(0) : std::max<int64_t>(F, 1);
+  Tensor padded;
+  if (!h16 && (F % 4 != 0 || ldh % 4 != 0 || reinterpret_cast<uintptr_t>(H) % 16 != 0)) {
+    const int64_t f4 = (F + 3) / 4 * 4;
+    const int64_t last = (Hin.storage_offset() + (a.K - 1) * ldh + f4) * int64_t(sizeof(float));
+    if (a.K > 0 && ldh % 4 == 0 && ldh >= f4 && reinterpret_cast<uintptr_t>(H) % 16 == 0 &&
+        last <= int64_t(Hin.storage().nbytes())) {
+      epi |= GC_EPI_H_PADDED;  // a view of wider rows: what lies beyond the width may be read, and is not used
+    } else if (F > 8 && a.nnz >= 4 * a.K && a.nnz >= (1 << 16)) {
+      // Rows that are not 16-byte aligned are gathered one float per lane.  Copying H to an aligned pitch first (8
+      // bytes per element, streamed) pays where every row is gathered several times: 169 K rows of 47, 15 non-zeros
+      // each, 136 us against 9 + 68.
+      padded = empty_f32(a.K, f4, dev);
+      check(abi.gc_pad_rows_f32(static_cast<const float*>(H), ldh, padded.data_ptr<float>(), f4, a.K, F, stream_of(dev)),
+            "gc_pad_rows_f32");
+      H = padded.data_ptr();
+      ldh = f4;
+      epi |= GC_EPI_H_PADDED;
+    }
+  }
   const int32_t* rp = a.rowptr.const_data_ptr<int32_t>();
   const int32_t* cp = a.col.const_data_ptr<int32_t>();
   const float* vp = a.val.const_data_ptr<float>();

@@ -37,7 +37,7 @@ inline void require(bool cond, const char* msg) {
   X(gc_spmm_scratch_bytes) X(gc_spmm_csr_f32) X(gc_spmm_csr_bf16h_f32) X(gc_gemm_workspace_bytes) X(gc_gemm_f32)    \
   X(gc_convert_f32_bf16) X(gc_gemm_bf16_workspace_bytes) X(gc_gemm_bf16_f32) X(gc_relu_backward_f32)                \
   X(gc_mask_mul_f32) X(gc_nll_workspace_bytes) X(gc_logsoftmax_nll_forward_f32) X(gc_logsoftmax_nll_backward_f32)   \
-  X(gc_argmax_accuracy_f32) X(gc_adam_step_f32) X(gc_sgd_step_f32) X(gc_csr_is_symmetric)
+  X(gc_argmax_accuracy_f32) X(gc_adam_step_f32) X(gc_sgd_step_f32) X(gc_csr_is_symmetric) X(gc_pad_rows_f32)
 struct Abi {
 #define X(name) decltype(&::name) name = nullptr;
   GC_HOST_FUNCTIONS(X)
@@ -121,9 +121,8 @@ struct Adj : torch::CustomClassHolder {
 };
 using AdjPtr = c10::intrusive_ptr<Adj>;
 
-// Y = A H (+bias)(ReLU)(mask)(gate); H is rows x F float32 (or bfloat16) with unit column stride.
-void spmm_into(Adj& a, const void* H, int64_t ldh, bool h16, int64_t F, float* Y, int64_t ldy, const Epi& ep,
-               bool accumulate, int64_t panel_cols);
+// Y = A H (+bias)(ReLU)(mask)(gate); H is float32 (or bfloat16) with unit column stride.
+void spmm_into(Adj& a, const Tensor& H, float* Y, int64_t ldy, const Epi& ep, bool accumulate, int64_t panel_cols);
 Tensor adj_matmul(Adj& a, Tensor H, int prec, const Epi& ep);
 
 // ------------------------------------------------------------------ layer, loss, optimizers (layer.cpp, tail.cpp)

@@ -54,6 +54,17 @@ Tensor pad_cols(const Tensor& t, int64_t width) {
   return out;
 }
 
+// For a product that is aggregated next: rows on a 16-byte pitch, so that an odd width is still gathered in vectors.
+Tensor product_to_gather(Tensor A, Tensor B, bool tb, int prec) {
+  const Mat a = as_operand(A);
+  Mat b = as_operand(B);
+  if (tb) b = b.t();
+  const int64_t n = b.cols, ld = (n + 3) / 4 * 4;
+  Tensor out = empty_f32(a.rows, ld, A.device());
+  gemm_into(a, b, out.data_ptr<float>(), std::max<int64_t>(ld, 1), Epi{}, false, prec, A.device());
+  return ld == n ? out : out.narrow(1, 0, n);
+}
+
 Tensor product(Tensor A, Tensor B, bool ta, bool tb, int prec, const Epi& ep) {
   Mat a = as_operand(A), b = as_operand(B);
   if (ta) a = a.t();
@@ -113,11 +124,9 @@ Tensor adj_matmul(Adj& a, Tensor H, int prec, const Epi& ep) {
     // bf16 tier, wide H on a graph with enough non-zeros per row: the aggregation gathers a bf16 copy (half the bytes
     // through the SM fill path, fp32 sums).  126 M non-zeros, F = 256: 6.9 ms + 0.6 ms for the copy against 8.8 ms;
     // narrower or sparser products do not repay the conversion pass.
-    const Tensor H16 = to_bf16(H, false);
-    spmm_into(a, H16.data_ptr(), F, true, F, out.data_ptr<float>(), ldy, ep, false, 0);
+    spmm_into(a, to_bf16(H, false), out.data_ptr<float>(), ldy, ep, false, 0);
   } else {
-    spmm_into(a, H.const_data_ptr<float>(), H.size(0) > 1 ? H.stride(0) : ldy, false, F, out.data_ptr<float>(), ldy,
-              ep, false, 0);
+    spmm_into(a, H, out.data_ptr<float>(), ldy, ep, false, 0);
   }
   return out;
 }
@@ -150,7 +159,7 @@ Forward layer_forward(const Tensor& X, Adj& a, const Tensor& W, const OptTensor&
     b = pad_cols(b, width);
     ep.bias = b.const_data_ptr<float>();
   }
-  const Tensor H = product(X, pad_cols(W, width), false, false, prec, Epi{});
+  const Tensor H = product_to_gather(X, pad_cols(W, width), false, prec);
   if (want_mask) {
     f.mask = empty_f32(a.M, width, X.device());
     ep.mask = f.mask.data_ptr<float>();
@@ -208,7 +217,7 @@ Grads layer_backward(Tensor G, const Tensor& X, Adj& a, const Tensor& W, bool re
   if (inter.defined()) {
     if (need_dW) r.dW = product(inter, G, true, false, prec, Epi{});
     // A, not A^T: reference gcn.cu:49
-    if (need_dX) r.dX = adj_matmul(a, product(G, W, false, true, prec, Epi{}), prec, gate);
+    if (need_dX) r.dX = adj_matmul(a, product_to_gather(G, W, true, prec), prec, gate);
   } else {
     // Y = A (X W), A symmetric: S = A^T G = A G
     const int64_t width = padded_width(X.size(0), W.size(0), out_dim);

@@ -199,6 +199,26 @@ struct Vec<8> {
   static __device__ __forceinline__ T mul(const T& x, const T& y) { return Float8{V4::mul(x.a, y.a), V4::mul(x.b, y.b)}; }
 };
 
+// One element of an output row whose rows are not 16-byte aligned (an odd width).
+__device__ __forceinline__ void finish_store_one(float v, float* yrow, float* mrow, int f, const Epilogue& ep,
+                                                 const float* grow) {
+  if (ep.accumulate) v += yrow[f];
+  if (ep.bias) v += __ldg(ep.bias + f);
+  if (ep.relu || mrow) {
+    const float m = v > 0.f ? 1.f : 0.f;
+    if (mrow) mrow[f] = m;
+    if (ep.relu) v *= m;
+  }
+  if (grow) v *= __ldcs(grow + f) > 0.f ? 1.f : 0.f;
+  yrow[f] = v;
+}
+
+// A vector of accumulated columns f .. f + 3 to a row of Y of F columns: SO (scalar output) when Y's rows are not
+// 16-byte aligned although H's are; partial sums (direct == false) always go to aligned scratch rows.
+template <int VW, bool SO>
+__device__ __forceinline__ void store_columns(const typename Vec<VW>::T& acc, float* yrow, float* mrow, int f, int F,
+                                              bool direct, const Epilogue& ep, const float* grow);
+
 // Applies accumulate / bias / mask / ReLU to one vector and stores it.
 template <int VW>
 __device__ __forceinline__ void finish_store(typename Vec<VW>::T acc, float* yrow, float* mrow, int f,
@@ -215,6 +235,22 @@ __device__ __forceinline__ void finish_store(typename Vec<VW>::T acc, float* yro
   V::store(yrow + f, acc);
 }
 
+template <int VW, bool SO>
+__device__ __forceinline__ void store_columns(const typename Vec<VW>::T& acc, float* yrow, float* mrow, int f, int F,
+                                              bool direct, const Epilogue& ep, const float* grow) {
+  if constexpr (SO) {
+    static_assert(VW == 4, "scalar output belongs to fp32 vector gathers");
+    if (direct) {
+      const float v[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (f + j < F) finish_store_one(v[j], yrow, mrow, f + j, ep, grow);
+      return;
+    }
+  }
+  finish_store<VW>(acc, yrow, mrow, f, ep, grow);
+}
+
 // ---------------------------------------------------------------- piece kernel
 // One group of GROUP lanes per piece; NACC vectors of VW floats per lane cover
 // GROUP*NACC*VW feature columns per pass; wider F loops over passes.
@@ -227,7 +263,8 @@ __device__ __forceinline__ void finish_store(typename Vec<VW>::T acc, float* yro
 // it keeps a whole round of U x NACC loads in flight.  Measured on the
 // 126 M-non-zero graph, F = 256: 12.6 ms unconstrained, 8.7 ms at 2, 8.4 ms
 // at 3; F = 100: 6.3 / 4.4 / 4.4 ms.
-template <int GROUP, int NACC, int VW, int U, bool PLANNED, int MIN_CTAS>
+// SO: F is the true width of Y; the columns up to the next multiple of 4 are gathered (H is padded) and dropped.
+template <int GROUP, int NACC, int VW, int U, bool PLANNED, int MIN_CTAS, bool SO>
 __global__ void __launch_bounds__(256, MIN_CTAS)
 spmm_pieces_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                    const float* __restrict__ val, int n_pieces, const int32_t* __restrict__ p_start,
@@ -267,13 +304,14 @@ spmm_pieces_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict
 
   // Feature columns beyond one pass are walked in turn -- or, when the matrix has too few pieces to fill the
   // GPU (a Cora-sized graph with a 1433-wide H), spread over gridDim.y so that the passes run side by side.
-  for (int f0 = blockIdx.y * PASS; f0 < F; f0 += gridDim.y * PASS) {
+  const int Fg = SO ? (F + 3) / 4 * 4 : F;
+  for (int f0 = blockIdx.y * PASS; f0 < Fg; f0 += gridDim.y * PASS) {
     typename V::T acc[NACC];
     bool live[NACC];
 #pragma unroll
     for (int a = 0; a < NACC; ++a) {
       acc[a] = V::zero();
-      live[a] = (f0 + (a * GROUP + lane_g) * VW) < F;
+      live[a] = (f0 + (a * GROUP + lane_g) * VW) < Fg;
     }
     int c_next = 0;
     float w_next = 0.f;
@@ -317,7 +355,8 @@ spmm_pieces_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict
     }
 #pragma unroll
     for (int a = 0; a < NACC; ++a)
-      if (live[a]) finish_store<VW>(acc[a], yrow, mrow, f0 + (a * GROUP + lane_g) * VW, my_ep, grow);
+      if (live[a])
+        store_columns<VW, SO>(acc[a], yrow, mrow, f0 + (a * GROUP + lane_g) * VW, F, direct, my_ep, grow);
   }
 }
 
@@ -327,7 +366,7 @@ spmm_pieces_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict
 // the 8 lanes' sums are combined by a butterfly of shuffles in a fixed order.
 // With 16..32-byte rows this keeps several times as many gathers in flight per
 // warp as the column-parallel mapping and needs no (col, val) broadcast.
-template <int NV, int U, bool PLANNED>
+template <int NV, int U, bool PLANNED, bool SO>
 __global__ void __launch_bounds__(256)
 spmm_pieces_narrow_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col,
                           const float* __restrict__ val, int n_pieces, const int32_t* __restrict__ p_start,
@@ -355,7 +394,7 @@ spmm_pieces_narrow_kernel(const int32_t* __restrict__ rowptr, const int32_t* __r
     if (lane_g == 0) *overflow = 1;
     return;
   }
-  const int units = F / 4;
+  const int units = SO ? (F + 3) / 4 : F / 4;
   float4 acc[NV];
 #pragma unroll
   for (int a = 0; a < NV; ++a) acc[a] = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -402,14 +441,14 @@ spmm_pieces_narrow_kernel(const int32_t* __restrict__ rowptr, const int32_t* __r
   // lane a stores vector a
 #pragma unroll
   for (int a = 0; a < NV; ++a)
-    if (lane_g == a && a < units) finish_store<4>(acc[a], yrow, mrow, a * 4, my_ep, grow);
+    if (lane_g == a && a < units) store_columns<4, SO>(acc[a], yrow, mrow, a * 4, F, direct, my_ep, grow);
 }
 
 // Matrices with too few pieces to fill the GPU (a Cora-sized graph): a warp per piece, S = 32 / UN non-zeros side by
 // side, each gathered by UN lanes of one vector, U rounds in flight; the S partial sums are folded by shuffles in a
 // fixed order.  With groups of 4 lanes walking a piece one non-zero at a time, the longest piece (128 non-zeros) took
 // 32 dependent gathers -- 10 us on a matrix whose average row has 5.
-template <int UN, int VW, bool PLANNED>
+template <int UN, int VW, bool PLANNED, bool SO>
 __global__ void __launch_bounds__(256)
 spmm_short_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__ col, const float* __restrict__ val,
                   int n_pieces, const int32_t* __restrict__ p_start, const int32_t* __restrict__ p_len,
@@ -436,7 +475,7 @@ spmm_short_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict_
     if (lane == 0) *overflow = 1;
     return;
   }
-  const bool live = f < F;
+  const bool live = f < (SO ? (F + 3) / 4 * 4 : F);
   typename V::T acc = V::zero();
   for (int base = start + slot; base < end; base += S * U) {
     int c[U];
@@ -461,7 +500,7 @@ spmm_short_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict_
   const float* grow = (direct && ep.gate) ? ep.gate + int64_t(target) * ldY : nullptr;
   Epilogue my_ep = ep;
   if (!direct) my_ep = Epilogue{nullptr, nullptr, nullptr, 0, 0};
-  finish_store<VW>(acc, yrow, mrow, f, my_ep, grow);
+  store_columns<VW, SO>(acc, yrow, mrow, f, F, direct, my_ep, grow);
 }
 
 // One warp per cut row: adds that row's partial sums in slot order, then the
@@ -697,7 +736,7 @@ constexpr int pieces_min_ctas(int group, int nacc, int vw) {
   return ((vw == 4 && nacc >= 3 && group <= 8) || (vw == 8 && nacc >= 2 && group <= 8)) ? 2 : 3;
 }
 
-template <int GROUP, int NACC, int VW, int U>
+template <int GROUP, int NACC, int VW, int U, bool SO = false>
 void launch_pieces(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
                    const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const typename Vec<VW>::HT* H,
                    int64_t ldH,
@@ -711,15 +750,16 @@ void launch_pieces(bool planned, const int32_t* rowptr, const int32_t* col, cons
   const dim3 grid(gx, gy);
   constexpr int MINB = pieces_min_ctas(GROUP, NACC, VW);
   if (planned)
-    spmm_pieces_kernel<GROUP, NACC, VW, U, true, MINB>
+    spmm_pieces_kernel<GROUP, NACC, VW, U, true, MINB, SO>
         <<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap, ovf, ep, rb);
   else
-    spmm_pieces_kernel<GROUP, NACC, VW, U, false, MINB>
+    spmm_pieces_kernel<GROUP, NACC, VW, U, false, MINB, SO>
         <<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap, ovf, ep, rb);
 }
 
-#define GC_PIECES(G, A, VWID, UU)                                                                                 \
-  launch_pieces<G, A, VWID, UU>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, \
+#define GC_PIECES(G, A, VWID, UU) GC_PIECES_SO(G, A, VWID, UU, false)
+#define GC_PIECES_SO(G, A, VWID, UU, SO_)                                                                         \
+  launch_pieces<G, A, VWID, UU, SO_>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, \
                                 cap, ovf, ep, rb, st)
 
 // Matrices that a warp per piece serves sooner than groups of lanes do.  Measured (us, groups / warp per piece): 20 K
@@ -727,37 +767,38 @@ void launch_pieces(bool planned, const int32_t* rowptr, const int32_t* col, cons
 // longer pieces F = 32 54 / 47; 175 K pieces F = 16 39 / 55, F = 64 79 / 78.
 inline bool short_pieces(int n_pieces, int F) { return n_pieces <= gc::kNumSMs * (F <= 8 ? 256 : 512); }
 
-template <int UN, int VW>
+template <int UN, int VW, bool SO>
 void launch_short(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
                   const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const float* H, int64_t ldH, float* Y,
                   int64_t ldY, float* scratch, int64_t ldS, int cap, int32_t* ovf, const Epilogue& ep,
                   const RowBlocks& rb, cudaStream_t st) {
   const dim3 grid(unsigned((n_pieces + 7) / 8), unsigned((F + UN * VW - 1) / (UN * VW)));
   if (planned)
-    spmm_short_kernel<UN, VW, true><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY,
+    spmm_short_kernel<UN, VW, true, SO><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY,
                                                           scratch, ldS, cap, ovf, ep, rb);
   else
-    spmm_short_kernel<UN, VW, false><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY,
+    spmm_short_kernel<UN, VW, false, SO><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY,
                                                            scratch, ldS, cap, ovf, ep, rb);
 }
-#define GC_SHORT(UN, VWID)                                                                                       \
-  launch_short<UN, VWID>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap,  \
+#define GC_SHORT(UN, VWID, SO_)                                                                                  \
+  launch_short<UN, VWID, SO_>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap,  \
                          ovf, ep, rb, st)
 
 // GROUP x NACC 128-bit vectors cover a row of H; small groups keep several
 // pieces in flight per warp and four accumulators per lane amortise the
 // (col, val) broadcast.
+template <bool SO>
 void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
                    const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const float* H, int64_t ldH,
                    float* Y, int64_t ldY, float* scratch, int64_t ldS, int cap, int32_t* ovf, const Epilogue& ep,
                    const RowBlocks& rb, cudaStream_t st) {
-  const int units = F / 4;  // 128-bit vectors per row
+  const int units = (F + 3) / 4;  // 128-bit vectors per row (SO: F may be odd, rows of H are padded)
   if (short_pieces(n_pieces, F) && units <= 16) {
-    if (units <= 1) GC_SHORT(1, 4);
-    else if (units <= 2) GC_SHORT(2, 4);
-    else if (units <= 4) GC_SHORT(4, 4);
-    else if (units <= 8) GC_SHORT(8, 4);
-    else GC_SHORT(16, 4);
+    if (units <= 1) GC_SHORT(1, 4, SO);
+    else if (units <= 2) GC_SHORT(2, 4, SO);
+    else if (units <= 4) GC_SHORT(4, 4, SO);
+    else if (units <= 8) GC_SHORT(8, 4, SO);
+    else GC_SHORT(16, 4, SO);
     return;
   }
   // Measured on the 126 M-non-zero graph: up to 8 floats the lane-per-non-zero kernel wins (F = 8: 0.99 ms
@@ -769,10 +810,10 @@ void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, cons
 #define GC_NARROW(NV, UU)                                                                                       \
   do {                                                                                                          \
     if (planned)                                                                                                \
-      spmm_pieces_narrow_kernel<NV, UU, true><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, \
+      spmm_pieces_narrow_kernel<NV, UU, true, SO><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, \
                                                                    ldH, Y, ldY, scratch, ldS, cap, ovf, ep, rb);    \
     else                                                                                                        \
-      spmm_pieces_narrow_kernel<NV, UU, false><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F,  \
+      spmm_pieces_narrow_kernel<NV, UU, false, SO><<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F,  \
                                                                     H, ldH, Y, ldY, scratch, ldS, cap, ovf, ep, rb); \
   } while (0)
     if (units <= 1) GC_NARROW(1, 4);
@@ -780,13 +821,13 @@ void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, cons
 #undef GC_NARROW
     return;
   }
-  if (units <= 4) GC_PIECES(4, 1, 4, 4);
-  else if (units <= 8) GC_PIECES(4, 2, 4, 4);  // F = 32: 1.54 ms; 8 lanes x 1 vector x 8 in flight: 1.73 ms
-  else if (units <= 12) GC_PIECES(4, 3, 4, 4);  // F = 48 on 126 M non-zeros: 2.24 ms against 2.35 ms with a fourth, idle vector
-  else if (units <= 16) GC_PIECES(4, 4, 4, 4);
-  else if (units <= 32) GC_PIECES(8, 4, 4, 4);
-  else if (units <= 64) GC_PIECES(16, 4, 4, 4);
-  else GC_PIECES(32, 4, 4, 2);
+  if (units <= 4) GC_PIECES_SO(4, 1, 4, 4, SO);
+  else if (units <= 8) GC_PIECES_SO(4, 2, 4, 4, SO);  // F = 32: 1.54 ms; 8 lanes x 1 vector x 8 in flight: 1.73 ms
+  else if (units <= 12) GC_PIECES_SO(4, 3, 4, 4, SO);  // F = 48 on 126 M non-zeros: 2.24 ms against 2.35 ms with a fourth, idle vector
+  else if (units <= 16) GC_PIECES_SO(4, 4, 4, 4, SO);
+  else if (units <= 32) GC_PIECES_SO(8, 4, 4, 4, SO);
+  else if (units <= 64) GC_PIECES_SO(16, 4, 4, 4, SO);
+  else GC_PIECES_SO(32, 4, 4, 2, SO);
 }
 
 void dispatch_scalar(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
@@ -794,9 +835,9 @@ void dispatch_scalar(bool planned, const int32_t* rowptr, const int32_t* col, co
                      float* Y, int64_t ldY, float* scratch, int64_t ldS, int cap, int32_t* ovf, const Epilogue& ep,
                      const RowBlocks& rb, cudaStream_t st) {
   if (short_pieces(n_pieces, F) && F <= 32) {
-    if (F <= 4) GC_SHORT(4, 1);
-    else if (F <= 8) GC_SHORT(8, 1);
-    else GC_SHORT(16, 1);
+    if (F <= 4) GC_SHORT(4, 1, false);
+    else if (F <= 8) GC_SHORT(8, 1, false);
+    else GC_SHORT(16, 1, false);
     return;
   }
   if (F <= 8) GC_PIECES(8, 1, 1, 4);
@@ -819,6 +860,8 @@ void dispatch_bf16(bool planned, const int32_t* rowptr, const int32_t* col, cons
   else GC_PIECES(32, 2, 8, 4);
 }
 #undef GC_PIECES
+#undef GC_PIECES_SO
+#undef GC_SHORT
 
 inline int64_t scratch_ld(int64_t F) { return (F + 3) & ~int64_t(3); }
 
@@ -971,7 +1014,8 @@ int spmm_run(const int32_t* rowptr, const int32_t* col, const float* val, int64_
              void* scratch, size_t scratch_bytes, void* stream) {
   GC_REQUIRE(M >= 0 && K >= 0 && F >= 0, "gc_spmm_csr_f32: negative size");
   GC_REQUIRE(M < INT32_MAX && K < INT32_MAX && F < INT32_MAX, "gc_spmm_csr_f32: size out of int32 range");
-  GC_REQUIRE((epilogue & ~(GC_EPI_RELU | GC_EPI_ACCUMULATE)) == 0, "gc_spmm_csr_f32: unknown epilogue bits");
+  GC_REQUIRE((epilogue & ~(GC_EPI_RELU | GC_EPI_ACCUMULATE | GC_EPI_H_PADDED)) == 0,
+             "gc_spmm_csr_f32: unknown epilogue bits");
   if (M == 0 || F == 0) return GC_OK;
   GC_REQUIRE(rowptr && Y, "gc_spmm_csr_f32: null rowptr/Y");
   GC_REQUIRE(ldY >= F && (K == 0 || ldH >= F), "gc_spmm_csr_f32: leading dimension smaller than F");
@@ -984,7 +1028,9 @@ int spmm_run(const int32_t* rowptr, const int32_t* col, const float* val, int64_
     for (int64_t b = 0; b * rb.block_rows < M; ++b) blocks_aligned = blocks_aligned && gc::aligned16(rb.base[b]);
   const bool out_vec4 = (ldY % 4 == 0) && gc::aligned16(Y) && blocks_aligned && (!bias || gc::aligned16(bias)) &&
                         (!mask || gc::aligned16(mask)) && (!gate || gc::aligned16(gate));
-  const bool vec4 = (F % 4 == 0) && (ldH % 4 == 0) && gc::aligned16(H) && out_vec4;
+  const bool in_vec4 = (ldH % 4 == 0) && gc::aligned16(H) &&
+                       (F % 4 == 0 || ((epilogue & GC_EPI_H_PADDED) && ldH >= scratch_ld(F)));
+  const bool vec4 = in_vec4 && F % 4 == 0 && out_vec4;
   if (H16 && !((F % 8 == 0) && (ldH % 8 == 0) && gc::aligned16(H16) && out_vec4))
     return gc::fail(GC_ERR_UNSUPPORTED,
                     "gc_spmm_csr_bf16h_f32: F and ldH must be multiples of 8, H16 / Y / bias / mask / gate 16-byte "
@@ -1021,7 +1067,9 @@ int spmm_run(const int32_t* rowptr, const int32_t* col, const float* val, int64_
   if (H16)
     dispatch_bf16(planned, rowptr, col, val, np, ps, pl, pt, int(F), H16, ldH, Y, ldY, sc, ldS, cap, ovf, ep, rb, st);
   else if (vec4)
-    dispatch_vec4(planned, rowptr, col, val, np, ps, pl, pt, int(F), H, ldH, Y, ldY, sc, ldS, cap, ovf, ep, rb, st);
+    dispatch_vec4<false>(planned, rowptr, col, val, np, ps, pl, pt, int(F), H, ldH, Y, ldY, sc, ldS, cap, ovf, ep, rb, st);
+  else if (in_vec4)
+    dispatch_vec4<true>(planned, rowptr, col, val, np, ps, pl, pt, int(F), H, ldH, Y, ldY, sc, ldS, cap, ovf, ep, rb, st);
   else
     dispatch_scalar(planned, rowptr, col, val, np, ps, pl, pt, int(F), H, ldH, Y, ldY, sc, ldS, cap, ovf, ep, rb, st);
   int rc = gc::check_launch("gc_spmm_csr_f32 (pieces)");

@@ -75,6 +75,10 @@ int64_t gc_spmm_default_panel_cols(int64_t K, int64_t F);
 /* Default segment length for a matrix of nnz non-zeros: a power of two in
  * [128, GC_SPMM_SEGMENT_MAX], about nnz / 8192. */
 int64_t gc_spmm_default_segment(int64_t nnz);
+/* dst[r, c] = src[r, c] for rows x cols floats, zeros in the columns cols .. ld_dst - 1 (ld_dst a multiple of 4, dst
+ * 16-byte aligned): gives a matrix with unaligned rows the pitch that vector gathers need. */
+int gc_pad_rows_f32(const float* src, int64_t ld_src, float* dst, int64_t ld_dst, int64_t rows, int64_t cols,
+                    void* stream);
 /* Segment length for a plan that serves products of feature width F: in
  * [128, GC_SPMM_SEGMENT_MAX], growing with the square root of nnz.  Shorter than
  * the default above on large matrices, where it bounds the time of the longest
@@ -250,6 +254,7 @@ int gc_spmm_csr_f32_noalloc(const int32_t* rowptr, const int32_t* col, const flo
                                   GC_PREC_TF32, which reads the fp32 operands in place
                                   (gc_gemm_resolve_precision tells which) */
 
+#define GC_EPI_H_PADDED 8 /* gc_spmm_csr_f32: every row of H is readable up to the next multiple of 4 columns */
 #define GC_EPI_TRANSPOSED_OUT 4 /* store C transposed: C is N x M with leading dimension ldc (mask likewise) */
 
 size_t gc_gemm_workspace_bytes(int transA, int transB, int64_t M, int64_t N, int64_t K, int precision);
