@@ -63,6 +63,8 @@ SIGNATURES = {
                                             _i64, _int, _f32p, _i64, _f32p, _i64, _f32p, _i64, _f32p, _i64, _void,
                                             _i64, _i64, _i64, _int, _void, _size, _void]),
     "gc_relu_backward_f32": (_int, [_f32p, _i64, _f32p, _i64, _f32p, _i64, _i64, _i64, _void]),
+    "gc_relu_bias_backward_workspace_bytes": (_size, [_i64, _i64]),
+    "gc_relu_bias_backward_f32": (_int, [_f32p, _i64, _f32p, _i64, _f32p, _i64, _i64, _i64, _f32p, _void, _size, _void]),
     "gc_mask_mul_f32": (_int, [_f32p, _i64, _f32p, _i64, _f32p, _i64, _i64, _i64, _void]),
     "gc_transpose_f32": (_int, [_f32p, _i64, _f32p, _i64, _i64, _i64, _void]),
     "gc_nll_workspace_bytes": (_size, [_i64]),

@@ -563,27 +563,32 @@ transpose_kernel(const float* __restrict__ in, int64_t ldin, float* __restrict__
   }
 }
 
-// C = sum over splits of partial[split], then the epilogue.  The order of the additions is fixed (eight
-// contiguous groups of splits summed in split order by eight warps, the eight group sums added in group order), so
-// the result is the same run to run; the groups run side by side because a capped-chain product has a thousand
-// partial tiles and one thread per element walking them all was latency-bound (0.22 ms for a 100 x 256 result).
+// C = sum over splits of partial[split], then the epilogue.  The order of the additions is fixed (G contiguous groups of
+// splits summed in split order side by side, the G group sums added in group order), so the result is the same run to
+// run; the groups run side by side because a capped-chain product has a thousand partial tiles and one thread per
+// element walking them all was latency-bound (0.22 ms for a 100 x 256 result; 17 us for the 1184 partial rows of a
+// 256-wide bias gradient with 8 groups, 5 us with 32).
+template <int G>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(int M, int N, int splits, const float* __restrict__ partial, float* __restrict__ C,
-                        int64_t ldc, gc::GemmEpilogue ep) {
-  __shared__ float sm[8][32];
-  const int e = threadIdx.x % 32, g = threadIdx.x / 32;
+                     int64_t ldc, gc::GemmEpilogue ep) {
+  constexpr int E = 256 / G;  // elements per CTA pass
+  __shared__ float sm[G][E];
+  const int e = threadIdx.x % E, g = threadIdx.x / E;
   const int64_t total = int64_t(M) * N;
-  const int per = (splits + 7) / 8;
-  const int z0 = g * per, z1 = min(splits, z0 + per);
-  for (int64_t base = int64_t(blockIdx.x) * 32; base < total; base += int64_t(gridDim.x) * 32) {
+  const int per = (splits + G - 1) / G;
+  const int z0 = min(splits, g * per), z1 = min(splits, z0 + per);
+  for (int64_t base = int64_t(blockIdx.x) * E; base < total; base += int64_t(gridDim.x) * E) {
     const int64_t i = base + e;
     float s = 0.f;
     if (i < total) {
       int z = z0;
-      for (; z + 4 <= z1; z += 4) {
-        const float a = partial[int64_t(z) * total + i], b = partial[int64_t(z + 1) * total + i],
-                    c = partial[int64_t(z + 2) * total + i], d = partial[int64_t(z + 3) * total + i];
-        s = (((s + a) + b) + c) + d;
+      for (; z + 8 <= z1; z += 8) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = partial[int64_t(z + k) * total + i];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += v[k];
       }
       for (; z < z1; ++z) s += partial[int64_t(z) * total + i];
     }
@@ -592,7 +597,7 @@ splitk_reduce_kernel(int M, int N, int splits, const float* __restrict__ partial
     if (g == 0 && i < total) {
       float t = sm[0][e];
 #pragma unroll
-      for (int k = 1; k < 8; ++k) t += sm[k][e];
+      for (int k = 1; k < G; ++k) t += sm[k][e];
       gc::epilogue_store(t, int(i / N), int(i % N), C, ldc, ep);
     }
     __syncthreads();
@@ -813,8 +818,13 @@ namespace gc {
 
 int splitk_reduce(int M, int N, int splits, const float* partial, float* C, int64_t ldc, const GemmEpilogue& ep,
                   cudaStream_t st) {
-  const unsigned g = unsigned(std::min<int64_t>(ceil_div(int64_t(M) * N, 32), kNumSMs * 8));
-  splitk_reduce_kernel<<<g, 256, 0, st>>>(M, N, splits, partial, C, ldc, ep);
+  // few elements and many splits: more groups side by side (rows of 32 bytes instead of 128 are read from the L2)
+  const int64_t total = int64_t(M) * N;
+  if (splits >= 64 && total <= 32 * kNumSMs)
+    splitk_reduce_kernel<32><<<unsigned(ceil_div(total, 8)), 256, 0, st>>>(M, N, splits, partial, C, ldc, ep);
+  else
+    splitk_reduce_kernel<8><<<unsigned(std::min<int64_t>(ceil_div(total, 32), kNumSMs * 8)), 256, 0, st>>>(
+        M, N, splits, partial, C, ldc, ep);
   return check_launch("split-K reduce");
 }
 

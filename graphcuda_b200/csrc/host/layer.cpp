@@ -184,6 +184,25 @@ Tensor relu_backward(const Tensor& dYin, const Tensor& Yin) {
   return G;
 }
 
+// The column sums of G; with Y, G is first multiplied by (Y > 0), in the same pass.
+static Tensor bias_gradient(Tensor& G, const Tensor& Yin) {
+  const int64_t M = G.size(0), N = G.size(1);
+  const at::Device dev = G.device();
+  Tensor db = at::empty({N}, at::TensorOptions().dtype(at::kFloat).device(dev));
+  const Scratch ws = scratch(kSpmm, abi.gc_relu_bias_backward_workspace_bytes(M, N), dev);
+  const Tensor dY = row_major(G);
+  const bool masked = Yin.defined();
+  const Tensor Y = masked ? row_major(Yin) : Tensor();
+  Tensor out = masked ? empty_f32(M, N, dev) : Tensor();
+  check(abi.gc_relu_bias_backward_f32(dY.const_data_ptr<float>(), ld_of(dY), masked ? Y.const_data_ptr<float>() : nullptr,
+                                      masked ? ld_of(Y) : 0, masked ? out.data_ptr<float>() : nullptr,
+                                      std::max<int64_t>(N, 1), M, N, db.data_ptr<float>(), ws.ptr, ws.bytes,
+                                      stream_of(dev)),
+        "gc_relu_bias_backward_f32");
+  if (masked) G = out;
+  return db;
+}
+
 Tensor mask_mul(const Tensor& dYin, const Tensor& maskin) {
   require(dYin.sizes() == maskin.sizes() && dYin.is_cuda() && maskin.is_cuda(), "mask_mul: shape/device mismatch");
   const Tensor dY = row_major(dYin), mask = row_major(maskin);
@@ -207,12 +226,12 @@ Grads layer_backward(Tensor G, const Tensor& X, Adj& a, const Tensor& W, bool re
                      bool gate_dx) {
   const c10::cuda::CUDAGuard guard(X.device());
   if (G.stride(1) != 1) G = G.contiguous();  // rows may keep a larger pitch (a padded gradient from the fused loss)
-  if (relu && !grad_is_gated) G = relu_backward(G, Y);
   Grads r;
+  if (need_db) r.db = bias_gradient(G, relu && !grad_is_gated ? Y : Tensor());
+  else if (relu && !grad_is_gated) G = relu_backward(G, Y);
   Epi gate;
   const bool fused_gate = gate_dx && need_dX && X.is_contiguous();
   if (fused_gate) gate.gate = X.const_data_ptr<float>();
-  if (need_db) r.db = G.sum(0);
   const int64_t out_dim = W.size(1);
   if (inter.defined()) {
     if (need_dW) r.dW = product(inter, G, true, false, prec, Epi{});

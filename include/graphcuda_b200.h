@@ -336,6 +336,11 @@ int gc_gcn_conv_backward_csr_f32(const int32_t* rowptr, const int32_t* col, cons
  * the mask re-derived from the saved activation instead of a stored fp32 mask). */
 int gc_relu_backward_f32(const float* dY, int64_t lddy, const float* Y, int64_t ldy,
                          float* G, int64_t ldg, int64_t M, int64_t N, void* stream);
+/* The same, and db[n] = sum over the rows of G[:, n] (the bias gradient) from the same pass.  Y null: no ReLU -- db
+ * sums dY and G is not touched.  Fixed order of additions. */
+size_t gc_relu_bias_backward_workspace_bytes(int64_t M, int64_t N);
+int gc_relu_bias_backward_f32(const float* dY, int64_t lddy, const float* Y, int64_t ldy, float* G, int64_t ldg,
+                              int64_t M, int64_t N, float* db, void* workspace, size_t workspace_bytes, void* stream);
 /* G = dY * mask for a stored fp32 mask (reference gcn.cu:36 verbatim). */
 int gc_mask_mul_f32(const float* dY, int64_t lddy, const float* mask, int64_t ldm,
                     float* G, int64_t ldg, int64_t M, int64_t N, void* stream);
