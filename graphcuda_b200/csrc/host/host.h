@@ -37,7 +37,7 @@ inline void require(bool cond, const char* msg) {
   X(gc_spmm_scratch_bytes) X(gc_spmm_csr_f32) X(gc_spmm_csr_bf16h_f32) X(gc_gemm_workspace_bytes) X(gc_gemm_f32)    \
   X(gc_convert_f32_bf16) X(gc_gemm_bf16_workspace_bytes) X(gc_gemm_bf16_f32) X(gc_relu_backward_f32)                \
   X(gc_mask_mul_f32) X(gc_nll_workspace_bytes) X(gc_logsoftmax_nll_forward_f32) X(gc_logsoftmax_nll_backward_f32)   \
-  X(gc_argmax_accuracy_f32) X(gc_adam_step_f32) X(gc_sgd_step_f32) X(gc_csr_is_symmetric) X(gc_pad_rows_f32)                         \
+  X(gc_argmax_accuracy_masks_f32) X(gc_logsoftmax_nll_backward_pad_f32) X(gc_adam_step_f32) X(gc_sgd_step_f32) X(gc_csr_is_symmetric) X(gc_pad_rows_f32)                         \
   X(gc_relu_bias_backward_workspace_bytes) X(gc_relu_bias_backward_f32)
 struct Abi {
 #define X(name) decltype(&::name) name = nullptr;

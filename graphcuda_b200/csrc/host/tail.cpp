@@ -41,19 +41,18 @@ struct NllFunction : torch::autograd::Function<NllFunction> {
     const int64_t ldz = M > 1 ? Z.stride(0) : std::max<int64_t>(C, 1);
     int64_t lddz = std::max<int64_t>(C, 1);
     Tensor dZ;
-    if (M > 1 && C < ldz && ldz <= C + 3 && ldz % 4 == 0) {
+    if (M > 1 && C < ldz && ldz <= C + 3 && ldz % 4 == 0 && reinterpret_cast<uintptr_t>(Z.data_ptr()) % 16 == 0) {
       // The logits are a view of a matrix padded to 16-byte rows (an odd class count): give the gradient the same
       // pitch with zero pad columns, so the layer below can aggregate it without re-padding a copy.
       lddz = ldz;
       Tensor buf = empty_f32(M, ldz, dev);
-      buf.narrow(1, C, ldz - C).zero_();
       register_zero_padded(buf);
       dZ = buf.narrow(1, 0, C);
     } else {
       dZ = empty_f32(M, C, dev);
     }
     const Tensor g = grads[0].to(at::kFloat).contiguous();
-    check(abi.gc_logsoftmax_nll_backward_f32(
+    check((lddz == C ? abi.gc_logsoftmax_nll_backward_f32 : abi.gc_logsoftmax_nll_backward_pad_f32)(
               Z.const_data_ptr<float>(), ldz, labels.const_data_ptr<int64_t>(),
               mask8.defined() ? static_cast<const uint8_t*>(mask8.data_ptr()) : nullptr, M, C,
               float(ctx->saved_data["scale"].toDouble()), g.const_data_ptr<float>(), dZ.data_ptr<float>(), lddz,
@@ -91,21 +90,21 @@ std::pair<Tensor, Tensor> argmax_accuracy(const Tensor& logits, const OptTensor&
   const at::Device dev = Z.device();
   const c10::cuda::CUDAGuard guard(dev);
   const bool labelled = labels_in && labels_in->defined();
-  Tensor labels, mask_mat;
-  int n_masks = 0;
+  Tensor labels;
+  std::vector<Tensor> rows;
+  const uint8_t* list[8] = {};
   if (masks) {
     require(labelled, "argmax_accuracy: masks need labels");
     require(masks->size() >= 1 && masks->size() <= 8, "argmax_accuracy: between 1 and 8 row selections");
-    std::vector<Tensor> rows;
     for (const Tensor& m : *masks) {
       require(m.numel() == M && m.device() == dev,
               "argmax_accuracy: every selection needs one entry per row, on the logits' device");
-      const Tensor flat = m.reshape({M});
-      rows.push_back(m.scalar_type() == at::kBool ? flat : flat.ne(0));
+      const bool bytes = m.scalar_type() == at::kBool || m.scalar_type() == at::kByte;
+      rows.push_back((bytes ? m : m.ne(0)).contiguous());
+      list[rows.size() - 1] = static_cast<const uint8_t*>(rows.back().data_ptr());
     }
-    mask_mat = at::stack(rows);
-    n_masks = int(rows.size());
   }
+  const int n_masks = int(rows.size());
   if (labelled) {
     require(labels_in->scalar_type() == at::kLong && labels_in->numel() == M && labels_in->device() == dev,
             "argmax_accuracy: labels must be int64 [M] on the logits' device");
@@ -115,9 +114,9 @@ std::pair<Tensor, Tensor> argmax_accuracy(const Tensor& logits, const OptTensor&
   const auto i64 = at::TensorOptions().dtype(at::kLong).device(dev);
   if (want_pred) pred = at::empty({M}, i64);
   if (labelled) counts = at::empty({std::max(n_masks, 1), 2}, i64);
-  check(abi.gc_argmax_accuracy_f32(Z.const_data_ptr<float>(), M > 1 ? Z.stride(0) : std::max<int64_t>(C, 1), M, C,
+  check(abi.gc_argmax_accuracy_masks_f32(Z.const_data_ptr<float>(), M > 1 ? Z.stride(0) : std::max<int64_t>(C, 1), M, C,
                                    labelled ? labels.const_data_ptr<int64_t>() : nullptr,
-                                   n_masks ? static_cast<const uint8_t*>(mask_mat.data_ptr()) : nullptr, n_masks,
+                                   list, n_masks,
                                    want_pred ? pred.data_ptr<int64_t>() : nullptr,
                                    labelled ? counts.data_ptr<int64_t>() : nullptr, stream_of(dev)),
         "gc_argmax_accuracy_f32");

@@ -367,6 +367,11 @@ int gc_logsoftmax_nll_forward_f32(const float* Z, int64_t ldz, const int64_t* la
 int gc_logsoftmax_nll_backward_f32(const float* Z, int64_t ldz, const int64_t* labels, const uint8_t* row_mask,
                                    int64_t M, int64_t C, float scale, const float* grad_loss,
                                    float* dZ, int64_t lddz, const void* workspace, void* stream);
+/* The same into rows whose pad up to the next multiple of 4 columns is dZ's own: zeros are written there (Z and dZ
+ * 16-byte aligned, both pitches multiples of 4). */
+int gc_logsoftmax_nll_backward_pad_f32(const float* Z, int64_t ldz, const int64_t* labels, const uint8_t* row_mask,
+                                   int64_t M, int64_t C, float scale, const float* grad_loss,
+                                   float* dZ, int64_t lddz, const void* workspace, void* stream);
 
 /*
  * Evaluation tail of the reference's script (tests/gcn/graphcuda_impl.py:63-68:
@@ -382,6 +387,10 @@ int gc_logsoftmax_nll_backward_f32(const float* Z, int64_t ldz, const int64_t* l
  */
 int gc_argmax_accuracy_f32(const float* Z, int64_t ldz, int64_t M, int64_t C, const int64_t* labels,
                            const uint8_t* masks, int n_masks, int64_t* pred, int64_t* counts, void* stream);
+/* The same with each selection in its own buffer (masks[0 .. n_masks - 1], M bytes each; n_masks 0: all rows). */
+int gc_argmax_accuracy_masks_f32(const float* Z, int64_t ldz, int64_t M, int64_t C, const int64_t* labels,
+                                 const uint8_t* const* masks, int n_masks, int64_t* pred, int64_t* counts,
+                                 void* stream);
 
 /* ---- optimizer step (reference tests/gcn/graphcuda_impl.py:45,56) --------- */
 
