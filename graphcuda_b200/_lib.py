@@ -82,6 +82,11 @@ SIGNATURES = {
     "gc_coo_rows_to_rowptr": (_int, [_i64p, _i64, _i64, _i32p, _void]),
     "gc_narrow_i64_i32": (_int, [_i64p, _i32p, _i64, _void]),
     "gc_gcn_norm_f32": (_int, [_i64p, _i64p, _i64, _i64, _f32p, _f32p, _void]),
+    "gc_edges_workspace_bytes": (_size, [_i64, _i64, _int]),
+    "gc_edges_sort": (_int, [_i64p, _i64p, _i64, _i64, _int, _i32p, _void, _size, _void, _void, _void]),
+    "gc_edges_to_csr": (_int, [_i64, _i64, _int, _int, _void, _size, _i32p, _i32p, _f32p, _void]),
+    "gc_degree_order_workspace_bytes": (_size, [_i64]),
+    "gc_degree_order": (_int, [_i64p, _i64, _i64, _i64p, _i64p, _i32p, _void, _size, _void]),
     "gc_csr_build_workspace_bytes": (_size, [_i64]),
     "gc_csr_count_unique": (_int, [_i64p, _i64p, _i64, _i32p, _i64p, _void, _size, _void]),
     "gc_csr_fill": (_int, [_i64p, _i64p, _f32p, _i64, _i64, _i32p, _i32p, _i32p, _f32p, _void]),

@@ -312,19 +312,20 @@ def degree_order(edge_index: torch.Tensor, num_nodes: int):
     the rows of a feature matrix that most gathers hit are contiguous."""
     _require(edge_index.dtype == torch.int64 and edge_index.dim() == 2 and edge_index.size(0) == 2,
              "edge_index must be an int64 [2, E] tensor")
-    deg = torch.bincount(edge_index[1], minlength=num_nodes)
-    perm = torch.argsort(deg, descending=True, stable=True)
-    inv = torch.empty_like(perm)
-    inv[perm] = torch.arange(num_nodes, device=perm.device, dtype=perm.dtype)
-    return perm, inv
+    if not edge_index.is_cuda:
+        deg = torch.bincount(edge_index[1], minlength=num_nodes)
+        perm = torch.argsort(deg, descending=True, stable=True)
+        inv = torch.empty_like(perm)
+        inv[perm] = torch.arange(num_nodes, device=perm.device, dtype=perm.dtype)
+        return perm, inv
+    return _lib.host.degree_order(edge_index, num_nodes, False)[:2]
 
 
 def normalized_adjacency(edge_index: torch.Tensor, num_nodes: int, *, add_self_loops: bool = True,
                          symmetric: Optional[bool] = None, reorder: Optional[str] = None) -> CSRAdjacency:
     """Edge list -> (+self-loops) -> symmetric normalisation -> coalesced int32
     CSR, the whole preprocessing of tests/gcn/graphcuda_impl.py:27-38 on the
-    GPU.  The (row, col) ordering uses torch.sort on the device; degree,
-    normalisation, de-duplication and CSR assembly are this library's kernels.
+    GPU (gc_edges_sort, gc_edges_to_csr).
 
     reorder="degree": the vertices are first relabelled by decreasing degree
     (degree_order); the result is the adjacency of the relabelled graph and
@@ -334,35 +335,11 @@ def normalized_adjacency(edge_index: torch.Tensor, num_nodes: int, *, add_self_l
     """
     _require(edge_index.is_cuda and edge_index.dtype == torch.int64, "edge_index must be a CUDA int64 tensor")
     _require(reorder in (None, "degree"), "reorder must be None or 'degree'")
+    perm = inv = relabel = None
     if reorder == "degree":
-        perm, inv = degree_order(edge_index, num_nodes)  # self-loops add one to every degree: same order
-        adj = normalized_adjacency(inv[edge_index], num_nodes, add_self_loops=add_self_loops, symmetric=symmetric)
-        adj.perm, adj.inv_perm = perm, inv
-        return adj
-    dev = edge_index.device
-    if add_self_loops:
-        loops = torch.arange(num_nodes, device=dev, dtype=torch.int64)
-        edge_index = torch.cat([edge_index, torch.stack([loops, loops])], dim=1)
-    w = gcn_norm(edge_index, num_nodes)
-    key = edge_index[0] * num_nodes + edge_index[1]
-    key, order = torch.sort(key, stable=True)
-    row = edge_index[0][order].contiguous()
-    col = edge_index[1][order].contiguous()
-    w = w[order].contiguous()
-    E = row.numel()
-    L = _lib.lib()
-    head = torch.empty(max(E, 1), dtype=torch.int32, device=dev)
-    nnz_dev = torch.empty(1, dtype=torch.int64, device=dev)
-    wsb = L.gc_csr_build_workspace_bytes(E)
-    ws = torch.empty(wsb, dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
-        s = _stream(dev)
-        _lib.check(L.gc_csr_count_unique(row.data_ptr(), col.data_ptr(), E, head.data_ptr(), nnz_dev.data_ptr(),
-                                         ws.data_ptr(), wsb, s), "gc_csr_count_unique")
-        nnz = int(nnz_dev.item())
-        rowptr = torch.empty(num_nodes + 1, dtype=torch.int32, device=dev)
-        ccol = torch.empty(nnz, dtype=torch.int32, device=dev)
-        cval = torch.empty(nnz, dtype=torch.float32, device=dev)
-        _lib.check(L.gc_csr_fill(row.data_ptr(), col.data_ptr(), w.data_ptr(), E, num_nodes, head.data_ptr(),
-                                 rowptr.data_ptr(), ccol.data_ptr(), cval.data_ptr(), s), "gc_csr_fill")
-    return CSRAdjacency(rowptr, ccol, cval, (num_nodes, num_nodes), symmetric=symmetric)
+        # self-loops add one to every degree: same order
+        perm, inv, relabel = _lib.host.degree_order(edge_index, num_nodes, True)
+    rowptr, col, val = _lib.host.edges_to_csr(edge_index, num_nodes, bool(add_self_loops), relabel)
+    adj = CSRAdjacency(rowptr, col, val, (num_nodes, num_nodes), symmetric=symmetric)
+    adj.perm, adj.inv_perm = perm, inv
+    return adj

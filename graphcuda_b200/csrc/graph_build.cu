@@ -9,7 +9,10 @@
 #include "common.cuh"
 
 #include <algorithm>
+#include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
+#include <thrust/iterator/counting_iterator.h>
+#include <thrust/iterator/transform_iterator.h>
 
 namespace {
 
@@ -104,6 +107,82 @@ csr_fill_kernel(const int64_t* __restrict__ row, const int64_t* __restrict__ col
   }
 }
 
+// ---------------------------------------------------------------- edge list -> sorted keys
+// The whole construction works on one integer per edge, row << bits | col with bits = ceil(log2 N): 32-bit keys up to
+// 65536 vertices, 64-bit above.  The radix sort runs over the 2 * bits that are used (36 for 169 K vertices: 5 passes
+// of 8 bytes instead of 8 of 16 for 64-bit keys with 64-bit permutations), the weights are computed from the degrees
+// when the CSR is written instead of being carried along.
+template <typename KEY>
+__global__ void __launch_bounds__(256)
+edge_key_kernel(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E, int64_t N, int bits,
+                const int32_t* __restrict__ relabel, KEY* __restrict__ keys, int32_t* __restrict__ deg, int64_t total) {
+  for (int64_t e = int64_t(blockIdx.x) * 256 + threadIdx.x; e < total; e += int64_t(gridDim.x) * 256) {
+    int64_t r = e - E, c = r;  // beyond the edges: the self-loops
+    if (e < E) {
+      r = row[e];
+      c = col[e];
+      if (relabel) {
+        r = relabel[r];
+        c = relabel[c];
+      }
+    }
+    keys[e] = (KEY(r) << bits) | KEY(c);
+    atomicAdd(deg + c, 1);  // integer counts: exact and order-independent
+  }
+}
+
+template <typename KEY>
+struct IsHead {  // entry e opens a new (row, col)
+  const KEY* keys;
+  __host__ __device__ int32_t operator()(int64_t e) const { return e == 0 || keys[e] != keys[e - 1] ? 1 : 0; }
+};
+
+// incl[e] = number of distinct (row, col) up to e, so the head of an entry writes element incl[e] - 1 of the CSR.
+template <typename KEY>
+__global__ void __launch_bounds__(256)
+csr_from_keys_kernel(const KEY* __restrict__ keys, const int32_t* __restrict__ incl, int64_t E, int64_t N, int bits,
+                     const float* __restrict__ dinv, int32_t* __restrict__ rowptr, int32_t* __restrict__ csr_col,
+                     float* __restrict__ csr_val) {
+  const KEY low = (KEY(1) << bits) - 1;
+  for (int64_t e = int64_t(blockIdx.x) * 256 + threadIdx.x; e < E; e += int64_t(gridDim.x) * 256) {
+    const KEY k = keys[e];
+    const int64_t r = int64_t(k >> bits), c = int64_t(k & low);
+    const bool first = e == 0;
+    const KEY kp = first ? KEY(0) : keys[e - 1];
+    if (first || kp != k) {
+      const int32_t j = incl[e] - 1;
+      for (int64_t q = first ? 0 : int64_t(kp >> bits) + 1; q <= r; ++q) rowptr[q] = j;
+      // dinv[row] * 1.0f * dinv[col], left to right; duplicates are added in input order (they are equal)
+      const float w = __fmul_rn(__fmul_rn(__ldg(dinv + r), 1.0f), __ldg(dinv + c));
+      float s = w;
+      for (int64_t d = e + 1; d < E && keys[d] == k; ++d) s = __fadd_rn(s, w);
+      csr_col[j] = int32_t(c);
+      csr_val[j] = s;
+    }
+    if (e == E - 1)
+      for (int64_t q = r + 1; q <= N; ++q) rowptr[q] = incl[e];
+  }
+}
+
+// Keys of the degree order: decreasing degree, ties by vertex (the sort is stable).
+__global__ void __launch_bounds__(256)
+degree_key_kernel(const int32_t* __restrict__ deg, uint32_t* __restrict__ keys, int32_t* __restrict__ ids, int64_t N) {
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < N; i += int64_t(gridDim.x) * 256) {
+    keys[i] = ~uint32_t(deg[i]);
+    ids[i] = int32_t(i);
+  }
+}
+__global__ void __launch_bounds__(256)
+degree_perm_kernel(const int32_t* __restrict__ ids, int64_t N, int64_t* __restrict__ perm, int64_t* __restrict__ inv,
+                   int32_t* __restrict__ relabel) {
+  for (int64_t i = int64_t(blockIdx.x) * 256 + threadIdx.x; i < N; i += int64_t(gridDim.x) * 256) {
+    const int32_t v = ids[i];
+    perm[i] = v;
+    inv[v] = i;
+    if (relabel) relabel[v] = int32_t(i);
+  }
+}
+
 __global__ void set_one_kernel(int32_t* out) { *out = 1; }
 
 // One warp per row; every entry (i, j, v) looks for (j, i) by bisection of
@@ -132,6 +211,15 @@ symmetric_kernel(const int32_t* __restrict__ rowptr, const int32_t* __restrict__
     }
   }
 }
+
+inline int id_bits(int64_t N) {
+  int b = 1;
+  while ((int64_t(1) << b) < N) ++b;
+  return b;
+}
+inline size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
+// Temporary storage of the sorts and scans, by formula so that it is the same without a GPU.
+inline size_t cub_bytes(int64_t n) { return (size_t(4) << 20) + size_t(n) / 4; }
 
 inline unsigned grid_for(int64_t n) {
   return unsigned(std::max<int64_t>(1, std::min<int64_t>(gc::ceil_div(n, 256), gc::kNumSMs * 16)));
@@ -169,6 +257,137 @@ int gc_gcn_norm_f32(const int64_t* row, const int64_t* col, int64_t E, int64_t N
   dinv_kernel<<<grid_for(N), 256, 0, st>>>(deg, N);
   norm_weight_kernel<<<grid_for(E), 256, 0, st>>>(row, col, E, deg_scratch, w);
   return gc::check_launch("gc_gcn_norm_f32", 3);
+}
+
+}  // extern "C"
+
+namespace {
+// Workspace: [keys][keys, other buffer][running counts][degrees, then their -1/2 powers][temporary storage]
+struct EdgeWs {
+  char *keys, *alt;
+  int32_t *incl, *deg;
+  void* cub;
+  size_t cub_bytes, total;
+};
+EdgeWs edge_ws(void* ws, int64_t total, int64_t N) {
+  EdgeWs w{};
+  char* p = static_cast<char*>(ws);
+  size_t off = 0;
+  auto take = [&](size_t bytes) {
+    char* q = p ? p + off : nullptr;
+    off += up256(bytes);
+    return q;
+  };
+  const size_t kb = (2 * id_bits(N) <= 32 ? 4 : 8) * size_t(std::max<int64_t>(total, 1));
+  w.keys = take(kb);
+  w.alt = take(kb);
+  w.incl = reinterpret_cast<int32_t*>(take(size_t(std::max<int64_t>(total, 1)) * 4));
+  w.deg = reinterpret_cast<int32_t*>(take(size_t(std::max<int64_t>(N, 1)) * 4));
+  w.cub_bytes = cub_bytes(total);
+  w.cub = take(w.cub_bytes);
+  w.total = off;
+  return w;
+}
+
+template <typename KEY>
+int sort_edges(const int64_t* row, const int64_t* col, int64_t E, int64_t N, int64_t total, const int32_t* relabel,
+               const EdgeWs& w, int* selector, cudaStream_t st) {
+  const int bits = id_bits(N);
+  KEY *k0 = reinterpret_cast<KEY*>(w.keys), *k1 = reinterpret_cast<KEY*>(w.alt);
+  edge_key_kernel<KEY><<<grid_for(total), 256, 0, st>>>(row, col, E, N, bits, relabel, k0, w.deg, total);
+  dinv_kernel<<<grid_for(N), 256, 0, st>>>(w.deg, N);
+  cub::DoubleBuffer<KEY> db(k0, k1);
+  size_t need = 0;
+  cudaError_t e = cub::DeviceRadixSort::SortKeys(nullptr, need, db, int(total), 0, 2 * bits, st);
+  if (e == cudaSuccess && need > w.cub_bytes)
+    return gc::fail(GC_ERR_WORKSPACE, "gc_edges_sort: sort needs %zu bytes of temporary storage", need);
+  need = w.cub_bytes;
+  if (e == cudaSuccess) e = cub::DeviceRadixSort::SortKeys(w.cub, need, db, int(total), 0, 2 * bits, st);
+  if (e != cudaSuccess) return gc::fail(GC_ERR_CUDA, "gc_edges_sort: sort: %s", cudaGetErrorString(e));
+  *selector = db.selector;
+  auto heads = thrust::make_transform_iterator(thrust::counting_iterator<int64_t>(0), IsHead<KEY>{db.Current()});
+  e = cub::DeviceScan::InclusiveSum(nullptr, need, heads, w.incl, int(total), st);
+  if (e == cudaSuccess && need > w.cub_bytes)
+    return gc::fail(GC_ERR_WORKSPACE, "gc_edges_sort: scan needs %zu bytes of temporary storage", need);
+  need = w.cub_bytes;
+  if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(w.cub, need, heads, w.incl, int(total), st);
+  if (e != cudaSuccess) return gc::fail(GC_ERR_CUDA, "gc_edges_sort: scan: %s", cudaGetErrorString(e));
+  return gc::check_launch("gc_edges_sort", 4);
+}
+}  // namespace
+
+extern "C" {
+
+size_t gc_edges_workspace_bytes(int64_t E, int64_t N, int self_loops) {
+  if (E < 0 || N < 0) return 0;
+  return edge_ws(nullptr, E + (self_loops ? N : 0), N).total;
+}
+
+int gc_edges_sort(const int64_t* row, const int64_t* col, int64_t E, int64_t N, int self_loops, const int32_t* relabel,
+                  void* workspace, size_t workspace_bytes, int* selector, const int32_t** nnz_at, void* stream) {
+  const int64_t total = E + (self_loops ? N : 0);
+  GC_REQUIRE(E >= 0 && N >= 0 && total < INT32_MAX, "gc_edges_sort: size out of int32 range");
+  GC_REQUIRE(total > 0 && (E == 0 || (row && col)) && workspace && selector && nnz_at, "gc_edges_sort: null pointer");
+  const EdgeWs w = edge_ws(workspace, total, N);
+  if (workspace_bytes < w.total) return gc::fail(GC_ERR_WORKSPACE, "gc_edges_sort: workspace too small");
+  cudaStream_t st = gc::as_stream(stream);
+  if (cudaMemsetAsync(w.deg, 0, size_t(N) * 4, st) != cudaSuccess)
+    return gc::fail(GC_ERR_CUDA, "gc_edges_sort: clearing the degrees failed");
+  *nnz_at = w.incl + total - 1;
+  return 2 * id_bits(N) <= 32 ? sort_edges<uint32_t>(row, col, E, N, total, relabel, w, selector, st)
+                              : sort_edges<uint64_t>(row, col, E, N, total, relabel, w, selector, st);
+}
+
+int gc_edges_to_csr(int64_t E, int64_t N, int self_loops, int selector, const void* workspace, size_t workspace_bytes,
+                    int32_t* rowptr, int32_t* csr_col, float* csr_val, void* stream) {
+  const int64_t total = E + (self_loops ? N : 0);
+  GC_REQUIRE(E >= 0 && N >= 0 && total > 0 && total < INT32_MAX, "gc_edges_to_csr: size out of range");
+  GC_REQUIRE(workspace && rowptr && csr_col && csr_val, "gc_edges_to_csr: null pointer");
+  const EdgeWs w = edge_ws(const_cast<void*>(workspace), total, N);
+  if (workspace_bytes < w.total) return gc::fail(GC_ERR_WORKSPACE, "gc_edges_to_csr: workspace too small");
+  cudaStream_t st = gc::as_stream(stream);
+  const int bits = id_bits(N);
+  const char* k = selector ? w.alt : w.keys;
+  const float* dinv = reinterpret_cast<const float*>(w.deg);
+  if (2 * bits <= 32)
+    csr_from_keys_kernel<uint32_t><<<grid_for(total), 256, 0, st>>>(reinterpret_cast<const uint32_t*>(k), w.incl, total, N,
+                                                                   bits, dinv, rowptr, csr_col, csr_val);
+  else
+    csr_from_keys_kernel<uint64_t><<<grid_for(total), 256, 0, st>>>(reinterpret_cast<const uint64_t*>(k), w.incl, total, N,
+                                                                   bits, dinv, rowptr, csr_col, csr_val);
+  return gc::check_launch("gc_edges_to_csr");
+}
+
+size_t gc_degree_order_workspace_bytes(int64_t N) {
+  if (N < 0) return 0;
+  return 5 * up256(size_t(std::max<int64_t>(N, 1)) * 4) + up256(cub_bytes(N));
+}
+
+int gc_degree_order(const int64_t* target, int64_t E, int64_t N, int64_t* perm, int64_t* inv, int32_t* relabel,
+                    void* workspace, size_t workspace_bytes, void* stream) {
+  GC_REQUIRE(E >= 0 && N >= 0 && N < INT32_MAX, "gc_degree_order: size out of range");
+  if (N == 0) return GC_OK;
+  GC_REQUIRE((E == 0 || target) && perm && inv && workspace, "gc_degree_order: null pointer");
+  if (workspace_bytes < gc_degree_order_workspace_bytes(N))
+    return gc::fail(GC_ERR_WORKSPACE, "gc_degree_order: workspace too small");
+  cudaStream_t st = gc::as_stream(stream);
+  const size_t b = up256(size_t(N) * 4);
+  char* p = static_cast<char*>(workspace);
+  int32_t* deg = reinterpret_cast<int32_t*>(p);
+  cub::DoubleBuffer<uint32_t> dk(reinterpret_cast<uint32_t*>(p + b), reinterpret_cast<uint32_t*>(p + 2 * b));
+  cub::DoubleBuffer<int32_t> dv(reinterpret_cast<int32_t*>(p + 3 * b), reinterpret_cast<int32_t*>(p + 4 * b));
+  size_t have = cub_bytes(N), need = 0;
+  if (cudaMemsetAsync(deg, 0, size_t(N) * 4, st) != cudaSuccess)
+    return gc::fail(GC_ERR_CUDA, "gc_degree_order: clearing the degrees failed");
+  if (E > 0) degree_kernel<<<grid_for(E), 256, 0, st>>>(target, E, deg);
+  degree_key_kernel<<<grid_for(N), 256, 0, st>>>(deg, dk.Current(), dv.Current(), N);
+  cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, need, dk, dv, int(N), 0, 32, st);
+  if (e == cudaSuccess && need > have)
+    return gc::fail(GC_ERR_WORKSPACE, "gc_degree_order: sort needs %zu bytes of temporary storage", need);
+  if (e == cudaSuccess) e = cub::DeviceRadixSort::SortPairs(p + 5 * b, have, dk, dv, int(N), 0, 32, st);
+  if (e != cudaSuccess) return gc::fail(GC_ERR_CUDA, "gc_degree_order: sort: %s", cudaGetErrorString(e));
+  degree_perm_kernel<<<grid_for(N), 256, 0, st>>>(dv.Current(), N, perm, inv, relabel);
+  return gc::check_launch("gc_degree_order", 4);
 }
 
 size_t gc_csr_build_workspace_bytes(int64_t E) {

@@ -224,6 +224,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("csr", &make_csr);
   m.def("dense", &make_dense);
 
+  m.def("degree_order", &degree_order, NoGil());
+  m.def("edges_to_csr", &edges_to_csr, NoGil());
+
   m.def("padded_width", &padded_width);
   m.def("zero_padded_base", &zero_padded_base);
   m.def("register_zero_padded", &register_zero_padded);

@@ -248,4 +248,51 @@ void spmm_into(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, 
           "gc_spmm_csr_f32");
 }
 
+// ------------------------------------------------------------------ graphs
+// (perm, inv, int32 inv) of the order by decreasing number of incoming edges.
+std::tuple<Tensor, Tensor, Tensor> degree_order(const Tensor& edge_index, int64_t n, bool want_relabel) {
+  const at::Device dev = edge_index.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const Tensor target = edge_index.select(0, 1).contiguous();
+  const auto i64 = at::TensorOptions().dtype(at::kLong).device(dev);
+  Tensor perm = at::empty({n}, i64), inv = at::empty({n}, i64), relabel;
+  if (want_relabel) relabel = at::empty({n}, i64.dtype(at::kInt));
+  const size_t wsb = abi.gc_degree_order_workspace_bytes(n);
+  Tensor ws = bytes_on(wsb, dev);
+  check(abi.gc_degree_order(target.const_data_ptr<int64_t>(), target.numel(), n, perm.data_ptr<int64_t>(),
+                            inv.data_ptr<int64_t>(), want_relabel ? relabel.data_ptr<int32_t>() : nullptr,
+                            ws.data_ptr(), wsb, stream_of(dev)),
+        "gc_degree_order");
+  return {perm, inv, relabel};
+}
+
+// (rowptr, col, val) of the normalised adjacency of an int64 [2, E] edge list.
+std::tuple<Tensor, Tensor, Tensor> edges_to_csr(const Tensor& edge_index, int64_t n, bool self_loops,
+                                                const OptTensor& relabel) {
+  const at::Device dev = edge_index.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const auto i32 = at::TensorOptions().dtype(at::kInt).device(dev);
+  const int64_t E = edge_index.size(1);
+  if (E + (self_loops ? n : 0) == 0)
+    return {at::zeros({n + 1}, i32), at::empty({0}, i32), at::empty({0}, i32.dtype(at::kFloat))};
+  const Tensor row = edge_index.select(0, 0).contiguous(), col = edge_index.select(0, 1).contiguous();
+  const size_t wsb = abi.gc_edges_workspace_bytes(E, n, self_loops);
+  Tensor ws = bytes_on(wsb, dev);
+  void* st = stream_of(dev);
+  int selector = 0;
+  const int32_t* nnz_at = nullptr;
+  check(abi.gc_edges_sort(row.const_data_ptr<int64_t>(), col.const_data_ptr<int64_t>(), E, n, self_loops,
+                          relabel ? relabel->const_data_ptr<int32_t>() : nullptr, ws.data_ptr(), wsb, &selector,
+                          &nnz_at, st),
+        "gc_edges_sort");
+  Tensor rowptr = at::empty({n + 1}, i32);
+  const int64_t at = reinterpret_cast<const char*>(nnz_at) - static_cast<const char*>(ws.data_ptr());
+  const int64_t nnz = ws.narrow(0, at, 4).view(at::kInt).item<int32_t>();  // the one host read
+  Tensor c = at::empty({nnz}, i32), v = at::empty({nnz}, i32.dtype(at::kFloat));
+  check(abi.gc_edges_to_csr(E, n, self_loops, selector, ws.data_ptr(), wsb, rowptr.data_ptr<int32_t>(),
+                            c.data_ptr<int32_t>(), v.data_ptr<float>(), st),
+        "gc_edges_to_csr");
+  return {rowptr, c, v};
+}
+
 }  // namespace gch

@@ -38,7 +38,8 @@ inline void require(bool cond, const char* msg) {
   X(gc_convert_f32_bf16) X(gc_gemm_bf16_workspace_bytes) X(gc_gemm_bf16_f32) X(gc_relu_backward_f32)                \
   X(gc_mask_mul_f32) X(gc_nll_workspace_bytes) X(gc_logsoftmax_nll_forward_f32) X(gc_logsoftmax_nll_backward_f32)   \
   X(gc_argmax_accuracy_masks_f32) X(gc_logsoftmax_nll_backward_pad_f32) X(gc_adam_step_f32) X(gc_sgd_step_f32) X(gc_csr_is_symmetric) X(gc_pad_rows_f32)                         \
-  X(gc_relu_bias_backward_workspace_bytes) X(gc_relu_bias_backward_f32)
+  X(gc_edges_workspace_bytes) X(gc_edges_sort) X(gc_edges_to_csr) X(gc_degree_order_workspace_bytes)                \
+  X(gc_degree_order) X(gc_relu_bias_backward_workspace_bytes) X(gc_relu_bias_backward_f32)
 struct Abi {
 #define X(name) decltype(&::name) name = nullptr;
   GC_HOST_FUNCTIONS(X)
@@ -125,6 +126,11 @@ using AdjPtr = c10::intrusive_ptr<Adj>;
 // Y = A H (+bias)(ReLU)(mask)(gate); H is float32 (or bfloat16) with unit column stride.
 void spmm_into(Adj& a, const Tensor& H, float* Y, int64_t ldy, const Epi& ep, bool accumulate, int64_t panel_cols);
 Tensor adj_matmul(Adj& a, Tensor H, int prec, const Epi& ep);
+
+// ------------------------------------------------------------------ graphs
+std::tuple<Tensor, Tensor, Tensor> degree_order(const Tensor& edge_index, int64_t n, bool want_relabel);
+std::tuple<Tensor, Tensor, Tensor> edges_to_csr(const Tensor& edge_index, int64_t n, bool self_loops,
+                                                const OptTensor& relabel);
 
 // ------------------------------------------------------------------ layer, loss, optimizers (layer.cpp, tail.cpp)
 struct Forward {

@@ -438,6 +438,25 @@ int gc_gcn_norm_f32(const int64_t* row, const int64_t* col, int64_t E, int64_t N
                     float* deg_scratch, float* w, void* stream);
 
 /*
+ * Edge list -> normalised CSR (tests/gcn/graphcuda_impl.py:27-38: add_self_loops, gcn_norm, coalesce) in two steps
+ * around the one size that depends on the data.  gc_edges_sort sorts the edges (and the N self-loops, when asked for)
+ * by (row, col) in the workspace, counts the degrees on the targets and leaves the number of distinct pairs at *nnz_at
+ * (a device address inside the workspace); *selector is passed on.  relabel (or null): int32[N], vertex v becomes
+ * relabel[v].  gc_edges_to_csr then writes rowptr[N+1], col[nnz], val[nnz].  Same values, bit for bit, as
+ * gc_gcn_norm_f32 on the list followed by coalescing.
+ */
+size_t gc_edges_workspace_bytes(int64_t E, int64_t N, int self_loops);
+int gc_edges_sort(const int64_t* row, const int64_t* col, int64_t E, int64_t N, int self_loops, const int32_t* relabel,
+                  void* workspace, size_t workspace_bytes, int* selector, const int32_t** nnz_at, void* stream);
+int gc_edges_to_csr(int64_t E, int64_t N, int self_loops, int selector, const void* workspace, size_t workspace_bytes,
+                    int32_t* rowptr, int32_t* csr_col, float* csr_val, void* stream);
+/* Vertices by decreasing number of edges that point at them (target[E]), ties by vertex: perm[new] = old,
+ * inv[old] = new, and the int32 copy of inv that gc_edges_sort takes (or null). */
+size_t gc_degree_order_workspace_bytes(int64_t N);
+int gc_degree_order(const int64_t* target, int64_t E, int64_t N, int64_t* perm, int64_t* inv, int32_t* relabel,
+                    void* workspace, size_t workspace_bytes, void* stream);
+
+/*
  * CSR from an edge list sorted by (row, col) with duplicates allowed:
  * duplicates are summed in input order (what coalesce() does,
  * tests/gcn/graphcuda_impl.py:33-38).  Two steps so the caller can size the
