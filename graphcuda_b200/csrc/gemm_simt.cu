@@ -18,19 +18,31 @@
 // (fma.rn.f32x2: two IEEE FMAs per issue slot), so the FMA pipe and not the
 // issue slots or the shared-memory reads set the pace.  For narrow outputs the
 // 256 threads split the k-values of a stage WK ways (a 64 x 16 tile alone would
-// keep two warps busy).  K is split further over a cluster of up to 8 CTAs that
-// add their tiles through distributed shared memory in rank order -- one launch,
-// no workspace -- and, for long sums, over gridDim.z with partial tiles in the
-// workspace and a second kernel.  Every order of additions is fixed.
+// keep two warps busy).
+//
+// Work is the list of all (tile, stage of k) units, tile by tile, and a CTA takes
+// a contiguous run of it: whole tiles when there are many, a share of one or the
+// ends of two where tiles alone would leave SMs idle or a last wave nearly empty
+// (2049 x 515 has 297 tiles of 64 x 64: one more than two per SM).  Sums of tiles
+// that ended up in several CTAs go to the workspace and a second kernel adds them
+// in CTA order.  Every order of additions is fixed.
 #include "common.cuh"
 #include "gemm_internal.cuh"
 
-#include <cooperative_groups.h>
-
-namespace cg = cooperative_groups;
-
 namespace {
 
+using u64 = unsigned long long;
+__device__ __forceinline__ u64 pack2(float a, float b) {
+  u64 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+// (c0, c1) += a * b, both halves (fma.rn.f32x2: the rounding of two fmaf)
+__device__ __forceinline__ void fma2(float& c0, float& c1, u64 a, u64 b) {
+  u64 c = pack2(c0, c1);
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c0), "=f"(c1) : "l"(c));
+}
 __device__ __forceinline__ void copy16(float* dst, const float* src, int bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(dst))),
                "l"(src), "r"(bytes) : "memory");
@@ -126,21 +138,20 @@ struct Args {
   float* C;
   int64_t ldc;
   gc::GemmEpilogue ep;
-  int k_per_split;
-  float* partial;  // [gridDim.z][M][N] or null
+  int tiles_n, stages;  // tiles along N; stages of k per tile
+  int64_t units;        // tiles * stages
+  int per_cta;          // units of a CTA
+  float* partial;       // [2 * gridDim.x][BM * BN]: the first and the last tile of a CTA, where it has only a share of it
 };
 
 template <int BM, int BN, int TM, int TN, int WK, int BK, int ST, bool TA, bool TB, bool VA, bool VB>
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(256, TM == 8 ? 2 : 3)
 gemm_simt_kernel(const __grid_constant__ Args p) {
   using T = Tile<BM, BN, TM, TN, WK, BK, ST, TA, TB>;
   using SA = typename T::SA;
   using SB = typename T::SB;
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x;
-  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
-  const int kb = blockIdx.z * p.k_per_split;
-  const int ke = min(p.K, kb + p.k_per_split);
   // a warp covers 8 threads along M (where the tile has them) x 4 along N
   constexpr int NM = BM / TM, NN = BN / TN, GROUP = NM * NN;
   constexpr int LM = NM >= 8 ? 8 : NM, LN = 32 / LM < NN ? 32 / LM : NN, PW = LM * LN;
@@ -148,212 +159,249 @@ gemm_simt_kernel(const __grid_constant__ Args p) {
   const int w = g / PW, l = g % PW;
   const int ty = (w % (NM / LM)) * LM + l % LM, tx = (w / (NM / LM)) * LN + l / LM;
 
-  float acc[TM][TN];
-#pragma unroll
-  for (int i = 0; i < TM; ++i)
-#pragma unroll
-    for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+  int64_t unit = int64_t(blockIdx.x) * p.per_cta;
+  const int64_t last_unit = min(p.units, unit + p.per_cta);
+  for (int segment = 0; unit < last_unit; ++segment) {
+    const int64_t tile = unit / p.stages;
+    const int kt0 = int(unit - tile * p.stages);
+    const int nkt = int(min(int64_t(p.stages - kt0), last_unit - unit));
+    unit += nkt;
+    const int m0 = int(tile / p.tiles_n) * BM, n0 = int(tile % p.tiles_n) * BN;
+    const int kb = kt0 * BK, ke = min(p.K, kb + nkt * BK);
 
-  const int nkt = (ke - kb + BK - 1) / BK;
-  const typename SA::template Copier<VA> copy_a(p.A, p.lda, m0, p.M, kb, ke, tid);
-  const typename SB::template Copier<VB> copy_b(p.B, p.ldb, n0, p.N, kb, ke, tid);
-  auto issue = [&](int kt) {
-    if (kt < nkt) {
-      float* s = sm + (kt % ST) * T::kStage;
-      copy_a(s, p.lda, kb + kt * BK, kt);
-      copy_b(s + SA::kFloats, p.ldb, kb + kt * BK, kt);
-    }
-    copies_commit();
-  };
+    float acc[TM][TN];
 #pragma unroll
-  for (int s = 0; s < ST - 1; ++s) issue(s);
-  for (int kt = 0; kt < nkt; ++kt) {
-    copies_wait<ST - 2>();
-    __syncthreads();
-    issue(kt + ST - 1);
-    const float* sa = sm + (kt % ST) * T::kStage;
-    const float* sb = sa + SA::kFloats;
+    for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int kk = 0; kk < BK / WK; kk += 4) {
-      float a[TM][4], b[TN][4];
-      SA::template frag<TM>(sa, ty, wk * (BK / WK) + kk, a);
-      SB::template frag<TN>(sb, tx, wk * (BK / WK) + kk, b);
+      for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+    const typename SA::template Copier<VA> copy_a(p.A, p.lda, m0, p.M, kb, ke, tid);
+    const typename SB::template Copier<VB> copy_b(p.B, p.ldb, n0, p.N, kb, ke, tid);
+    auto issue = [&](int kt) {
+      if (kt < nkt) {
+        float* s = sm + (kt % ST) * T::kStage;
+        copy_a(s, p.lda, kb + kt * BK, kt);
+        copy_b(s + SA::kFloats, p.ldb, kb + kt * BK, kt);
+      }
+      copies_commit();
+    };
+    __syncthreads();  // the previous tile's shared memory is free
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+    for (int s = 0; s < ST - 1; ++s) issue(s);
+    for (int kt = 0; kt < nkt; ++kt) {
+      copies_wait<ST - 2>();
+      __syncthreads();
+      issue(kt + ST - 1);
+      const float* sa = sm + (kt % ST) * T::kStage;
+      const float* sb = sa + SA::kFloats;
 #pragma unroll
-        for (int i = 0; i < TM; ++i)
+      for (int kk = 0; kk < BK / WK; kk += 4) {
+        float a[TM][4], b[TN][4];
+        SA::template frag<TM>(sa, ty, wk * (BK / WK) + kk, a);
+        SB::template frag<TN>(sb, tx, wk * (BK / WK) + kk, b);
+        if constexpr (TB) {  // pairs of columns are not neighbours in registers: packing them costs more than it saves
 #pragma unroll
-          for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i][q], b[j][q], acc[i][j]);
-    }
-  }
-  copies_wait<0>();
-
-  cg::cluster_group cluster = cg::this_cluster();
-  const int ranks = int(cluster.num_blocks());
-  float* partial = p.partial ? p.partial + int64_t(blockIdx.z) * p.M * p.N : nullptr;
-  if (WK == 1 && ranks == 1) {
-    const bool vec = !TB && !p.ep.transposed && !partial && (p.ldc % 4 == 0) &&
-                     (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && !p.ep.mask && !p.ep.gate;
+          for (int q = 0; q < 4; ++q)
 #pragma unroll
-    for (int i = 0; i < TM; ++i) {
-      const int gm = m0 + SA::template index<TM>(ty, i);
-      if (gm >= p.M) continue;
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int h = 0; h < TN; h += 4) {
-        float v[4] = {acc[i][h], acc[i][h + 1], acc[i][h + 2], acc[i][h + 3]};
-        const int gn = n0 + SB::template index<TN>(tx, h);
-        if (vec && gn + 4 <= p.N) {
+              for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i][q], b[j][q], acc[i][j]);
+        } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (p.ep.bias) v[j] += __ldg(p.ep.bias + gn + j);
-            if (p.ep.relu) v[j] *= v[j] > 0.f ? 1.f : 0.f;
+          for (int q = 0; q < 4; ++q) {
+            u64 bb[TN / 2];
+#pragma unroll
+            for (int j = 0; j < TN / 2; ++j) bb[j] = pack2(b[2 * j][q], b[2 * j + 1][q]);
+#pragma unroll
+            for (int i = 0; i < TM; ++i) {
+              const u64 aa = pack2(a[i][q], a[i][q]);
+#pragma unroll
+              for (int j = 0; j < TN / 2; ++j) fma2(acc[i][2 * j], acc[i][2 * j + 1], aa, bb[j]);
+            }
           }
-          *reinterpret_cast<float4*>(p.C + int64_t(gm) * p.ldc + gn) = make_float4(v[0], v[1], v[2], v[3]);
-          continue;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int n = n0 + SB::template index<TN>(tx, h + j);
-          if (n >= p.N) continue;
-          if (partial) partial[int64_t(gm) * p.N + n] = v[j];
-          else gc::epilogue_store(v[j], gm, n, p.C, p.ldc, p.ep);
         }
       }
     }
-    return;
-  }
+    copies_wait<0>();
 
-  // Sums of the WK groups, then of the cluster's CTAs, added in order.
-  __syncthreads();
+    // a share of a tile: raw sums to the workspace, row-major BM x BN
+    float* share = nkt < p.stages ? p.partial + (2 * int64_t(blockIdx.x) + (segment ? 1 : 0)) * (BM * BN) : nullptr;
+    if (WK == 1) {
+      const bool vec = !TB && !p.ep.transposed && (p.ldc % 4 == 0) && (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 &&
+                       !p.ep.mask && !p.ep.gate;
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+      for (int i = 0; i < TM; ++i) {
+        const int mi = SA::template index<TM>(ty, i), gm = m0 + mi;
 #pragma unroll
-    for (int j = 0; j < TN; ++j)
-      sm[wk * (BM * BN) + SA::template index<TM>(ty, i) * BN + SB::template index<TN>(tx, j)] = acc[i][j];
-  __syncthreads();
-  const bool last = ranks == 1;
-  for (int e = tid; e < BM * BN; e += 256) {
-    float s = sm[e];
+        for (int h = 0; h < TN; h += 4) {
+          float v[4] = {acc[i][h], acc[i][h + 1], acc[i][h + 2], acc[i][h + 3]};
+          if (share) {
 #pragma unroll
-    for (int q = 1; q < WK; ++q) s += sm[q * (BM * BN) + e];
-    if (!last) {
-      sm[e] = s;
+            for (int j = 0; j < 4; ++j) share[mi * BN + SB::template index<TN>(tx, h + j)] = v[j];
+            continue;
+          }
+          if (gm >= p.M) continue;
+          const int gn = n0 + SB::template index<TN>(tx, h);
+          if (vec && gn + 4 <= p.N) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              if (p.ep.bias) v[j] += __ldg(p.ep.bias + gn + j);
+              if (p.ep.relu) v[j] *= v[j] > 0.f ? 1.f : 0.f;
+            }
+            *reinterpret_cast<float4*>(p.C + int64_t(gm) * p.ldc + gn) = make_float4(v[0], v[1], v[2], v[3]);
+            continue;
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int n = n0 + SB::template index<TN>(tx, h + j);
+            if (n < p.N) gc::epilogue_store(v[j], gm, n, p.C, p.ldc, p.ep);
+          }
+        }
+      }
       continue;
     }
-    const int gm = m0 + e / BN, gn = n0 + e % BN;
-    if (gm >= p.M || gn >= p.N) continue;
-    if (partial) partial[int64_t(gm) * p.N + gn] = s;
-    else gc::epilogue_store(s, gm, gn, p.C, p.ldc, p.ep);
+
+    // the sums of the WK groups, added in order
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
+        sm[wk * (BM * BN) + SA::template index<TM>(ty, i) * BN + SB::template index<TN>(tx, j)] = acc[i][j];
+    __syncthreads();
+    for (int e = tid; e < BM * BN; e += 256) {
+      float s = sm[e];
+#pragma unroll
+      for (int q = 1; q < WK; ++q) s += sm[q * (BM * BN) + e];
+      const int gm = m0 + e / BN, gn = n0 + e % BN;
+      if (share) share[e] = s;
+      else if (gm < p.M && gn < p.N) gc::epilogue_store(s, gm, gn, p.C, p.ldc, p.ep);
+    }
   }
-  if (last) return;
-  cluster.sync();
-  const int rank = int(cluster.block_rank());
-  for (int e = rank * 256 + tid; e < BM * BN; e += ranks * 256) {
-    const int gm = m0 + e / BN, gn = n0 + e % BN;
-    if (gm >= p.M || gn >= p.N) continue;
+}
+
+// Adds up the shares of the tiles that several CTAs worked on.  G = 1: four elements per thread, the shares in order
+// (2049 x 515: two to four per tile).  G = 8, few tiles and long sums: 32 elements per CTA, eight contiguous groups of
+// shares side by side, the group sums in order.
+template <int BM, int BN, int G>
+__global__ void __launch_bounds__(256)
+gemm_shares_kernel(const __grid_constant__ Args p) {
+  constexpr int E = G == 1 ? 1024 : 32, kPerTile = (BM * BN + E - 1) / E;
+  const unsigned tile = blockIdx.x / kPerTile, chunk = blockIdx.x % kPerTile;
+  const unsigned long long u0 = static_cast<unsigned long long>(tile) * p.stages;
+  const int c0 = int(u0 / unsigned(p.per_cta)), c1 = int((u0 + p.stages - 1) / unsigned(p.per_cta));
+  if (c0 == c1) return;  // one CTA had all of it
+  const int m0 = int(tile / unsigned(p.tiles_n)) * BM, n0 = int(tile % unsigned(p.tiles_n)) * BN;
+  // only the first contributor can have begun with an earlier tile; every later one began with this tile
+  const bool first0 = static_cast<unsigned long long>(c0) * p.per_cta == u0;
+  if constexpr (G == 1) {
+    const int e = int(chunk) * E + int(threadIdx.x) * 4;
+    if (e >= BM * BN) return;
+    const int m = m0 + e / BN, n = n0 + e % BN;
+    if (m >= p.M || n >= p.N) return;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int c = c0; c <= c1; ++c) {
+      const int slot = (c > c0 || first0) ? 0 : 1;
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p.partial + (2 * int64_t(c) + slot) * (BM * BN) + e));
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    const float v[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (n + j < p.N) gc::epilogue_store(v[j], m, n + j, p.C, p.ldc, p.ep);
+  } else {
+    __shared__ float sm[G][32];
+    const int lane = threadIdx.x % 32, g = threadIdx.x / 32, e = int(chunk) * E + lane;
+    const int per = (c1 - c0 + G) / G;
     float s = 0.f;
-    for (int r = 0; r < ranks; ++r) s += cluster.map_shared_rank(sm, r)[e];
-    gc::epilogue_store(s, gm, gn, p.C, p.ldc, p.ep);
+    for (int c = c0 + g * per; c <= min(c1, c0 + (g + 1) * per - 1); ++c)
+      s += __ldg(p.partial + (2 * int64_t(c) + ((c > c0 || first0) ? 0 : 1)) * (BM * BN) + e);
+    sm[g][lane] = s;
+    __syncthreads();
+    const int m = m0 + e / BN, n = n0 + e % BN;
+    if (g > 0 || m >= p.M || n >= p.N) return;
+#pragma unroll
+    for (int k = 1; k < G; ++k) s += sm[k][lane];
+    gc::epilogue_store(s, m, n, p.C, p.ldc, p.ep);
   }
-  cluster.sync();  // the peers read this CTA's tile until here
 }
 
 // ------------------------------------------------------------------ host
 struct Shape {
   int bm, bn, bk;
+  int resident;  // CTAs per SM (registers and shared memory)
+  double rate;   // FMA rate of a full SM relative to the largest tile's
 };
-// Narrow tiles by the width of the output; 64 x 64 and 128 x 128 for the rest.
-constexpr Shape kShapes[] = {{64, 8, 64}, {64, 16, 64}, {64, 32, 32}, {64, 64, 16}, {128, 128, 16}};
+// Narrow tiles by the width of the output; 64 x 64 and 128 x 128 for the rest (4096 x 4096 x 1024: 41.8 and 52.0 TFLOP/s).
+constexpr Shape kShapes[] = {{64, 8, 64, 3, 0.3}, {64, 16, 64, 3, 0.5}, {64, 32, 32, 3, 0.7}, {64, 64, 32, 3, 0.8}, {128, 128, 32, 2, 1.0}};
 
 struct Choice {
-  int shape, splits;
-  bool cluster;  // the splits are one cluster (else partial tiles and a second kernel)
-  int64_t k_per_split;
+  int shape;
+  int64_t tiles, stages, per_cta, ctas;
+  bool shared() const { return per_cta % stages != 0; }
 };
 
 Choice choose(int64_t M, int64_t N, int64_t K) {
   using gc::ceil_div;
-  using gc::kNumSMs;
   Choice best{};
-  auto tiles = [&](int s) { return ceil_div(M, kShapes[s].bm) * ceil_div(N, kShapes[s].bn); };
-  if (N <= 32) {
-    best.shape = N <= 8 ? 0 : N <= 16 ? 1 : 2;
-    // about two CTAs per SM; a split keeps at least two stages of k-values
-    const int64_t want = ceil_div(2 * kNumSMs, std::max<int64_t>(tiles(best.shape), 1));
-    const int64_t most = std::max<int64_t>(1, K / (2 * kShapes[best.shape].bk));
-    int64_t s = std::min(want, most);
-    if (s > 8 && K > 8192) {  // long sums: more splits than a cluster has CTAs, at least 512 k-values each
-      best.splits = int(std::min<int64_t>({s, ceil_div(K, 512), 512}));
-    } else {
-      s = s >= 8 ? 8 : s >= 4 ? 4 : s >= 2 ? 2 : 1;
-      best.splits = int(s);
-      best.cluster = s > 1;
+  double least = -1;
+  const int lo = N <= 8 ? 0 : N <= 16 ? 1 : N <= 32 ? 2 : 3, hi = N <= 32 ? lo : 4;
+  for (int s = lo; s <= hi; ++s) {
+    const Shape& sh = kShapes[s];
+    Choice c{};
+    c.shape = s;
+    c.tiles = ceil_div(M, sh.bm) * ceil_div(N, sh.bn);
+    c.stages = std::max<int64_t>(1, ceil_div(K, sh.bk));
+    const int64_t slots = int64_t(gc::kNumSMs) * sh.resident, units = c.tiles * c.stages;
+    const double unit = double(sh.bm) * sh.bn * sh.bk / 128.0 / sh.rate;  // clocks of an SM
+    // whole tiles: as long as the SM that gets the most of them
+    c.per_cta = c.stages;
+    c.ctas = c.tiles;
+    double t = double(ceil_div(c.tiles, gc::kNumSMs)) * c.stages * unit + 1000.0;
+    // or equal shares, at least 64 k-values each, plus a second kernel (4 to 7 us)
+    const int64_t share = std::max<int64_t>(ceil_div(units, slots), std::min<int64_t>(c.stages, std::max(1, 64 / sh.bk)));
+    const double shared_t = double(ceil_div(ceil_div(units, share), gc::kNumSMs)) * share * unit + 9000.0;
+    if (c.stages > 1 && share != c.stages && shared_t < t) {
+      c.per_cta = share;
+      c.ctas = ceil_div(units, share);
+      t = shared_t;
     }
-  } else {
-    // Time of the busiest SM in FMA clocks: CTAs on it x tile x k-values, the smaller tile at 0.8 of the larger one's
-    // rate, plus the latency of a CTA's first stage and of the exchange of a split tile.
-    double least = 0;
-    for (int s = 3; s <= 4; ++s)
-      for (int64_t z = 1; z <= 8; z *= 2) {
-        if (z > 1 && K / z < 64) break;
-        const double area = double(kShapes[s].bm) * kShapes[s].bn;
-        const double per_sm = double(ceil_div(tiles(s) * z, kNumSMs));
-        const double t = per_sm * (area * double(ceil_div(K, z)) / 128.0 * (s == 3 ? 1.25 : 1.0) +
-                                   (z > 1 ? area / 4 : 0.0) + 1000.0);
-        if (least == 0 || t < least) {
-          least = t;
-          best.shape = s;
-          best.splits = int(z);
-          best.cluster = z > 1;
-        }
-      }
-    const int64_t t = tiles(best.shape);
-    if (t * 8 < kNumSMs && K > 8192) {  // weight gradients: few tiles, long sums
-      best.cluster = false;
-      best.splits = int(std::min<int64_t>({ceil_div(2 * kNumSMs, t), ceil_div(K, 512), 512}));
+    if (least < 0 || t < least) {
+      least = t;
+      best = c;
     }
   }
-  const int64_t bk = kShapes[best.shape].bk;
-  best.k_per_split = std::max<int64_t>(bk, ceil_div(ceil_div(K, best.splits), bk) * bk);
-  if (!best.cluster) best.splits = int(std::max<int64_t>(1, ceil_div(K, best.k_per_split)));
   return best;
 }
 
 template <int BM, int BN, int TM, int TN, int WK, int BK, int ST, bool TA, bool TB, bool VA, bool VB>
-int launch_one(const Args& p, dim3 grid, int cluster, cudaStream_t st) {
+int launch_one(const Args& p, unsigned ctas, cudaStream_t st) {
   using T = Tile<BM, BN, TM, TN, WK, BK, ST, TA, TB>;
   auto kern = gemm_simt_kernel<BM, BN, TM, TN, WK, BK, ST, TA, TB, VA, VB>;
   if (T::kBytes > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kBytes);
     if (e != cudaSuccess) return gc::fail(GC_ERR_CUDA, "gemm_simt: %s", cudaGetErrorString(e));
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = T::kBytes;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 1;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = unsigned(cluster);
-  cfg.attrs = at;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, kern, p);
+  kern<<<ctas, 256, T::kBytes, st>>>(p);
   return gc::check_launch("gemm_simt");
 }
 
 // A tile shape in the four layouts; aligned rows on both operands or on neither (one variant each).
 template <int BM, int BN, int TM, int TN, int WK, int BK, int ST>
-int launch(bool ta, bool tb, bool vec, const Args& p, dim3 grid, int cluster, cudaStream_t st) {
-#define GC_L(TA_, TB_)                                                                                   \
-  (vec ? launch_one<BM, BN, TM, TN, WK, BK, ST, TA_, TB_, true, true>(p, grid, cluster, st)              \
-       : launch_one<BM, BN, TM, TN, WK, BK, ST, TA_, TB_, false, false>(p, grid, cluster, st))
-  if (!ta && !tb) return GC_L(false, false);
-  if (!ta) return GC_L(false, true);
-  if (!tb) return GC_L(true, false);
-  return GC_L(true, true);
+int launch(bool ta, bool tb, bool vec, const Args& p, const Choice& c, cudaStream_t st) {
+  const unsigned n = unsigned(c.ctas);
+  int rc;
+#define GC_L(TA_, TB_)                                                                           \
+  (vec ? launch_one<BM, BN, TM, TN, WK, BK, ST, TA_, TB_, true, true>(p, n, st)                  \
+       : launch_one<BM, BN, TM, TN, WK, BK, ST, TA_, TB_, false, false>(p, n, st))
+  if (!ta && !tb) rc = GC_L(false, false);
+  else if (!ta) rc = GC_L(false, true);
+  else if (!tb) rc = GC_L(true, false);
+  else rc = GC_L(true, true);
 #undef GC_L
+  if (rc != GC_OK || !p.partial) return rc;
+  if (c.stages > 16 * c.per_cta) gemm_shares_kernel<BM, BN, 8><<<unsigned(c.tiles * (BM * BN / 32)), 256, 0, st>>>(p);
+  else gemm_shares_kernel<BM, BN, 1><<<unsigned(c.tiles * ((BM * BN + 1023) / 1024)), 256, 0, st>>>(p);
+  return gc::check_launch("gemm_simt (shares)");
 }
 
 }  // namespace
@@ -370,44 +418,34 @@ size_t simt_workspace_bytes(bool ta, int64_t M, int64_t N, int64_t K) {
     return b ? kFlagBytes + b : 0;
   }
   const Choice c = choose(M, N, K);
-  return c.splits > 1 && !c.cluster ? kFlagBytes + size_t(c.splits) * size_t(M) * size_t(N) * sizeof(float) : 0;
+  return c.shared() ? kFlagBytes + size_t(2 * c.ctas) * kShapes[c.shape].bm * kShapes[c.shape].bn * sizeof(float) : 0;
 }
 
 int gemm_simt(bool ta, bool tb, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B,
               int64_t ldb, float* C, int64_t ldc, const GemmEpilogue& ep, void* workspace, size_t workspace_bytes,
               cudaStream_t st) {
-  if (narrow_supported(ta, M, N, K)) {
-    const size_t need = narrow_partial_bytes(ta, M, N, K);
-    const bool have = need && workspace && workspace_bytes >= kFlagBytes + need;
-    return gemm_narrow(ta, tb, M, N, K, A, lda, B, ldb, C, ldc, ep,
-                       have ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kFlagBytes) : nullptr, st);
-  }
+  const size_t need = simt_workspace_bytes(ta, M, N, K);
+  float* shares = need && workspace && workspace_bytes >= need
+                      ? reinterpret_cast<float*>(static_cast<char*>(workspace) + kFlagBytes)
+                      : nullptr;
+  if (narrow_supported(ta, M, N, K)) return gemm_narrow(ta, tb, M, N, K, A, lda, B, ldb, C, ldc, ep, shares, st);
   Choice c = choose(M, N, K);
-  Args p{int(M), int(N), int(K), A, lda, B, ldb, C, ldc, ep, 0, nullptr};
-  if (c.splits > 1 && !c.cluster) {
-    if (!workspace || workspace_bytes < simt_workspace_bytes(ta, M, N, K)) {
-      c.splits = 1;
-      c.k_per_split = ceil_div(std::max<int64_t>(K, 1), kShapes[c.shape].bk) * kShapes[c.shape].bk;
-    } else {
-      p.partial = reinterpret_cast<float*>(static_cast<char*>(workspace) + kFlagBytes);
-    }
+  if (c.shared() && !shares) {  // no workspace: whole tiles
+    c.per_cta = c.stages;
+    c.ctas = c.tiles;
   }
-  p.k_per_split = int(std::min<int64_t>(c.k_per_split, INT32_MAX));
+  if (c.ctas > INT32_MAX || c.tiles * (kShapes[c.shape].bm * kShapes[c.shape].bn / 32) > INT32_MAX)
+    return fail(GC_ERR_UNSUPPORTED, "gemm_simt: too many tiles for one launch");
+  const Args p{int(M), int(N), int(K), A, lda, B, ldb, C, ldc, ep, int(ceil_div(N, kShapes[c.shape].bn)), int(c.stages),
+               c.tiles * c.stages, int(c.per_cta), c.shared() ? shares : nullptr};
   const bool vec = lda % 4 == 0 && aligned16(A) && ldb % 4 == 0 && aligned16(B);
-  const dim3 grid(unsigned(ceil_div(M, kShapes[c.shape].bm)), unsigned(ceil_div(N, kShapes[c.shape].bn)),
-                  unsigned(c.splits));
-  if (grid.y > 65535u) return fail(GC_ERR_UNSUPPORTED, "gemm_simt: N too large for this launch shape");
-  const int cluster = c.cluster ? c.splits : 1;
-  int rc;
   switch (c.shape) {
-    case 0: rc = launch<64, 8, 4, 4, 8, 64, 3>(ta, tb, vec, p, grid, cluster, st); break;
-    case 1: rc = launch<64, 16, 4, 4, 4, 64, 3>(ta, tb, vec, p, grid, cluster, st); break;
-    case 2: rc = launch<64, 32, 4, 4, 2, 32, 3>(ta, tb, vec, p, grid, cluster, st); break;
-    case 3: rc = launch<64, 64, 4, 4, 1, 16, 4>(ta, tb, vec, p, grid, cluster, st); break;
-    default: rc = launch<128, 128, 8, 8, 1, 16, 3>(ta, tb, vec, p, grid, cluster, st); break;
+    case 0: return launch<64, 8, 4, 4, 8, 64, 3>(ta, tb, vec, p, c, st);
+    case 1: return launch<64, 16, 4, 4, 4, 64, 3>(ta, tb, vec, p, c, st);
+    case 2: return launch<64, 32, 4, 4, 2, 32, 3>(ta, tb, vec, p, c, st);
+    case 3: return launch<64, 64, 4, 4, 1, 32, 3>(ta, tb, vec, p, c, st);
+    default: return launch<128, 128, 8, 8, 1, 32, 3>(ta, tb, vec, p, c, st);
   }
-  if (rc != GC_OK || !p.partial) return rc;
-  return splitk_reduce(int(M), int(N), c.splits, p.partial, C, ldc, ep, st);
 }
 
 }  // namespace gc
