@@ -21,6 +21,7 @@
 //   warps 4-7     epilogue group 0: tcgen05.ld -> bias/ReLU/mask/gate -> global, even 32-column chunks
 //   warps 8-11    converter (three-pass mode): A tile -> A_lo tile (and B -> B_lo)    conv[s]
 //   warps 12-15   epilogue group 1: the odd 32-column chunks
+// or a pair of such CTAs on a 256 x BN tile (PAIR, see the kernel).
 // Two TMEM accumulators (2 x BN columns) let the epilogue of tile i overlap
 // the main loop of tile i+1.
 //
@@ -68,6 +69,22 @@ __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Arrives at the barrier of that offset in CTA 0 of the cluster (the pair's leader).
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .b32 r;\n\t"
+      "mapa.shared::cluster.u32 r, %0, 0;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [r];\n\t}" ::"r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
 // Bounded wait.  Returns false when the CTA is aborting (this wait or another
 // ran out).
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_s) {
@@ -87,36 +104,60 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
       ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
-__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+// The same from either CTA of a pair, counted at the barrier of that offset in the leader (clearing bit 24 of a shared
+// address names the pair's even CTA).
+__device__ __forceinline__ void tma_load_2d_leader(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar & 0xFEFFFFFFu)
+      : "memory");
 }
+template <bool PAIR>
+__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t ncols) {
+  if constexpr (PAIR) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  } else {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(ncols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+}
+template <bool PAIR>
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+  else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void umma_tf32(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// One MMA of 32 bytes of K: kind::tf32 (8 values), or kind::f16 with bf16 operands (16 values).  PAIR: M = 256 over the
+// two CTAs of a cluster, issued by the leader; each CTA holds its 128 rows of A and half of the rows of B at the same
+// shared-memory offsets, and its 128 rows of D.
+template <bool PAIR, bool BF16>
+__device__ __forceinline__ void umma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                     uint32_t accumulate) {
+#define GC_UMMA(GROUP, KIND)                                                                         \
+  asm volatile(                                                                                      \
+      "{\n\t.reg .pred p;\n\t"                                                                      \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                                    \
+      "tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),      \
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                                            \
+      : "memory")
+  if constexpr (PAIR && BF16) GC_UMMA("2", "f16");
+  else if constexpr (PAIR) GC_UMMA("2", "tf32");
+  else if constexpr (BF16) GC_UMMA("1", "f16");
+  else GC_UMMA("1", "tf32");
+#undef GC_UMMA
 }
-// kind::f16 with bf16 operands (K = 16 per instruction: the same 32 bytes of every row as one kind::tf32 step)
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
+// Arrives at `bar` -- of both CTAs when PAIR -- once the MMAs issued so far have completed.
+template <bool PAIR>
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+  if constexpr (PAIR)
+    asm volatile(
+        "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+        "h"(uint16_t(3))
+        : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -165,23 +206,23 @@ __device__ __forceinline__ uint64_t smem_desc_operand(uint32_t saddr, bool mn_ma
 }
 
 // Instruction descriptor for kind::tf32 with fp32 accumulation.
-__host__ __device__ constexpr uint32_t make_idesc(int bn, bool a_mn, bool b_mn) {
+__host__ __device__ constexpr uint32_t make_idesc(int bm, int bn, bool a_mn, bool b_mn) {
   return (1u << 4)                      // D format: F32
          | (2u << 7)                    // A format: TF32
          | (2u << 10)                   // B format: TF32
          | (uint32_t(a_mn ? 1 : 0) << 15)  // A major: 0 = K, 1 = MN
          | (uint32_t(b_mn ? 1 : 0) << 16)  // B major
          | (uint32_t(bn >> 3) << 17)    // N / 8
-         | (uint32_t(BM >> 4) << 24);   // M / 16
+         | (uint32_t(bm >> 4) << 24);   // M / 16
 }
 
 // Instruction descriptor for kind::f16 with bf16 operands (both K-major) and fp32 accumulation.
-__host__ __device__ constexpr uint32_t make_idesc_bf16(int bn) {
+__host__ __device__ constexpr uint32_t make_idesc_bf16(int bm, int bn) {
   return (1u << 4)                     // D format: F32
          | (1u << 7)                   // A format: BF16
          | (1u << 10)                  // B format: BF16
          | (uint32_t(bn >> 3) << 17)   // N / 8
-         | (uint32_t(BM >> 4) << 24);  // M / 16
+         | (uint32_t(bm >> 4) << 24);  // M / 16
 }
 
 struct TcParams {
@@ -196,11 +237,12 @@ struct TcParams {
   float* partial;
 };
 
-template <int BN, int PASSES>
+template <int BN, int PASSES, bool PAIR = false>
 struct Cfg {
   static constexpr int BK = block_k<BN, PASSES>();
+  static constexpr int BNC = PAIR ? BN / 2 : BN;  // rows of B that a CTA holds
   static constexpr int kABytes = BM * BK * 4;
-  static constexpr int kBBytes = BN * BK * 4;
+  static constexpr int kBBytes = BNC * BK * 4;
   static constexpr int kStageBytes = (PASSES == 3 ? 2 : 1) * (kABytes + kBBytes);
   static constexpr int kStages = (200 * 1024 / kStageBytes) > 8 ? 8 : (200 * 1024 / kStageBytes);
   static constexpr int kStagingBytes = 8 * 32 * 32 * 4;  // one 32 x 32 fp32 tile per epilogue warp
@@ -218,13 +260,26 @@ struct Cfg {
 // pre-split copy (weights).
 // BF16: the operands are bf16 matrices (K-major, 64 elements = 128 bytes per row of a stage), one kind::f16
 // MMA per 32-byte step; everything else -- pipeline, TMEM, epilogue -- is the single-pass fp32 kernel.
-template <int BN, int PASSES, bool A_MN, bool B_MN, bool CONV_B, bool BF16 = false>
+// PAIR: two CTAs of a cluster work on one 256 x BN tile with cta_group::2 MMAs.  A CTA stages and splits only its half
+// of B and the tensor core reads half as much of it per SM, which is what bounded the three-pass products: TMA, split,
+// MMA operands and the epilogue's turn together moved more than shared memory's 128 bytes per clock.  The leader (rank 0)
+// issues the MMAs; `conv` collects both CTAs' "stage ready" (single pass: both CTAs' copies are counted at the leader's
+// `full`), `tempty` both epilogues, commits go to both CTAs.  The remote arrivals have the default scope: at cluster
+// scope every one of them waited for the CTA's outstanding stores, 2000 clocks per stage, and a pair was half as fast as
+// one CTA; what the MMAs read was ordered by fence.proxy.async before the arrival.
+template <int BN, int PASSES, bool A_MN, bool B_MN, bool CONV_B, bool BF16 = false, bool PAIR = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                  const __grid_constant__ CUtensorMap mapBlo, TcParams p) {
-  using C_ = Cfg<BN, PASSES>;
+  using C_ = Cfg<BN, PASSES, PAIR>;
   constexpr int S = C_::kStages;
   constexpr int BK = C_::BK;
+  constexpr int BNC = C_::BNC;
+  constexpr int TM = PAIR ? 2 * BM : BM;  // rows of a tile
+  constexpr bool kAtLeader = PAIR && PASSES == 1;  // both CTAs' copies are counted at the leader's `full`
+  const uint32_t rank = PAIR ? cluster_rank() : 0;
+  const int first_item = PAIR ? int(blockIdx.x / 2) : int(blockIdx.x);
+  const int item_step = PAIR ? int(gridDim.x / 2) : int(gridDim.x);
   constexpr int KE = BF16 ? 2 * BK : BK;  // K elements per stage (a stage row is BK * 4 bytes either way)
   static_assert(!BF16 || (PASSES == 1 && !A_MN && !B_MN), "bf16 operands are K-major, one pass");
   constexpr bool kConvB = CONV_B && PASSES == 3;
@@ -249,7 +304,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   const int tiles_n = (p.N + BN - 1) / BN;
-  const int tiles_m = (p.M + BM - 1) / BM;
+  const int tiles_m = (p.M + TM - 1) / TM;
   const int nkb_total = (p.K + KE - 1) / KE;
   const int splits = p.splits > 1 ? p.splits : 1;
   const int kb_per = splits > 1 ? p.kb_per_split : nkb_total;
@@ -258,7 +313,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
   auto item_coords = [&](int item, int& m0, int& n0, int& kb0, int& kb1, int& split) {
     const int t = item % (tiles_m * tiles_n);
     split = item / (tiles_m * tiles_n);
-    m0 = (t / tiles_n) * BM;
+    m0 = (t / tiles_n) * TM + int(rank) * BM;  // first row of this CTA's half
     n0 = (t % tiles_n) * BN;
     kb0 = split * kb_per;
     kb1 = min(nkb_total, kb0 + kb_per);
@@ -269,16 +324,20 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
     for (int s = 0; s < S; ++s) {
       mbar_init(bar_full(s), 1);
       mbar_init(bar_empty(s), 1);
-      mbar_init(bar_conv(s), 4);
+      mbar_init(bar_conv(s), PAIR ? 8 : 4);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(bar_tfull(b), 1);
-      mbar_init(bar_tempty(b), 8);
+      mbar_init(bar_tempty(b), PAIR ? 16 : 8);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async_smem();
   }
-  if (warp == 2) tmem_alloc(smem_u32(&tmem_base_s), C_::kTmemCols);
+  if (PAIR) {
+    __syncthreads();
+    cluster_sync_all();  // both CTAs' barriers exist before either is signalled
+  }
+  if (warp == 2) tmem_alloc<PAIR>(smem_u32(&tmem_base_s), C_::kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -291,34 +350,41 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
       uint32_t it = 0;
       bool ok = true;
       constexpr uint32_t kTx = C_::kABytes + ((PASSES == 3 && !kConvB) ? 2 : 1) * C_::kBBytes;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+      for (int item = first_item; item < num_items && ok; item += item_step) {
         int m0, n0, kb0, kb1, split;
         item_coords(item, m0, n0, kb0, kb1, split);
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % S;
           const uint32_t ph = (it / S) & 1u;
           if (!mbar_wait(bar_empty(s), ph ^ 1u, abort_p)) { ok = false; break; }
-          mbar_expect_tx(bar_full(s), kTx);
+          if (!kAtLeader) mbar_expect_tx(bar_full(s), kTx);
+          else if (rank == 0) mbar_expect_tx(bar_full(s), 2 * kTx);
+          auto load = [&](uint32_t dst, const CUtensorMap* map, int x, int y) {
+            if (kAtLeader) tma_load_2d_leader(dst, map, x, y, bar_full(s));
+            else tma_load_2d(dst, map, x, y, bar_full(s));
+          };
           if (A_MN) {
 #pragma unroll
             for (int c = 0; c < BM / 32; ++c)
-              tma_load_2d(sA(s) + c * (BK * 128), &mapA, m0 + c * 32, kb * BK, bar_full(s));
+              load(sA(s) + c * (BK * 128), &mapA, m0 + c * 32, kb * BK);
           } else {
-            tma_load_2d(sA(s), &mapA, kb * KE, m0, bar_full(s));
+            load(sA(s), &mapA, kb * KE, m0);
           }
+          const int nb = n0 + int(rank) * BNC;  // this CTA's rows of B
           if (B_MN) {
 #pragma unroll
-            for (int c = 0; c < BN / 32; ++c)
-              tma_load_2d(sB(s) + c * (BK * 128), &mapB, n0 + c * 32, kb * BK, bar_full(s));
+            for (int c = 0; c < BNC / 32; ++c)
+              load(sB(s) + c * (BK * 128), &mapB, nb + c * 32, kb * BK);
           } else {
-            tma_load_2d(sB(s), &mapB, kb * KE, n0, bar_full(s));
-            if (PASSES == 3 && !kConvB) tma_load_2d(sBlo(s), &mapBlo, kb * BK, n0, bar_full(s));
+            load(sB(s), &mapB, kb * KE, nb);
+            if (PASSES == 3 && !kConvB) load(sBlo(s), &mapBlo, kb * BK, nb);
           }
         }
       }
       // Drain: every copy issued must have landed before the CTA may exit.
       // `it` stages were issued; the last min(S, it) of them may be in flight.
-      const uint32_t pending = it < uint32_t(S) ? it : uint32_t(S);
+      // (Counted at the leader: it waits for both CTAs', and the peer for the leader at the end.)
+      const uint32_t pending = kAtLeader && rank != 0 ? 0u : it < uint32_t(S) ? it : uint32_t(S);
       for (uint32_t j = 0; j < pending; ++j) {
         const uint32_t q = it - 1 - j;
         const uint32_t bar = bar_full(q % S), par = (q / S) & 1u;
@@ -330,14 +396,14 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = BF16 ? make_idesc_bf16(BN) : make_idesc(BN, A_MN, B_MN);
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = BF16 ? make_idesc_bf16(TM, BN) : make_idesc(TM, BN, A_MN, B_MN);
       constexpr uint32_t kMnLbo = BK * 128;  // bytes between 32-column chunks of an MN-major tile
       constexpr uint32_t kAStep = A_MN ? 1024u : uint32_t(UMMA_K * 4);  // start-address advance per k-step
       constexpr uint32_t kBStep = B_MN ? 1024u : uint32_t(UMMA_K * 4);
       uint32_t it = 0, tcount = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++tcount) {
+      for (int item = first_item; item < num_items && ok; item += item_step, ++tcount) {
         int m0, n0, kb0, kb1, split;
         item_coords(item, m0, n0, kb0, kb1, split);
         const int b = tcount & 1;
@@ -361,18 +427,16 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
             const uint64_t ab = uint64_t((k * kBStep) >> 4);
             const uint32_t acc = (kb > kb0 || k > 0) ? 1u : 0u;
             if (PASSES == 3) {
-              umma_tf32(d_tmem, dal + aa, db + ab, idesc, acc);
-              umma_tf32(d_tmem, da + aa, dbl + ab, idesc, 1u);
-              umma_tf32(d_tmem, da + aa, db + ab, idesc, 1u);
-            } else if (BF16) {
-              umma_bf16(d_tmem, da + aa, db + ab, idesc, acc);
+              umma<PAIR, false>(d_tmem, dal + aa, db + ab, idesc, acc);
+              umma<PAIR, false>(d_tmem, da + aa, dbl + ab, idesc, 1u);
+              umma<PAIR, false>(d_tmem, da + aa, db + ab, idesc, 1u);
             } else {
-              umma_tf32(d_tmem, da + aa, db + ab, idesc, acc);
+              umma<PAIR, BF16>(d_tmem, da + aa, db + ab, idesc, acc);
             }
           }
-          umma_commit(bar_empty(s));  // frees the stage once these MMAs have read it
+          umma_commit<PAIR>(bar_empty(s));  // frees the stage once these MMAs have read it
         }
-        if (ok) umma_commit(bar_tfull(b));
+        if (ok) umma_commit<PAIR>(bar_tfull(b));
       }
     }
   } else if ((warp >= 4 && warp < 8) || warp >= 12) {
@@ -384,7 +448,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
     const int grp = warp >= 12 ? 1 : 0;  // chunk parity
     uint32_t tcount = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x, ++tcount) {
+    for (int item = first_item; item < num_items && ok; item += item_step, ++tcount) {
       int m0, n0, kb0, kb1, split;
       item_coords(item, m0, n0, kb0, kb1, split);
       const int b = tcount & 1;
@@ -402,9 +466,9 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
       const bool vec = raw_out ? (p.N % 4 == 0) : (p.vec_store != 0);
       // Gate values of the NEXT tile of this CTA are requested into the L2 now, a whole tile time before the
       // epilogue reads them (they come from DRAM: 128 KB per tile, read once).
-      if (ep.gate && item + int(gridDim.x) < num_items) {
+      if (ep.gate && item + item_step < num_items) {
         int nm0, nn0, nk0, nk1, nsplit;
-        item_coords(item + int(gridDim.x), nm0, nn0, nk0, nk1, nsplit);
+        item_coords(item + item_step, nm0, nn0, nk0, nk1, nsplit);
         const int prow = nm0 + q * 32 + lane;
         if (prow < p.M) {
           const char* g = reinterpret_cast<const char*>(ep.gate + int64_t(prow) * ldc + nn0);
@@ -492,7 +556,10 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(bar_tempty(b));
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_leader(bar_tempty(b));
+        else mbar_arrive(bar_tempty(b));
+      }
     }
   } else if (warp >= 8 && PASSES == 3) {
     // ------------------------------------------------------------ converter
@@ -500,7 +567,7 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
     constexpr int kVecs = (C_::kABytes + (kConvB ? C_::kBBytes : 0)) / 16;  // A (and B) are contiguous in a stage
     uint32_t it = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < num_items && ok; item += gridDim.x) {
+    for (int item = first_item; item < num_items && ok; item += item_step) {
       int m0, n0, kb0, kb1, split;
       item_coords(item, m0, n0, kb0, kb1, split);
       for (int kb = kb0; kb < kb1; ++kb, ++it) {
@@ -521,7 +588,10 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
         }
         fence_async_smem();  // generic-proxy writes -> visible to the tensor core's async-proxy reads
         __syncwarp();
-        if (lane == 0) mbar_arrive(bar_conv(s));
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_leader(bar_conv(s));
+          else mbar_arrive(bar_conv(s));
+        }
       }
     }
   }
@@ -529,8 +599,9 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();  // the peer's MMAs read this CTA's shared memory and write its TMEM until here
   tc_fence_after();
-  if (warp == 2) tmem_dealloc(tmem_base, C_::kTmemCols);
+  if (warp == 2) tmem_dealloc<PAIR>(tmem_base, C_::kTmemCols);
   if (threadIdx.x == 0 && abort_s && p.flag) atomicExch(p.flag, 1);
 }
 
@@ -745,9 +816,19 @@ struct Plan {
   bool transpose_b;  // B given K x N, re-laid N x K in the workspace
   bool b_mn;         // B consumed MN-major in place
   bool conv_b;       // B_lo made in shared memory (else pre-split into the workspace)
+  bool pair;         // two CTAs per tile of 256 rows
   int bn;
   int splits, kb_per_split;
 };
+
+// Two CTAs per tile where M fills 256-row tiles and there are at least as many tiles as CTA pairs.  Measured, one CTA ->
+// a pair: three passes 4096^3 623 -> 583 us, 2^20 x 256 x 100 505 -> 443, 32768^2 x 256 2.9 -> 2.4 ms; one pass 4096^3
+// 234 -> 209, 8192^3 1764 -> 1537; but a single-pass 256 x 256 weight gradient split along k 321 -> 355 (74 pairs share
+// what 148 CTAs took), and 64-column tiles gain nothing (a CTA's half of B is 32 rows).
+bool use_pair(int64_t M, int64_t N, int bn, int64_t splits, int passes) {
+  if (M <= BM || bn < 128 || (passes == 1 && splits > 1)) return false;
+  return gc::ceil_div(M, 2 * BM) * gc::ceil_div(N, bn) * splits >= gc::kNumSMs / 2;
+}
 
 Plan make_plan(bool ta, bool tb, int64_t M, int64_t N, int64_t K, int passes) {
   Plan pl{};
@@ -787,29 +868,42 @@ Plan make_plan(bool ta, bool tb, int64_t M, int64_t N, int64_t K, int passes) {
   if (passes == 3 && splits > 1)
     pl.kb_per_split = int(std::max<int64_t>(1, std::min<int64_t>(pl.kb_per_split, kMaxChainK / bk)));
   pl.splits = int(gc::ceil_div(nkb, pl.kb_per_split));
+  pl.pair = use_pair(M, N, pl.bn, pl.splits, passes);
   return pl;
 }
 
-template <int BN, int PASSES, bool A_MN, bool B_MN, bool CONV_B>
+template <int BN, int PASSES, bool A_MN, bool B_MN, bool CONV_B, bool BF16, bool PAIR>
 int launch_tc(const CUtensorMap& mA, const CUtensorMap& mB, const CUtensorMap& mBlo, const TcParams& p,
               cudaStream_t st) {
-  using C_ = Cfg<BN, PASSES>;
-  auto kern = gemm_tf32_kernel<BN, PASSES, A_MN, B_MN, CONV_B>;
+  using C_ = Cfg<BN, PASSES, PAIR>;
+  auto kern = gemm_tf32_kernel<BN, PASSES, A_MN, B_MN, CONV_B, BF16, PAIR>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C_::kSmemBytes);
   if (e != cudaSuccess) return gc::fail(GC_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  const int64_t items = gc::ceil_div(p.M, BM) * gc::ceil_div(p.N, BN) * (p.splits > 1 ? p.splits : 1);
-  const unsigned grid = unsigned(std::min<int64_t>(items, gc::kNumSMs));
-  kern<<<grid, kThreads, C_::kSmemBytes, st>>>(mA, mB, mBlo, p);
+  constexpr int kCtas = PAIR ? 2 : 1;
+  const int64_t items = gc::ceil_div(p.M, BM * kCtas) * gc::ceil_div(p.N, BN) * (p.splits > 1 ? p.splits : 1);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(std::min<int64_t>(items, gc::kNumSMs / kCtas)) * kCtas);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = C_::kSmemBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = PAIR ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, mA, mB, mBlo, p);
   return gc::check_launch("gemm_tf32_kernel");
 }
 
-template <int BN, int PASSES>
+template <int BN, int PASSES, bool PAIR>
 int launch_layout(const Plan& pl, const CUtensorMap& mA, const CUtensorMap& mB, const CUtensorMap& mBlo,
                   const TcParams& p, cudaStream_t st) {
-  if (pl.a_mn && pl.b_mn) return launch_tc<BN, PASSES, true, true, true>(mA, mB, mBlo, p, st);
-  if (pl.b_mn) return launch_tc<BN, PASSES, false, true, true>(mA, mB, mBlo, p, st);
-  if (pl.conv_b && PASSES == 3) return launch_tc<BN, PASSES, false, false, true>(mA, mB, mBlo, p, st);
-  return launch_tc<BN, PASSES, false, false, false>(mA, mB, mBlo, p, st);
+  if (pl.a_mn && pl.b_mn) return launch_tc<BN, PASSES, true, true, true, false, PAIR>(mA, mB, mBlo, p, st);
+  if (pl.b_mn) return launch_tc<BN, PASSES, false, true, true, false, PAIR>(mA, mB, mBlo, p, st);
+  if (pl.conv_b && PASSES == 3) return launch_tc<BN, PASSES, false, false, true, false, PAIR>(mA, mB, mBlo, p, st);
+  return launch_tc<BN, PASSES, false, false, false, false, PAIR>(mA, mB, mBlo, p, st);
 }
 
 }  // namespace
@@ -909,10 +1003,10 @@ int gemm_tc(bool ta, bool tb, int64_t M, int64_t N, int64_t K, const float* A, i
   else rc = make_map(&mA, Aop, M, K, lda_op, BM, false, bk);
   if (rc != GC_OK) return rc;
   if (pl.b_mn) rc = make_map(&mB, Bop, K, N, ldb_op, bk, true, bk);
-  else rc = make_map(&mB, Bop, N, K, ldb_op, pl.bn, false, bk);
+  else rc = make_map(&mB, Bop, N, K, ldb_op, pl.pair ? pl.bn / 2 : pl.bn, false, bk);
   if (rc != GC_OK) return rc;
   if (pl.b_mn) mBlo = mB;
-  else if ((rc = make_map(&mBlo, Blo, N, K, ldblo, pl.bn, false, bk)) != GC_OK) return rc;
+  else if ((rc = make_map(&mBlo, Blo, N, K, ldblo, pl.pair ? pl.bn / 2 : pl.bn, false, bk)) != GC_OK) return rc;
 
   TcParams p;
   p.M = int(M);
@@ -929,15 +1023,14 @@ int gemm_tc(bool ta, bool tb, int64_t M, int64_t N, int64_t K, const float* A, i
   p.splits = pl.splits;
   p.kb_per_split = pl.kb_per_split;
   p.partial = partial;
-  if (passes == 3) {
-    if (pl.bn == 64) rc = launch_layout<64, 3>(pl, mA, mB, mBlo, p, st);
-    else if (pl.bn == 128) rc = launch_layout<128, 3>(pl, mA, mB, mBlo, p, st);
-    else rc = launch_layout<256, 3>(pl, mA, mB, mBlo, p, st);
-  } else {
-    if (pl.bn == 64) rc = launch_layout<64, 1>(pl, mA, mB, mBlo, p, st);
-    else if (pl.bn == 128) rc = launch_layout<128, 1>(pl, mA, mB, mBlo, p, st);
-    else rc = launch_layout<256, 1>(pl, mA, mB, mBlo, p, st);
-  }
+#define GC_LAYOUT(P)                                                                          \
+  (pl.bn == 64    ? launch_layout<64, P, false>(pl, mA, mB, mBlo, p, st)                      \
+   : pl.bn == 128 ? (pl.pair ? launch_layout<128, P, true>(pl, mA, mB, mBlo, p, st)           \
+                             : launch_layout<128, P, false>(pl, mA, mB, mBlo, p, st))         \
+                  : (pl.pair ? launch_layout<256, P, true>(pl, mA, mB, mBlo, p, st)           \
+                             : launch_layout<256, P, false>(pl, mA, mB, mBlo, p, st)))
+  rc = passes == 3 ? GC_LAYOUT(3) : GC_LAYOUT(1);
+#undef GC_LAYOUT
   if (rc != GC_OK) return rc;
   if (pl.splits > 1) {
     rc = splitk_reduce(int(M), int(N), pl.splits, partial, C, ldc, ep, st);
@@ -1001,18 +1094,14 @@ int gemm_bf16_core(int64_t M, int64_t N, int64_t K, const uint16_t* A, int64_t l
   p.partial = p.splits > 1 ? reinterpret_cast<float*>(ws) : nullptr;
   CUtensorMap mA, mB;
   int rc = make_map_bf16(&mA, A, M, K, lda, BM);
-  if (rc == GC_OK) rc = make_map_bf16(&mB, Bt, N, K, ldb, bn);
+  const bool pair = use_pair(M, N, bn, p.splits, 1);
+  if (rc == GC_OK) rc = make_map_bf16(&mB, Bt, N, K, ldb, pair ? bn / 2 : bn);
   if (rc != GC_OK) return rc;
-  auto run = [&](auto kern, int smem, int bn_) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return fail(GC_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-    const int64_t items = ceil_div(M, BM) * ceil_div(N, bn_) * (p.splits > 1 ? p.splits : 1);
-    kern<<<unsigned(std::min<int64_t>(items, kNumSMs)), kThreads, smem, st>>>(mA, mB, mB, p);
-    return check_launch("gemm_tf32_kernel (bf16 operands)");
-  };
-  if (bn == 64) rc = run(gemm_tf32_kernel<64, 1, false, false, false, true>, Cfg<64, 1>::kSmemBytes, 64);
-  else if (bn == 128) rc = run(gemm_tf32_kernel<128, 1, false, false, false, true>, Cfg<128, 1>::kSmemBytes, 128);
-  else rc = run(gemm_tf32_kernel<256, 1, false, false, false, true>, Cfg<256, 1>::kSmemBytes, 256);
+  if (bn == 64) rc = launch_tc<64, 1, false, false, false, true, false>(mA, mB, mB, p, st);
+  else if (bn == 128 && pair) rc = launch_tc<128, 1, false, false, false, true, true>(mA, mB, mB, p, st);
+  else if (bn == 128) rc = launch_tc<128, 1, false, false, false, true, false>(mA, mB, mB, p, st);
+  else if (pair) rc = launch_tc<256, 1, false, false, false, true, true>(mA, mB, mB, p, st);
+  else rc = launch_tc<256, 1, false, false, false, true, false>(mA, mB, mB, p, st);
   if (rc != GC_OK) return rc;
   if (p.splits > 1) {
     rc = splitk_reduce(int(M), int(N), p.splits, p.partial, C, ldc, ep, st);
