@@ -36,45 +36,61 @@ struct TensorList {
 // state[0] = steps taken so far (read by every CTA before it counts itself in
 // state[1]); the CTA that arrives last writes the new step count and clears
 // the arrival counter, so no CTA can observe the incremented value.
+//
+// On a Cora-sized model the launch is a latency chain, not a stream: the two
+// bias corrections (a double pow each) are computed by two warps at a time and
+// the first chunk is on its way from memory meanwhile (one thread computing
+// both before the first load: 5.9 us for 23 K parameters, 4.3 so).
 __global__ void __launch_bounds__(256)
 adam_kernel(TensorList tl, double lr, double beta1, double beta2, float eps, float weight_decay,
             unsigned long long* __restrict__ state) {
-  __shared__ unsigned long long step_s;
   __shared__ float consts_s[2];
-  if (threadIdx.x == 0) {
-    step_s = *reinterpret_cast<volatile unsigned long long*>(state);
+  const int64_t total = tl.first_chunk[tl.count];
+  float pv[4], gv[4], mv[4], vv[4];
+  int k = 0;
+  int64_t base = 0, n = 0;
+  auto load = [&](int64_t vc) {  // chunks come in ascending order: k only grows
+    while (k + 1 < tl.count && vc >= tl.first_chunk[k + 1]) ++k;
+    base = (vc - tl.first_chunk[k]) * kChunk + threadIdx.x;
+    n = tl.n[k];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t i = base + u * 256;
+      const bool ok = i < n;
+      pv[u] = ok ? tl.p[k][i] : 0.f;
+      gv[u] = ok ? tl.g[k][i] : 0.f;
+      mv[u] = ok ? tl.m[k][i] : 0.f;
+      vv[u] = ok ? tl.v[k][i] : 0.f;
+    }
+  };
+  int64_t vc = blockIdx.x;
+  unsigned long long step = 0;
+  if (threadIdx.x % 32 == 0 && threadIdx.x < 64) step = *reinterpret_cast<volatile unsigned long long*>(state);
+  if (vc < total) load(vc);
+  if (threadIdx.x % 32 == 0 && threadIdx.x < 64) {
     // scalar part in double, as the Python arithmetic of torch.optim.Adam does it
-    const double t = double(step_s + 1ull);
-    consts_s[0] = float(lr / (1.0 - pow(beta1, t)));
-    consts_s[1] = float(sqrt(1.0 - pow(beta2, t)));
+    const double rest = 1.0 - pow(threadIdx.x ? beta2 : beta1, double(step + 1ull));
+    consts_s[threadIdx.x / 32] = float(threadIdx.x ? sqrt(rest) : lr / rest);
   }
   __syncthreads();
   const float step_size = consts_s[0];
   const float bc2_sqrt = consts_s[1];
   const float w1 = float(1.0 - beta1), w2 = float(1.0 - beta2), b2 = float(beta2);
-  const int64_t total = tl.first_chunk[tl.count];
-  for (int64_t vc = blockIdx.x; vc < total; vc += gridDim.x) {
-    int k = 0;
-    while (k + 1 < tl.count && vc >= tl.first_chunk[k + 1]) ++k;
-    const int64_t base = (vc - tl.first_chunk[k]) * kChunk;
-    float* __restrict__ p = tl.p[k];
-    const float* __restrict__ g = tl.g[k];
-    float* __restrict__ m = tl.m[k];
-    float* __restrict__ v = tl.v[k];
-    const int64_t n = tl.n[k];
+  while (vc < total) {
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int64_t i = base + u * 256 + threadIdx.x;
+      const int64_t i = base + u * 256;
       if (i < n) {
-        const float pi = p[i];
-        const float gi = g[i] + weight_decay * pi;
-        const float mi = m[i] + (gi - m[i]) * w1;
-        const float vi = v[i] * b2 + gi * gi * w2;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] = pi - step_size * (mi / (sqrtf(vi) / bc2_sqrt + eps));
+        const float gi = gv[u] + weight_decay * pv[u];
+        const float mi = mv[u] + (gi - mv[u]) * w1;
+        const float vi = vv[u] * b2 + gi * gi * w2;
+        tl.m[k][i] = mi;
+        tl.v[k][i] = vi;
+        tl.p[k][i] = pv[u] - step_size * (mi / (sqrtf(vi) / bc2_sqrt + eps));
       }
     }
+    vc += gridDim.x;
+    if (vc < total) load(vc);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -82,7 +98,7 @@ adam_kernel(TensorList tl, double lr, double beta1, double beta2, float eps, flo
     const unsigned long long arrived = atomicAdd(state + 1, 1ull);
     if (arrived == gridDim.x - 1) {
       state[1] = 0ull;
-      state[0] = step_s + 1ull;
+      state[0] = step + 1ull;
     }
   }
 }
