@@ -830,6 +830,18 @@ void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, cons
     else GC_SHORT(16, 4, SO);
     return;
   }
+  // Wider rows: several warps per piece (grid.y), fewer lanes per non-zero -- and so more non-zeros side by side -- the
+  // less there is to gather.  Measured (us for the product, groups of lanes / this with 8, 16, 32 lanes): 1 K rows, 41 K
+  // non-zeros F = 128 22.8 / 10.4, 14.3, 21.1; 9 K rows, 89 K non-zeros F = 72 23.5 / 15.4, 16.7, 21.6, F = 256 31.5 /
+  // 29.9, 25.0, 26.3; 20 K rows, 180 K non-zeros F = 128 26.2 / 28.5, 22.1, 23.4, F = 256 34.7 / 51.8, 36.1, 32.4; 40 K
+  // rows F = 128 29.9 / 53.9, 33.8, 26.5, F = 200 41.7 / 93, 65, 50.
+  const int64_t vectors = int64_t(n_pieces) * units;
+  if (units > 16 && units <= 64 && vectors <= gc::kNumSMs * int64_t(9216)) {
+    if (vectors <= gc::kNumSMs * 1536) GC_SHORT(8, 4, SO);
+    else if (vectors <= gc::kNumSMs * 4096) GC_SHORT(16, 4, SO);
+    else GC_SHORT(32, 4, SO);
+    return;
+  }
   // Measured on the 126 M-non-zero graph: up to 8 floats the lane-per-non-zero kernel wins (F = 8: 0.99 ms
   // against 2.0 ms); from 12 to 32 floats groups of 4 lanes with one or two 128-bit vectors per lane and 4
   // non-zeros in flight do (F = 32: 1.5 ms against 1.7 ms for 8 lanes x 1 vector, 3.4 ms for 2 lanes x 4
