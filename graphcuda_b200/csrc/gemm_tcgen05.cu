@@ -498,17 +498,18 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
             if (gn < p.N && gm < p.M) gc::epilogue_store(__uint_as_float(r[j]), gm, gn, Cb, ldc, ep);
           }
           if (have_next) tmem_ld32(taddr + uint32_t((c + 2) * 32), r);
-        } else if (vec && gn0 + 32 <= p.N) {
+        } else if (vec && (gn0 + 32 <= p.N || p.N % 4 == 0)) {
           // The accumulator arrives one row per lane.  Stored like that, every 128-bit store of the warp would
           // touch 32 different lines.  The 32 x 32 block is turned through shared memory -- 128-bit accesses both
           // ways, the 16-byte chunk index XORed with the row so that neither direction has bank conflicts -- and
           // every store instruction covers four complete 128-byte row segments.  The TMEM load of the next 32
           // columns and the gate values of this block are in flight while the block is turned.
+          const int passes_left = gn0 + c4 < p.N ? rows_left : 0;  // the last block may have fewer columns (48: 16)
           float4 gv[8];
           if (ep.gate) {
 #pragma unroll
             for (int pass = 0; pass < 8; ++pass)
-              gv[pass] = 4 * pass < rows_left
+              gv[pass] = 4 * pass < passes_left
                              ? __ldcs(reinterpret_cast<const float4*>(ep.gate + row0_off + int64_t(4 * pass) * ldc + gn0))
                              : make_float4(0.f, 0.f, 0.f, 0.f);
           }
@@ -520,12 +521,12 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
           if (have_next) tmem_ld32(taddr + uint32_t((c + 2) * 32), r);
           __syncwarp();
           float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (ep.bias) bv = __ldg(reinterpret_cast<const float4*>(ep.bias + gn0 + c4));
+          if (ep.bias && passes_left > 0) bv = __ldg(reinterpret_cast<const float4*>(ep.bias + gn0 + c4));
 #pragma unroll
           for (int pass = 0; pass < 8; ++pass) {
             const int row = pass * 4 + row_in_quarter;
             float4 v = tile4[row * 8 + ((lane & 7) ^ (row & 7))];
-            if (4 * pass < rows_left) {
+            if (4 * pass < passes_left) {
               const int64_t off = row0_off + int64_t(4 * pass) * ldc + gn0;
               v.x += bv.x; v.y += bv.y; v.z += bv.z; v.w += bv.w;
               if (ep.relu || ep.mask) {
@@ -543,14 +544,24 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
           }
           __syncwarp();
         } else {
-          if (gm < p.M) {
+          // Rows of C that are not 16-byte aligned, or the ragged last columns: turned the same way, then stored one
+          // float per lane, 32 consecutive columns of a row at a time (stored as they arrive, the lanes of a warp would
+          // write 32 different rows).
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-              const int gn = gn0 + j;
-              if (gn < p.N) gc::epilogue_store(__uint_as_float(r[j]), gm, gn, Cb, ldc, ep);
-            }
-          }
+          for (int j4 = 0; j4 < 8; ++j4)
+            tile4[lane * 8 + (j4 ^ (lane & 7))] =
+                make_float4(__uint_as_float(r[4 * j4]), __uint_as_float(r[4 * j4 + 1]), __uint_as_float(r[4 * j4 + 2]),
+                            __uint_as_float(r[4 * j4 + 3]));
           if (have_next) tmem_ld32(taddr + uint32_t((c + 2) * 32), r);
+          __syncwarp();
+          const float* tile = reinterpret_cast<const float*>(tile4);
+          const int rows = min(32, p.M - (m0 + q * 32));
+          if (gn0 + lane < p.N)
+#pragma unroll 4
+            for (int row = 0; row < rows; ++row)
+              gc::epilogue_store(tile[row * 32 + ((lane >> 2) ^ (row & 7)) * 4 + (lane & 3)], m0 + q * 32 + row, gn0 + lane, Cb,
+                                 ldc, ep);
+          __syncwarp();
         }
         if (have_next) tmem_ld_wait();
       }
@@ -576,15 +587,21 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
         if (!mbar_wait(bar_full(s), ph, abort_p)) { ok = false; break; }
         const float4* src = reinterpret_cast<const float4*>(smem + s * C_::kStageBytes);
         float4* dst = reinterpret_cast<float4*>(smem + s * C_::kStageBytes + C_::kABytes + C_::kBBytes);
-#pragma unroll 8
-        for (int i = ct; i < kVecs; i += 128) {
-          const float4 v = src[i];
-          float4 lo;
-          lo.x = v.x - __uint_as_float(__float_as_uint(v.x) & 0xFFFFE000u);
-          lo.y = v.y - __uint_as_float(__float_as_uint(v.y) & 0xFFFFE000u);
-          lo.z = v.z - __uint_as_float(__float_as_uint(v.z) & 0xFFFFE000u);
-          lo.w = v.w - __uint_as_float(__float_as_uint(v.w) & 0xFFFFE000u);
-          dst[i] = lo;
+        constexpr int kIter = kVecs / 128, kBatch = kIter % 8 == 0 ? 8 : kIter % 6 == 0 ? 6 : 4;
+        static_assert(kVecs % 128 == 0 && kIter % kBatch == 0, "whole batches");
+#pragma unroll
+        for (int i0 = 0; i0 < kIter; i0 += kBatch) {
+          float4 v[kBatch];  // all loads of a batch before its first store: they may alias for all the compiler knows
+#pragma unroll
+          for (int j = 0; j < kBatch; ++j) v[j] = src[(i0 + j) * 128 + ct];
+#pragma unroll
+          for (int j = 0; j < kBatch; ++j) {
+            v[j].x -= __uint_as_float(__float_as_uint(v[j].x) & 0xFFFFE000u);
+            v[j].y -= __uint_as_float(__float_as_uint(v[j].y) & 0xFFFFE000u);
+            v[j].z -= __uint_as_float(__float_as_uint(v[j].z) & 0xFFFFE000u);
+            v[j].w -= __uint_as_float(__float_as_uint(v[j].w) & 0xFFFFE000u);
+            dst[(i0 + j) * 128 + ct] = v[j];
+          }
         }
         fence_async_smem();  // generic-proxy writes -> visible to the tensor core's async-proxy reads
         __syncwarp();
