@@ -261,8 +261,8 @@ __device__ __forceinline__ void store_columns(const typename Vec<VW>::T& acc, fl
 // of the tuning: left to itself the compiler settles near 78 registers and
 // serialises the gathers; told its budget (80 registers at 3 CTAs, 128 at 2)
 // it keeps a whole round of U x NACC loads in flight.  Measured on the
-// 126 M-non-zero graph, F = 256: 12.6 ms unconstrained, 8.7 ms at 2, 8.4 ms
-// at 3; F = 100: 6.3 / 4.4 / 4.4 ms.
+// 126 M-non-zero graph, F = 256 on groups of 16: 12.6 ms unconstrained, 8.7 ms
+// at 2, 8.4 ms at 3; F = 100: 6.3 / 4.4 / 4.4 ms.
 // SO: F is the true width of Y; the columns up to the next multiple of 4 are gathered (H is padded) and dropped.
 template <int GROUP, int NACC, int VW, int U, bool PLANNED, int MIN_CTAS, bool SO>
 __global__ void __launch_bounds__(256, MIN_CTAS)
@@ -757,15 +757,7 @@ int count_rows(const int32_t* rowptr, const int32_t* col, int M, int K, int pane
 }
 
 // ---------------------------------------------------------------- dispatch
-// Two resident CTAs (128 registers) for the 3- and 4-accumulator mappings on groups
-// of up to 8 lanes: on a 2.3 M-non-zero graph they run F = 48..128 in
-// 0.11-0.13 ms against 0.15-0.22 ms at three; everything else is as fast or
-// faster at three (F = 512 on 126 M non-zeros: 17.9 against 20.5 ms).
-constexpr int pieces_min_ctas(int group, int nacc, int vw) {
-  return ((vw == 4 && nacc >= 3 && group <= 8) || (vw == 8 && nacc >= 2 && group <= 8)) ? 2 : 3;
-}
-
-template <int GROUP, int NACC, int VW, int U, bool SO = false>
+template <int GROUP, int NACC, int VW, int U, int MINB, bool SO>
 void launch_pieces(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
                    const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const typename Vec<VW>::HT* H,
                    int64_t ldH,
@@ -777,7 +769,6 @@ void launch_pieces(bool planned, const int32_t* rowptr, const int32_t* col, cons
   // few pieces and several passes: one CTA row per pass (up to about eight CTAs per SM in total)
   const unsigned gy = unsigned(std::max(1, std::min<int>(passes, int(gc::kNumSMs * 8 / std::max(gx, 1u)))));
   const dim3 grid(gx, gy);
-  constexpr int MINB = pieces_min_ctas(GROUP, NACC, VW);
   if (planned)
     spmm_pieces_kernel<GROUP, NACC, VW, U, true, MINB, SO>
         <<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap, ovf, ep, rb);
@@ -786,10 +777,9 @@ void launch_pieces(bool planned, const int32_t* rowptr, const int32_t* col, cons
         <<<grid, 256, 0, st>>>(rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap, ovf, ep, rb);
 }
 
-#define GC_PIECES(G, A, VWID, UU) GC_PIECES_SO(G, A, VWID, UU, false)
-#define GC_PIECES_SO(G, A, VWID, UU, SO_)                                                                         \
-  launch_pieces<G, A, VWID, UU, SO_>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, \
-                                cap, ovf, ep, rb, st)
+#define GC_PIECES(G, A, VWID, UU, MB, SO_)                                                                            \
+  launch_pieces<G, A, VWID, UU, MB, SO_>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, \
+                                         ldS, cap, ovf, ep, rb, st)
 
 // Matrices that a warp per piece serves sooner than groups of lanes do.  Measured (us, groups / warp per piece): 20 K
 // pieces F = 16 19.5 / 11.2, F = 64 28.5 / 16.1; 61 K pieces F = 7 19.3 / 21.4, F = 16 24.5 / 23.9, F = 64 35 / 29; 77 K
@@ -813,9 +803,19 @@ void launch_short(bool planned, const int32_t* rowptr, const int32_t* col, const
   launch_short<UN, VWID, SO_>(planned, rowptr, col, val, n_pieces, ps, pl, pt, F, H, ldH, Y, ldY, scratch, ldS, cap,  \
                          ovf, ep, rb, st)
 
-// GROUP x NACC 128-bit vectors cover a row of H; small groups keep several
-// pieces in flight per warp and four accumulators per lane amortise the
-// (col, val) broadcast.
+// GROUP x NACC 128-bit vectors cover a row of H; small groups keep several pieces in flight per warp and the accumulators
+// of a lane amortise the (col, val) broadcast.  The gather is bound by the path from the L2 to the SMs (15 TB/s at best)
+// and, below that, by load instructions: a vector slot with no column behind it costs as much as a full one (100 columns
+// on 32 slots take the time of 128), so the slots follow the width in steps of a third, and what a lane has in flight
+// (U rounds) is set against the CTAs that the registers then leave room for.  Measured (us; 126 M / 2.5 M / 12.6 M non-
+// zeros on 2.4 M / 169 K / 600 K rows), a mapping of four vectors, four rounds -> the one below:
+//   F =  64: 2638 / 73 / 365 -> 2486 / 68 / 297    F =  96: 3950 / 113 / 500 -> 3511 / 92 / 421
+//   F = 192: 7775 / 197 / 940 -> 6800 / 167 / 755  F = 200: 8520 / 211 / 989 -> 7676 / 187 / 869
+//   F = 256: 9012 / 218 / 1025 -> 8694 / 202 / 943 F = 384: 15732 / 343 / 1719 -> 14075 / 309 / 1535
+//   F = 512: 18789 / 403 / 2007 -> 17948 / 390 / 1931; 600 as two passes of 96 vectors 637 -> 565 on the second
+// Rows of several passes: passes of 96 vectors where no more of them are needed than of 128 (a pass is paid in full).
+inline bool narrow_passes(int units) { return (units + 95) / 96 == (units + 127) / 128; }
+
 template <bool SO>
 void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
                    const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const float* H, int64_t ldH,
@@ -862,13 +862,23 @@ void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, cons
 #undef GC_NARROW
     return;
   }
-  if (units <= 4) GC_PIECES_SO(4, 1, 4, 4, SO);
-  else if (units <= 8) GC_PIECES_SO(4, 2, 4, 4, SO);  // F = 32: 1.54 ms; 8 lanes x 1 vector x 8 in flight: 1.73 ms
-  else if (units <= 12) GC_PIECES_SO(4, 3, 4, 4, SO);  // F = 48 on 126 M non-zeros: 2.24 ms against 2.35 ms with a fourth, idle vector
-  else if (units <= 16) GC_PIECES_SO(4, 4, 4, 4, SO);
-  else if (units <= 32) GC_PIECES_SO(8, 4, 4, 4, SO);
-  else if (units <= 64) GC_PIECES_SO(16, 4, 4, 4, SO);
-  else GC_PIECES_SO(32, 4, 4, 2, SO);
+  if (units <= 4) GC_PIECES(4, 1, 4, 4, 3, SO);
+  else if (units <= 8) GC_PIECES(4, 2, 4, 4, 3, SO);  // F = 32: 1.54 ms; 8 lanes x 1 vector x 8 in flight: 1.73 ms
+  else if (units <= 12) {
+    // Three CTAs where there are pieces for many waves (F = 48, 126 M non-zeros: 2.20 -> 2.10 ms; 600 K rows 273 -> 257
+    // us); on fewer the last wave is as long as the rest and two CTAs with more registers finish it sooner (169 K rows 60
+    // us against 70).
+    if (n_pieces >= gc::kNumSMs * 1536) GC_PIECES(4, 3, 4, 4, 3, SO);
+    else GC_PIECES(4, 3, 4, 4, 2, SO);
+  } else if (units <= 16) GC_PIECES(8, 2, 4, 4, 4, SO);
+  else if (units <= 24) GC_PIECES(8, 3, 4, 2, 3, SO);
+  else if (units <= 32) GC_PIECES(8, 4, 4, 4, 2, SO);
+  else if (units <= 48) GC_PIECES(16, 3, 4, 2, 4, SO);
+  else if (units <= 56) GC_PIECES(8, 7, 4, 2, 2, SO);
+  else if (units <= 64) GC_PIECES(8, 8, 4, 2, 2, SO);
+  else if (!SO && units > 96 && units <= 128) GC_PIECES(32, 4, 4, 2, 4, SO);  // odd widths: 3 CTAs, F = 385 534 / 544 us
+  else if (narrow_passes(units)) GC_PIECES(32, 3, 4, 2, 4, SO);
+  else GC_PIECES(32, 4, 4, 2, 3, SO);
 }
 
 void dispatch_scalar(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
@@ -881,27 +891,33 @@ void dispatch_scalar(bool planned, const int32_t* rowptr, const int32_t* col, co
     else GC_SHORT(16, 1, false);
     return;
   }
-  if (F <= 8) GC_PIECES(8, 1, 1, 4);
-  else if (F <= 16) GC_PIECES(16, 1, 1, 4);
-  else if (F <= 32) GC_PIECES(32, 1, 1, 4);
-  else if (F <= 64) GC_PIECES(32, 2, 1, 4);
-  else GC_PIECES(32, 4, 1, 4);
+  if (F <= 8) GC_PIECES(8, 1, 1, 4, 3, false);
+  else if (F <= 16) GC_PIECES(16, 1, 1, 4, 3, false);
+  else if (F <= 32) GC_PIECES(32, 1, 1, 4, 3, false);
+  else if (F <= 64) GC_PIECES(32, 2, 1, 4, 3, false);
+  else GC_PIECES(32, 4, 1, 4, 3, false);
 }
-// H in bf16: 8 elements per 16-byte vector; the same bytes in flight per lane as the fp32 mappings
-// (two accumulator vectors of 8 floats, up to 8 rows of H per round).
+// H in bf16: 8 elements per 16-byte vector.  As above the slots follow the width.  Measured (us, the same matrices),
+// two vectors per lane -> this: F = 96 3206 / 109 / 423 -> 2502 / 83 / 317, F = 128 3212 / 105 / 430 -> 3006 / 97 / 375,
+// F = 192 6483 / 181 / 785 -> 4782 / 138 / 580, F = 256 6714 / 187 / 811 -> 5870 / 162 / 696, F = 384 13171 / 315 / 1454
+// -> 9908 / 231 / 1080, F = 512 14036 / 335 / 1531 -> 12857 / 305 / 1393, F = 640 - / 564 / 2772 -> - / 436 / 2148.
 void dispatch_bf16(bool planned, const int32_t* rowptr, const int32_t* col, const float* val, int n_pieces,
                    const int32_t* ps, const int32_t* pl, const int32_t* pt, int F, const uint16_t* H, int64_t ldH,
                    float* Y, int64_t ldY, float* scratch, int64_t ldS, int cap, int32_t* ovf, const Epilogue& ep,
                    const RowBlocks& rb, cudaStream_t st) {
   const int units = F / 8;
-  if (units <= 4) GC_PIECES(4, 1, 8, 4);
-  else if (units <= 8) GC_PIECES(4, 2, 8, 4);
-  else if (units <= 16) GC_PIECES(8, 2, 8, 8);
-  else if (units <= 32) GC_PIECES(16, 2, 8, 8);
-  else GC_PIECES(32, 2, 8, 4);
+  if (units <= 4) GC_PIECES(4, 1, 8, 4, 3, false);
+  else if (units <= 8) GC_PIECES(4, 2, 8, 4, 2, false);
+  else if (units <= 12) GC_PIECES(4, 3, 8, 4, 2, false);
+  else if (units <= 16) GC_PIECES(4, 4, 8, 4, 2, false);
+  else if (units <= 24) GC_PIECES(8, 3, 8, 4, 2, false);
+  else if (units <= 32) GC_PIECES(8, 4, 8, 4, 2, false);
+  else if (units <= 48) GC_PIECES(16, 3, 8, 2, 3, false);
+  else if (units <= 64) GC_PIECES(16, 4, 8, 4, 2, false);
+  else if (narrow_passes(units)) GC_PIECES(32, 3, 8, 2, 3, false);
+  else GC_PIECES(32, 4, 8, 4, 2, false);
 }
 #undef GC_PIECES
-#undef GC_PIECES_SO
 #undef GC_SHORT
 
 inline int64_t scratch_ld(int64_t F) { return (F + 3) & ~int64_t(3); }
