@@ -15,7 +15,7 @@
 // Splits across CTAs are added in order, by a cluster through distributed
 // shared memory when one cluster covers the output, else by a second kernel.
 // Bound: latency of a few dependent loads, then instruction issue.  Measured:
-// 2708 x 16 x 1433 19.8 -> 12.1 us, 1433 x 16 x 2708 24.9 -> 12.8 us,
+// 2708 x 16 x 1433 19.8 -> 12.1 us, 1433 x 16 x 2708 24.9 -> 10.6 us,
 // 16 x 7 x 2708 14.1 -> 5.3 us.
 #include "common.cuh"
 #include "gemm_internal.cuh"
@@ -239,8 +239,9 @@ MPlan m_plan(int64_t M, int64_t N, int64_t K) {
   MPlan pl{};
   pl.r = M <= 32 ? 1 : 2;
   const int64_t tiles = ceil_div(M, 32 * pl.r);
-  // about 16 warps per SM, at least 16 k-values per warp
-  int64_t s = std::min<int64_t>(ceil_div(2 * gc::kNumSMs, tiles), std::max<int64_t>(1, K / 128));
+  // Two CTAs per SM and not one more (299 of them for 296 places: 1433 x 16 x 2708 12.7 us, 276 10.6; 3703 x 16 x 3327
+  // 26.8 and 22.3), at least 16 k-values per warp.
+  int64_t s = std::min<int64_t>(std::max<int64_t>(1, 2 * gc::kNumSMs / tiles), std::max<int64_t>(1, K / 128));
   pl.cluster = tiles == 1 && s > 1 && K <= 8192;
   if (pl.cluster) s = s >= 8 ? 8 : s >= 4 ? 4 : 2;
   pl.splits = int(s);
