@@ -220,10 +220,12 @@ void spmm_into(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, 
     if (a.K > 0 && ldh % 4 == 0 && ldh >= f4 && reinterpret_cast<uintptr_t>(H) % 16 == 0 &&
         last <= int64_t(Hin.storage().nbytes())) {
       epi |= GC_EPI_H_PADDED;  // a view of wider rows: what lies beyond the width may be read, and is not used
-    } else if (F > 8 && a.nnz >= 4 * a.K && a.nnz >= (1 << 16)) {
+    } else if (F > 8 && a.nnz >= 4 * a.K && a.nnz >= (F <= 32 ? 1 << 16 : F <= 64 ? 1 << 18 : F <= 256 ? 5 << 17 : 1 << 17)) {
       // Rows that are not 16-byte aligned are gathered one float per lane.  Copying H to an aligned pitch first (8
       // bytes per element, streamed) pays where every row is gathered several times: 169 K rows of 47, 15 non-zeros
-      // each, 136 us against 9 + 68.
+      // each, 136 us against 9 + 68.  On small graphs the copy's launch and the wider stores cost more than the scalar
+      // gathers at 65 to 256 columns (us, copied / as it is: 16.5 K rows, 96 K non-zeros F = 87 26 / 19, 468 K 35 / 31,
+      // 40 K rows, 840 K non-zeros 45 / 49) and, on smaller ones still, at 33 to 64 (F = 47: 19 / 16, 22 / 24, 34 / 40).
       padded = empty_f32(a.K, f4, dev);
       check(abi.gc_pad_rows_f32(static_cast<const float*>(H), ldh, padded.data_ptr<float>(), f4, a.K, F, stream_of(dev)),
             "gc_pad_rows_f32");
