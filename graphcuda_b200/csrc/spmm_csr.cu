@@ -856,6 +856,7 @@ void launch_short(bool planned, const int32_t* rowptr, const int32_t* col, const
 //   F =  64: 2638 / 73 / 365 -> 2486 / 68 / 297    F =  96: 3950 / 113 / 500 -> 3511 / 92 / 421
 //   F = 192: 7775 / 197 / 940 -> 6800 / 167 / 755  F = 200: 8520 / 211 / 989 -> 7676 / 187 / 869
 //   F = 256: 9012 / 218 / 1025 -> 8694 / 202 / 943 F = 384: 15732 / 343 / 1719 -> 14075 / 309 / 1535
+//   F = 100: 4520 / 122 / 861 -> 4356 / 105 / 819   F = 128: 4430 / 124 / 848 -> 4301 / 112 / 812 (three CTAs for two)
 //   F = 512: 18789 / 403 / 2007 -> 17948 / 390 / 1931; 600 as two passes of 96 vectors 637 -> 565 on the second
 // Rows of several passes: passes of 96 vectors where no more of them are needed than of 128 (a pass is paid in full).
 inline bool narrow_passes(int units) { return (units + 95) / 96 == (units + 127) / 128; }
@@ -916,7 +917,7 @@ void dispatch_vec4(bool planned, const int32_t* rowptr, const int32_t* col, cons
     else GC_PIECES(4, 3, 4, 4, 2, SO);
   } else if (units <= 16) GC_PIECES(8, 2, 4, 4, 4, SO);
   else if (units <= 24) GC_PIECES(8, 3, 4, 2, 3, SO);
-  else if (units <= 32) GC_PIECES(8, 4, 4, 4, 2, SO);
+  else if (units <= 32) GC_PIECES(8, 4, 4, 4, 3, SO);
   else if (units <= 48) GC_PIECES(16, 3, 4, 2, 4, SO);
   else if (units <= 64 && n_pieces <= gc::kNumSMs * 512)
     GC_PIECES(16, 4, 4, 3, 3, SO);  // few pieces: more lanes on each (40 K rows, 840 K non-zeros, F = 256: 83 -> 71 us)
