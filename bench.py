@@ -135,33 +135,25 @@ class ClockSampler:
 
 # ---------------------------------------------------------------- SpMM timer
 class SpmmTimer:
-    """CUDA-event pairs around every CSR aggregation enqueued while active
-    (events are recorded on the stream the kernels run on)."""
+    """Device times of every CSR aggregation enqueued while active: the native host side brackets each with CUDA events
+    on the stream the kernels run on; the ones that store into other GPUs' buffers are wrapped here."""
 
     def __init__(self):
         self.records = []
-        self.active = False
+        self._active = False
+
+    @property
+    def active(self):
+        return self._active
+
+    @active.setter
+    def active(self, on):
+        from graphcuda_b200 import _lib
+        self._active = on
+        _lib.host.record_spmm(on)
 
     def wrap(self, cls):
         timer = self
-        orig = cls.matmul
-
-        def timed(self_adj, H, **kw):
-            if not timer.active:
-                return orig(self_adj, H, **kw)
-            a = torch.cuda.Event(enable_timing=True)
-            b = torch.cuda.Event(enable_timing=True)
-            a.record()
-            out = orig(self_adj, H, **kw)
-            b.record()
-            M, K = self_adj.shape
-            F = H.size(1)
-            # algorithmic (compulsory) bytes: rowptr + col + val + H read once + Y written once
-            nbytes = 4 * (M + 1) + 8 * self_adj.nnz + 4 * K * F + 4 * M * F
-            timer.records.append((a, b, nbytes, F, self_adj.nnz))
-            return out
-
-        cls.matmul = timed
         orig_blocks = cls.matmul_into_blocks
 
         def timed_blocks(self_adj, H, *a, **kw):  # the aggregation whose stores go to the owners' buffers
@@ -182,8 +174,12 @@ class SpmmTimer:
     def summary(self):
         tot_ms, tot_b, gather_b = 0.0, 0, 0
         per_f = {}
-        for a, b, nbytes, F, nnz in self.records:
-            ms = a.elapsed_time(b)
+        from graphcuda_b200 import _lib
+        # algorithmic (compulsory) bytes: rowptr + col + val + H read once + Y written once
+        timed = [(ms, 4 * (M + 1) + 8 * nnz + 4 * K * F + 4 * M * F, F, nnz)
+                 for ms, M, K, F, nnz in _lib.host.take_spmm_records()]
+        timed += [(a.elapsed_time(b), nbytes, F, nnz) for a, b, nbytes, F, nnz in self.records]
+        for ms, nbytes, F, nnz in timed:
             tot_ms += ms
             tot_b += nbytes
             gather_b += nbytes + 4 * nnz * F
@@ -191,7 +187,7 @@ class SpmmTimer:
             d[0] += ms
             d[1] += nbytes
             d[2] += 1
-        return tot_ms, tot_b, gather_b, per_f, len(self.records)
+        return tot_ms, tot_b, gather_b, per_f, len(timed)
 
 
 def gather_ceiling(dev, n_rows_h: int, F: int = 256):

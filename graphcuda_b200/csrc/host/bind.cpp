@@ -228,6 +228,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("edges_to_csr", &edges_to_csr, NoGil());
 
   m.def("padded_width", &padded_width);
+  m.def("record_spmm", &record_spmm);
+  m.def("take_spmm_records", &take_spmm_records, NoGil());
   m.def("zero_padded_base", &zero_padded_base);
   m.def("register_zero_padded", &register_zero_padded);
   m.def("zero_padded_count", &zero_padded_count);

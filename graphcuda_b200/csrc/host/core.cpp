@@ -3,7 +3,10 @@
 
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <dlfcn.h>
+
+#include <atomic>
 
 #include <unordered_map>
 
@@ -203,7 +206,51 @@ bool Adj::is_symmetric() {
   return symmetric != 0;
 }
 
+// Device times of the aggregations issued while recording is on: the layers call them without passing through Python,
+// where a benchmark would otherwise put its events.
+namespace {
+struct SpmmRecord {
+  at::cuda::CUDAEvent begin{cudaEventDefault}, end{cudaEventDefault};
+  int64_t M, K, F, nnz;
+};
+std::atomic<bool> spmm_recording{false};
+std::mutex spmm_records_mutex;
+std::vector<SpmmRecord>& spmm_record_list() {
+  static auto* v = new std::vector<SpmmRecord>();
+  return *v;
+}
+}  // namespace
+
+void record_spmm(bool on) { spmm_recording = on; }
+
+// (ms, M, K, F, nnz) of every recorded aggregation, waiting for the last; clears the list.
+std::vector<std::tuple<double, int64_t, int64_t, int64_t, int64_t>> take_spmm_records() {
+  const std::lock_guard<std::mutex> lock(spmm_records_mutex);
+  std::vector<std::tuple<double, int64_t, int64_t, int64_t, int64_t>> out;
+  for (auto& r : spmm_record_list()) {
+    r.end.synchronize();
+    out.emplace_back(r.begin.elapsed_time(r.end), r.M, r.K, r.F, r.nnz);
+  }
+  spmm_record_list().clear();
+  return out;
+}
+
+static void spmm_launch(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, bool accumulate,
+                        int64_t panel_cols);
+
 void spmm_into(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, bool accumulate, int64_t panel_cols) {
+  if (!spmm_recording.load(std::memory_order_relaxed)) return spmm_launch(a, Hin, Y, ldy, ep, accumulate, panel_cols);
+  const auto st = at::cuda::getCurrentCUDAStream(a.device().index());
+  SpmmRecord r;
+  r.M = a.M; r.K = a.K; r.F = Hin.size(1); r.nnz = a.nnz;
+  r.begin.record(st);
+  spmm_launch(a, Hin, Y, ldy, ep, accumulate, panel_cols);
+  r.end.record(st);
+  const std::lock_guard<std::mutex> lock(spmm_records_mutex);
+  spmm_record_list().push_back(std::move(r));
+}
+
+static void spmm_launch(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, bool accumulate, int64_t panel_cols) {
   const at::Device dev = a.device();
   const int64_t F = Hin.size(1);
   const bool h16 = Hin.scalar_type() == at::kBFloat16;

@@ -125,6 +125,8 @@ using AdjPtr = c10::intrusive_ptr<Adj>;
 
 // Y = A H (+bias)(ReLU)(mask)(gate); H is float32 (or bfloat16) with unit column stride.
 void spmm_into(Adj& a, const Tensor& H, float* Y, int64_t ldy, const Epi& ep, bool accumulate, int64_t panel_cols);
+void record_spmm(bool on);
+std::vector<std::tuple<double, int64_t, int64_t, int64_t, int64_t>> take_spmm_records();
 Tensor adj_matmul(Adj& a, Tensor H, int prec, const Epi& ep);
 
 // ------------------------------------------------------------------ graphs
