@@ -55,6 +55,7 @@ SIGNATURES = {
                                 _void, _size, _void]),
     "gc_gemm_resolve_precision": (_int, [_int, _int, _i64, _i64, _i64, _i64, _i64, _i64, _int]),
     "gc_gemm_check_flag": (_int, [_void, _void]),
+    "gc_gemm_error_word": (_int, [_void]),
     "gc_gcn_layer_workspace_bytes": (_size, [_i64, _i64, _i64, _i64, _int, _int]),
     "gc_gcn_conv_forward_csr_f32": (_int, [_i32p, _i32p, _f32p, _i64, _i64, _i64, _f32p, _i64, _f32p, _i64, _f32p,
                                            _int, _f32p, _i64, _f32p, _f32p, _i64, _void, _i64, _i64, _i64, _int,

@@ -118,6 +118,11 @@ int gc_gemm_bf16_f32(int64_t M, int64_t N, int64_t K, const uint16_t* A, int64_t
   return gc::gemm_bf16_core(M, N, K, A, lda, Bt, ldb, C, ldc, ep, workspace, workspace_bytes, gc::as_stream(stream));
 }
 
+int gc_gemm_error_word(int32_t** word) {
+  GC_REQUIRE(word, "gc_gemm_error_word: null pointer");
+  return gc::wait_error_word(word);
+}
+
 int gc_gemm_check_flag(const void* workspace, void* stream) {
   GC_REQUIRE(workspace, "gc_gemm_check_flag: null workspace");
   int h = 0;

@@ -43,6 +43,7 @@ int splitk_reduce(int M, int N, int splits, const float* partial, float* C, int6
                   cudaStream_t st);
 
 // Tensor-core path (gemm_tcgen05.cu)
+int wait_error_word(int32_t** word);
 bool tc_supported(bool ta, bool tb, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc);
 size_t tc_workspace_bytes(bool ta, bool tb, int64_t M, int64_t N, int64_t K, int passes);
 int gemm_tc(bool ta, bool tb, int64_t M, int64_t N, int64_t K, const float* A, int64_t lda, const float* B,

@@ -225,6 +225,10 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int bm, int bn) {
          | (uint32_t(bm >> 4) << 24);  // M / 16
 }
 
+// Set when a wait of any launch on this GPU ran out, beside the word in that launch's workspace: a workspace may be the
+// launch's own (a recorded launch takes it from the graph's memory), and then nobody reads it.
+__device__ int g_wait_ran_out;
+
 struct TcParams {
   int M, N, K;
   float* C;
@@ -619,7 +623,10 @@ gemm_tf32_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant
   if (PAIR) cluster_sync_all();  // the peer's MMAs read this CTA's shared memory and write its TMEM until here
   tc_fence_after();
   if (warp == 2) tmem_dealloc<PAIR>(tmem_base, C_::kTmemCols);
-  if (threadIdx.x == 0 && abort_s && p.flag) atomicExch(p.flag, 1);
+  if (threadIdx.x == 0 && abort_s) {
+    atomicExch(p.flag, 1);
+    atomicExch(&g_wait_ran_out, 1);
+  }
 }
 
 // B_lo = B - trunc19(B) over an R x Kc view.
@@ -926,6 +933,14 @@ int launch_layout(const Plan& pl, const CUtensorMap& mA, const CUtensorMap& mB, 
 }  // namespace
 
 namespace gc {
+
+int wait_error_word(int32_t** word) {
+  void* p = nullptr;
+  const cudaError_t e = cudaGetSymbolAddress(&p, g_wait_ran_out);
+  if (e != cudaSuccess) return fail(GC_ERR_CUDA, "gc_gemm_error_word: %s", cudaGetErrorString(e));
+  *word = static_cast<int32_t*>(p);
+  return GC_OK;
+}
 
 int splitk_reduce(int M, int N, int splits, const float* partial, float* C, int64_t ldc, const GemmEpilogue& ep,
                   cudaStream_t st) {

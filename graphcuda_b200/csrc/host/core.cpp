@@ -65,9 +65,7 @@ Tensor scratch_buffer(Tag tag, size_t bytes, const at::Device& dev) {
   Tensor& b = buffers()[Key{dev.index(), stream.stream()}].buf[tag];
   if (!b.defined() || size_t(b.numel()) < bytes) {
     const size_t size = std::max<size_t>(256, (bytes + bytes / 4 + 255) & ~size_t(255));  // growth is rare
-    Tensor n = bytes_on(size, dev).zero_();
-    if (b.defined()) n.narrow(0, 0, 256).copy_(b.narrow(0, 0, 256));
-    b = n;
+    b = bytes_on(size, dev);
   }
   return b;
 }

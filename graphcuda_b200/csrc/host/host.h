@@ -51,10 +51,10 @@ void check(int status, const char* what);
 
 // ------------------------------------------------------------------ scratch
 // Grow-only scratch, one buffer per (device, stream, tag).  Kernels of one stream run in order, so a buffer is never
-// in use by two launches at once.  New buffers are zero-filled and the first 256 bytes move along when a buffer grows:
-// the GEMM keeps a sticky error word there.  While a stream is being captured the scratch is allocated for that call
-// alone, from the graph's own pool: a buffer shared with eager launches could be outgrown and released while the graph
-// still replays on it.
+// in use by two launches at once.  While a stream is being captured the scratch is allocated for that call alone, from
+// the graph's own pool: a buffer shared with eager launches could be outgrown and released while the graph still
+// replays on it.  Nothing in a buffer outlives its call: what a tensor-core GEMM reports about a wait that ran out is
+// read from the device's own word (gc_gemm_error_word).
 enum Tag { kGemm = 0, kSpmm = 1, kTags = 2 };
 struct Scratch {
   void* ptr;

@@ -136,9 +136,13 @@ def gemm_path(A: torch.Tensor, B: torch.Tensor, precision: Optional[str] = None)
 
 
 def check_gemm_flag(device: torch.device) -> None:
-    """Raises if a tensor-core GEMM on this device/stream gave up a bounded wait."""
-    ws = arena.get("gemm", 256, device)
-    _lib.check(_lib.lib().gc_gemm_check_flag(ws.data_ptr(), _stream(device)), "gc_gemm_check_flag")
+    """Raises if a tensor-core GEMM of this process on this device -- issued or replayed, on any stream -- gave up a
+    bounded wait.  Waits for the current stream."""
+    import ctypes
+    word = ctypes.c_void_p()
+    with torch.cuda.device(device):
+        _lib.check(_lib.lib().gc_gemm_error_word(ctypes.byref(word)), "gc_gemm_error_word")
+        _lib.check(_lib.lib().gc_gemm_check_flag(word, _stream(device)), "gc_gemm_check_flag")
 
 
 # ---------------------------------------------------------------- element-wise

@@ -291,6 +291,11 @@ int gc_gemm_bf16_f32(int64_t M, int64_t N, int64_t K,
  * at the start of the workspace.  Synchronises `stream`, reads it back and
  * returns GC_OK or GC_ERR_DEVICE_FLAG (debug / test use). */
 int gc_gemm_check_flag(const void* workspace, void* stream);
+/* *word <- the address, on the current device, of the word that every such
+ * launch on that device sets as well, whichever workspace it was given (one for
+ * the process, never cleared by the library): gc_gemm_check_flag(*word, stream)
+ * tells whether a wait has run out on the device, recorded launches included. */
+int gc_gemm_error_word(int32_t** word);
 
 /* ---- the layer as one call (reference gcn.cu:5-52) ------------------------ */
 
