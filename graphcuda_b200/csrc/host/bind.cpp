@@ -218,7 +218,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("use_plan", &Adj::use_plan)
       .def_readwrite("segment", &Adj::segment)
       .def_readwrite("A16", &Adj::A16)
-      .def_readwrite("symmetric", &Adj::symmetric)
+      .def_property("symmetric", [](const Adj& a) { return a.symmetric.load(); }, [](Adj& a, int v) { a.symmetric = v; })
       .def("is_symmetric", &Adj::is_symmetric, NoGil())
       .def("plan_for", &Adj::plan_for, NoGil());
   m.def("csr", &make_csr);

@@ -188,6 +188,8 @@ std::shared_ptr<Plan> Adj::plan_for(int64_t F, int64_t panel_cols) {
 
 bool Adj::is_symmetric() {
   if (symmetric < 0) {
+    std::lock_guard<std::mutex> lock(symmetry_mutex_);
+    if (symmetric >= 0) return symmetric != 0;
     if (M != K) {
       symmetric = 0;
     } else if (dense) {

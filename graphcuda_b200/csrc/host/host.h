@@ -11,6 +11,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/custom_class.h>
 
+#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -104,7 +105,7 @@ struct Plan {
 struct Adj : torch::CustomClassHolder {
   bool dense = false;
   int64_t M = 0, K = 0, nnz = 0;
-  int symmetric = -1;  // -1: not known yet
+  std::atomic<int> symmetric{-1};  // -1: not known yet
   // CSR
   Tensor rowptr, col, val;
   bool use_plan = true;
@@ -117,7 +118,8 @@ struct Adj : torch::CustomClassHolder {
   bool is_symmetric();
 
  private:
-  std::mutex mutex_;
+  std::mutex mutex_;           // the plans
+  std::mutex symmetry_mutex_;  // held while the verdict is found, so that it is found once
   std::map<std::pair<int64_t, int64_t>, std::shared_ptr<Plan>> plans_;  // by panel width and segment
   std::map<int64_t, std::shared_ptr<Plan>> by_width_;  // by F, default panel width
 };
