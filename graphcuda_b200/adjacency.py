@@ -18,7 +18,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from .ops import _require, _stream, arena, EPI_RELU
+from .ops import _require, _stream, EPI_RELU
 
 
 class CSRAdjacency:
@@ -113,7 +113,7 @@ class CSRAdjacency:
             plan = self.plan_for(F, panel_cols) if self.use_plan else None
             scratch = None
             if plan is not None and plan.n_cut > 0:
-                scratch = arena.get("spmm", L.gc_spmm_scratch_bytes(plan.n_slots, F), dev)
+                scratch = torch.empty(L.gc_spmm_scratch_bytes(plan.n_slots, F), dtype=torch.uint8, device=dev)
             ldh = H.stride(0) if H.size(0) > 1 else max(F, 1)
             st = L.gc_spmm_csr_f32_blocks(self.rowptr.data_ptr(), self.col.data_ptr(), self.val.data_ptr(), M, K, F,
                                           H.data_ptr(), ldh, bias.data_ptr() if bias is not None else None,

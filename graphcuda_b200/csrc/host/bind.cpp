@@ -193,14 +193,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("spmm", &spmm);
   m.def("relu_backward", &relu_backward, NoGil());
   m.def("mask_mul", &mask_mul, NoGil());
-  m.def("scratch_buffer", [](int tag, size_t bytes, int device) {
-    const at::Device dev(at::kCUDA, c10::DeviceIndex(device));
-    const c10::cuda::CUDAGuard guard(dev);
-    return scratch_buffer(Tag(tag), bytes, dev);
-  }, NoGil());
   m.def("scratch_clear", &scratch_clear, NoGil());
-  m.attr("GEMM") = int(kGemm);
-  m.attr("SPMM") = int(kSpmm);
 
   py::class_<Plan, std::shared_ptr<Plan>>(m, "SpmmPlan")
       .def_readonly("buf", &Plan::buf)

@@ -43,11 +43,16 @@ struct Key {
 struct KeyHash {
   size_t operator()(const Key& k) const { return std::hash<void*>()(k.stream) * 31 + size_t(k.device); }
 };
+struct Buffer {
+  std::mutex turn;  // held from the first launch that uses the buffer to the last of the same call
+  Tensor mem;
+};
 struct Buffers {
-  Tensor buf[kTags];
+  Buffer of[kTags];
 };
 std::mutex scratch_mutex;
-// Never destroyed: the tensors must not outlive torch's allocator at process exit.
+// Never destroyed: the tensors must not outlive torch's allocator at process exit.  Entries stay when their memory is
+// given back: another thread may be waiting for its turn.
 std::unordered_map<Key, Buffers, KeyHash>& buffers() {
   static auto* m = new std::unordered_map<Key, Buffers, KeyHash>();
   return *m;
@@ -57,27 +62,35 @@ Tensor bytes_on(size_t n, const at::Device& dev) {
 }
 }  // namespace
 
-Tensor scratch_buffer(Tag tag, size_t bytes, const at::Device& dev) {
-  const auto stream = at::cuda::getCurrentCUDAStream(dev.index());
-  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-    return bytes_on(std::max<size_t>(256, bytes), dev);
-  std::lock_guard<std::mutex> lock(scratch_mutex);
-  Tensor& b = buffers()[Key{dev.index(), stream.stream()}].buf[tag];
-  if (!b.defined() || size_t(b.numel()) < bytes) {
-    const size_t size = std::max<size_t>(256, (bytes + bytes / 4 + 255) & ~size_t(255));  // growth is rare
-    b = bytes_on(size, dev);
-  }
-  return b;
-}
-
 Scratch scratch(Tag tag, size_t bytes, const at::Device& dev) {
-  Tensor t = scratch_buffer(tag, bytes, dev);
-  return Scratch{t.data_ptr(), size_t(t.numel()), t};
+  Scratch s;
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+    s.keep = bytes_on(std::max<size_t>(256, bytes), dev);
+  } else {
+    Buffer* b;
+    {
+      std::lock_guard<std::mutex> lock(scratch_mutex);
+      b = &buffers()[Key{dev.index(), at::cuda::getCurrentCUDAStream(dev.index()).stream()}].of[tag];
+    }
+    s.turn = std::unique_lock<std::mutex>(b->turn);
+    if (!b->mem.defined() || size_t(b->mem.numel()) < bytes) {
+      const size_t size = std::max<size_t>(256, (bytes + bytes / 4 + 255) & ~size_t(255));  // growth is rare
+      b->mem = bytes_on(size, dev);
+    }
+    s.keep = b->mem;
+  }
+  s.ptr = s.keep.data_ptr();
+  s.bytes = size_t(s.keep.numel());
+  return s;
 }
 
 void scratch_clear() {
   std::lock_guard<std::mutex> lock(scratch_mutex);
-  buffers().clear();
+  for (auto& entry : buffers())
+    for (Buffer& b : entry.second.of) {
+      std::lock_guard<std::mutex> turn(b.turn);
+      b.mem = Tensor();
+    }
 }
 
 // ------------------------------------------------------------------ layouts
@@ -255,7 +268,7 @@ static void spmm_launch(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const 
   const int64_t F = Hin.size(1);
   const bool h16 = Hin.scalar_type() == at::kBFloat16;
   std::shared_ptr<Plan> plan = a.use_plan ? a.plan_for(F, panel_cols) : nullptr;
-  Scratch s{nullptr, 0, Tensor()};
+  Scratch s;
   if (plan && plan->n_cut > 0) s = scratch(kSpmm, abi.gc_spmm_scratch_bytes(plan->n_slots, F), dev);
   int epi = (ep.relu ? GC_EPI_RELU : 0) | (accumulate ? GC_EPI_ACCUMULATE : 0);
   const void* H = Hin.data_ptr();

@@ -52,18 +52,20 @@ void check(int status, const char* what);
 
 // ------------------------------------------------------------------ scratch
 // Grow-only scratch, one buffer per (device, stream, tag).  Kernels of one stream run in order, so a buffer is never
-// in use by two launches at once.  While a stream is being captured the scratch is allocated for that call alone, from
+// in use by two launches at once -- provided the launches of one call follow each other on the stream.  Several threads
+// may issue on one stream, so a Scratch holds its buffer until it is destroyed: keep it until the call that uses it has
+// returned, and take no second one of the same tag meanwhile.  While a stream is being captured the scratch is allocated for that call alone, from
 // the graph's own pool: a buffer shared with eager launches could be outgrown and released while the graph still
 // replays on it.  Nothing in a buffer outlives its call: what a tensor-core GEMM reports about a wait that ran out is
 // read from the device's own word (gc_gemm_error_word).
 enum Tag { kGemm = 0, kSpmm = 1, kTags = 2 };
 struct Scratch {
-  void* ptr;
-  size_t bytes;
-  Tensor keep;  // holds a per-call buffer
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  Tensor keep;  // a per-call buffer, or one that another thread has outgrown by now
+  std::unique_lock<std::mutex> turn;
 };
 Scratch scratch(Tag tag, size_t bytes, const at::Device& dev);
-Tensor scratch_buffer(Tag tag, size_t bytes, const at::Device& dev);
 void scratch_clear();
 
 inline void* stream_of(const at::Device& dev) { return at::cuda::getCurrentCUDAStream(dev.index()).stream(); }

@@ -51,12 +51,8 @@ def _prec(precision: Optional[str]) -> int:
 class _Arena:
     """Grow-only scratch buffers of the native host side, one set per (device, stream, tag) -- see csrc/host/host.h."""
 
-    def get(self, tag: str, nbytes: int, device: torch.device) -> torch.Tensor:
-        h = _lib.host
-        index = device.index if device.index is not None else torch.cuda.current_device()
-        return h.scratch_buffer({"gemm": h.GEMM, "spmm": h.SPMM}[tag], nbytes, index)
-
     def clear(self):
+        """Gives the buffers back to torch's allocator."""
         _lib.host.scratch_clear()
 
 
