@@ -52,10 +52,11 @@ class CSRAdjacency:
     def segment(self, value: Optional[int]) -> None:
         self._h.segment = int(value or 0)
 
-    def plan_for(self, F: int, panel_cols: Optional[int] = None):
+    def plan_for(self, F: int, panel_cols: Optional[int] = None, segment: Optional[int] = None):
         """The processing plan for feature width F (built on first use and kept): buf, n_pieces, n_slots, n_cut,
-        panel_cols."""
-        return self._h.plan_for(F, int(panel_cols or 0))
+        panel_cols.  segment: the longest piece of this plan alone.  A plan for gc_spmm_csr_f32_noalloc, whose scratch
+        is limited, wants long pieces (gc_spmm_default_segment(nnz), or up to 2048) rather than the fast ones."""
+        return self._h.plan_for(F, int(panel_cols or 0), int(segment or 0))
 
     @property
     def symmetric(self) -> bool:

@@ -213,7 +213,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readwrite("A16", &Adj::A16)
       .def_property("symmetric", [](const Adj& a) { return a.symmetric.load(); }, [](Adj& a, int v) { a.symmetric = v; })
       .def("is_symmetric", &Adj::is_symmetric, NoGil())
-      .def("plan_for", &Adj::plan_for, NoGil());
+      .def("plan_for", &Adj::plan_for, py::arg("F"), py::arg("panel_cols") = 0, py::arg("segment") = 0, NoGil());
   m.def("csr", &make_csr);
   m.def("dense", &make_dense);
 

@@ -154,15 +154,15 @@ void gemm_bf16_into(const Tensor& A16, const Tensor& Bt16, float* C, int64_t ldc
 }
 
 // ------------------------------------------------------------------ CSR
-std::shared_ptr<Plan> Adj::plan_for(int64_t F, int64_t panel_cols) {
+std::shared_ptr<Plan> Adj::plan_for(int64_t F, int64_t panel_cols, int64_t segment_len) {
   std::lock_guard<std::mutex> lock(mutex_);
-  const bool standard = panel_cols <= 0;
+  const bool standard = panel_cols <= 0 && segment_len <= 0;
   if (standard) {
     auto it = by_width_.find(F);
     if (it != by_width_.end()) return it->second;
-    panel_cols = abi.gc_spmm_default_panel_cols(K, std::max<int64_t>(F, 1));
   }
-  const int64_t seg = segment > 0 ? segment : abi.gc_spmm_segment(nnz, F);
+  if (panel_cols <= 0) panel_cols = abi.gc_spmm_default_panel_cols(K, std::max<int64_t>(F, 1));
+  const int64_t seg = segment_len > 0 ? segment_len : segment > 0 ? segment : abi.gc_spmm_segment(nnz, F);
   const auto key = std::make_pair(panel_cols, seg);
   auto hit = plans_.find(key);
   std::shared_ptr<Plan> p = hit != plans_.end() ? hit->second : nullptr;

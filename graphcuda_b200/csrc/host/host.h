@@ -116,7 +116,7 @@ struct Adj : torch::CustomClassHolder {
   Tensor A, A16;
 
   at::Device device() const { return dense ? A.device() : val.device(); }
-  std::shared_ptr<Plan> plan_for(int64_t F, int64_t panel_cols = 0);
+  std::shared_ptr<Plan> plan_for(int64_t F, int64_t panel_cols = 0, int64_t segment_len = 0);
   bool is_symmetric();
 
  private:

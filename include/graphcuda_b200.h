@@ -82,7 +82,7 @@ int gc_pad_rows_f32(const float* src, int64_t ld_src, float* dst, int64_t ld_dst
 /* Segment length for a plan that serves products of feature width F: in
  * [128, GC_SPMM_SEGMENT_MAX], growing with the square root of nnz.  Shorter than
  * the default above on large matrices, where it bounds the time of the longest
- * piece. */
+ * piece; more partial-sum rows come with it (see gc_spmm_csr_f32_noalloc). */
 int64_t gc_spmm_segment(int64_t nnz, int64_t F);
 /* Scratch for plan construction; pass n_pieces = 0 for gc_spmm_plan_count. */
 size_t gc_spmm_plan_workspace_bytes(int64_t M, int64_t n_pieces);
@@ -210,7 +210,11 @@ int gc_gather_sum_f32(const float* H, int64_t ldH, int64_t K, int64_t F,
  *
  *  - Limit: gc_spmm_scratch_bytes(n_slots, F) must not exceed
  *    GC_SPMM_STATIC_SCRATCH_BYTES; larger problems are refused with
- *    GC_ERR_WORKSPACE and a message, never truncated.
+ *    GC_ERR_WORKSPACE and a message, never truncated.  n_slots falls with the
+ *    segment length of the plan: build it with gc_spmm_default_segment, or with
+ *    anything up to GC_SPMM_SEGMENT_MAX.  gc_spmm_segment is chosen for speed
+ *    and on matrices of more than about a million non-zeros cuts shorter, so
+ *    that its plan may not fit where those do.
  *  - The first call on a device looks up the buffer's device address
  *    (cudaGetSymbolAddress) with that device current; make that first call
  *    outside any stream capture.  The device that owns `stream` must be the
