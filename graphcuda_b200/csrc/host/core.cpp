@@ -263,6 +263,18 @@ void spmm_into(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, 
   spmm_record_list().push_back(std::move(r));
 }
 
+// Whether H is copied to an aligned pitch first.  Rows that are not 16-byte aligned are gathered one float per lane; the
+// copy (8 bytes per element, streamed) pays where every row is gathered several times: 169 K rows of 47, 15 non-zeros each,
+// 136 us against 9 + 68.  On small graphs the copy's launch and the wider stores cost more than the scalar gathers at 65
+// to 256 columns (us, copied / as it is: 16.5 K rows, 96 K non-zeros F = 87 26 / 19, 468 K 35 / 31, 40 K rows, 840 K
+// non-zeros 45 / 49) and, on smaller ones still, at 33 to 64 (F = 47: 19 / 16, 22 / 24, 34 / 40).
+static bool copy_pays(int64_t F, int64_t K, int64_t nnz) {
+  return F > 8 && nnz >= 4 * K && nnz >= (F <= 32 ? 1 << 16 : F <= 64 ? 1 << 18 : F <= 256 ? 5 << 17 : 1 << 17);
+}
+
+// Largest such copy at a time; wider matrices take it in slabs of columns.
+constexpr int64_t kCopyBytes = int64_t(1) << 30;
+
 static void spmm_launch(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, bool accumulate, int64_t panel_cols) {
   const at::Device dev = a.device();
   const int64_t F = Hin.size(1);
@@ -270,44 +282,49 @@ static void spmm_launch(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const 
   std::shared_ptr<Plan> plan = a.use_plan ? a.plan_for(F, panel_cols) : nullptr;
   Scratch s;
   if (plan && plan->n_cut > 0) s = scratch(kSpmm, abi.gc_spmm_scratch_bytes(plan->n_slots, F), dev);
-  int epi = (ep.relu ? GC_EPI_RELU : 0) | (accumulate ? GC_EPI_ACCUMULATE : 0);
-  const void* H = Hin.data_ptr();
-  int64_t ldh = Hin.size(0) > 1 ? Hin.stride(0) : std::max<int64_t>(F, 1);
-  Tensor padded;
-  if (!h16 && (F % 4 != 0 || ldh % 4 != 0 || reinterpret_cast<uintptr_t>(H) % 16 != 0)) {
-    const int64_t f4 = (F + 3) / 4 * 4;
-    const int64_t last = (Hin.storage_offset() + (a.K - 1) * ldh + f4) * int64_t(sizeof(float));
-    if (a.K > 0 && ldh % 4 == 0 && ldh >= f4 && reinterpret_cast<uintptr_t>(H) % 16 == 0 &&
-        last <= int64_t(Hin.storage().nbytes())) {
-      epi |= GC_EPI_H_PADDED;  // a view of wider rows: what lies beyond the width may be read, and is not used
-    } else if (F > 8 && a.nnz >= 4 * a.K && a.nnz >= (F <= 32 ? 1 << 16 : F <= 64 ? 1 << 18 : F <= 256 ? 5 << 17 : 1 << 17)) {
-      // Rows that are not 16-byte aligned are gathered one float per lane.  Copying H to an aligned pitch first (8
-      // bytes per element, streamed) pays where every row is gathered several times: 169 K rows of 47, 15 non-zeros
-      // each, 136 us against 9 + 68.  On small graphs the copy's launch and the wider stores cost more than the scalar
-      // gathers at 65 to 256 columns (us, copied / as it is: 16.5 K rows, 96 K non-zeros F = 87 26 / 19, 468 K 35 / 31,
-      // 40 K rows, 840 K non-zeros 45 / 49) and, on smaller ones still, at 33 to 64 (F = 47: 19 / 16, 22 / 24, 34 / 40).
-      padded = empty_f32(a.K, f4, dev);
-      check(abi.gc_pad_rows_f32(static_cast<const float*>(H), ldh, padded.data_ptr<float>(), f4, a.K, F, stream_of(dev)),
-            "gc_pad_rows_f32");
-      H = padded.data_ptr();
-      ldh = f4;
-      epi |= GC_EPI_H_PADDED;
-    }
-  }
+  const int epi = (ep.relu ? GC_EPI_RELU : 0) | (accumulate ? GC_EPI_ACCUMULATE : 0);
   const int32_t* rp = a.rowptr.const_data_ptr<int32_t>();
   const int32_t* cp = a.col.const_data_ptr<int32_t>();
   const float* vp = a.val.const_data_ptr<float>();
   const void* pb = plan ? plan->buf.data_ptr() : nullptr;
   const int64_t np = plan ? plan->n_pieces : 0, ns = plan ? plan->n_slots : 0, nc = plan ? plan->n_cut : 0;
   void* st = stream_of(dev);
-  if (h16)
-    check(abi.gc_spmm_csr_bf16h_f32(rp, cp, vp, a.M, a.K, F, static_cast<const uint16_t*>(H), ldh, ep.bias, epi, Y,
-                                    ldy, ep.mask, ep.gate, pb, np, ns, nc, s.ptr, s.bytes, st),
+  const int64_t ldh = Hin.size(0) > 1 ? Hin.stride(0) : std::max<int64_t>(F, 1);
+  if (h16) {
+    check(abi.gc_spmm_csr_bf16h_f32(rp, cp, vp, a.M, a.K, F, static_cast<const uint16_t*>(Hin.data_ptr()), ldh, ep.bias,
+                                    epi, Y, ldy, ep.mask, ep.gate, pb, np, ns, nc, s.ptr, s.bytes, st),
           "gc_spmm_csr_f32");
-  else
-    check(abi.gc_spmm_csr_f32(rp, cp, vp, a.M, a.K, F, static_cast<const float*>(H), ldh, ep.bias, epi, Y, ldy,
-                              ep.mask, ep.gate, pb, np, ns, nc, s.ptr, s.bytes, st),
+    return;
+  }
+  // columns f0 .. f0 + n of Y from n columns at H
+  const auto columns = [&](const float* H, int64_t ld, int64_t f0, int64_t n, int flags) {
+    const auto at_f0 = [&](auto* p) { return p ? p + f0 : nullptr; };
+    check(abi.gc_spmm_csr_f32(rp, cp, vp, a.M, a.K, n, H, ld, at_f0(ep.bias), epi | flags, Y + f0, ldy, at_f0(ep.mask),
+                              at_f0(ep.gate), pb, np, ns, nc, s.ptr, s.bytes, st),
           "gc_spmm_csr_f32");
+  };
+  const float* H = Hin.const_data_ptr<float>();
+  const bool aligned = ldh % 4 == 0 && reinterpret_cast<uintptr_t>(H) % 16 == 0;
+  if (aligned && F % 4 == 0) return columns(H, ldh, 0, F, 0);
+  const int64_t f4 = (F + 3) / 4 * 4;
+  const int64_t last = (Hin.storage_offset() + (a.K - 1) * ldh + f4) * int64_t(sizeof(float));
+  if (aligned && a.K > 0 && ldh >= f4 && last <= int64_t(Hin.storage().nbytes()))
+    return columns(H, ldh, 0, F, GC_EPI_H_PADDED);  // a view of wider rows: what lies beyond the width may be read, and is not used
+  if (!copy_pays(F, a.K, a.nnz)) return columns(H, ldh, 0, F, 0);
+  const int64_t slabs = (a.K * f4 * int64_t(sizeof(float)) + kCopyBytes - 1) / kCopyBytes;
+  const int64_t width = ((f4 / 4 + slabs - 1) / slabs) * 4;
+  Tensor copy;
+  try {
+    copy = empty_f32(a.K, width, dev);
+  } catch (const c10::OutOfMemoryError&) {
+    return columns(H, ldh, 0, F, 0);
+  }
+  float* to = copy.data_ptr<float>();
+  for (int64_t f0 = 0; f0 < F; f0 += width) {
+    const int64_t n = std::min(width, F - f0);
+    check(abi.gc_pad_rows_f32(H + f0, ldh, to, width, a.K, n, st), "gc_pad_rows_f32");
+    columns(to, width, f0, n, GC_EPI_H_PADDED);
+  }
 }
 
 // ------------------------------------------------------------------ graphs
