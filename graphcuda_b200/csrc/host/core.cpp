@@ -263,13 +263,23 @@ void spmm_into(Adj& a, const Tensor& Hin, float* Y, int64_t ldy, const Epi& ep, 
   spmm_record_list().push_back(std::move(r));
 }
 
-// Whether H is copied to an aligned pitch first.  Rows that are not 16-byte aligned are gathered one float per lane; the
-// copy (8 bytes per element, streamed) pays where every row is gathered several times: 169 K rows of 47, 15 non-zeros each,
-// 136 us against 9 + 68.  On small graphs the copy's launch and the wider stores cost more than the scalar gathers at 65
-// to 256 columns (us, copied / as it is: 16.5 K rows, 96 K non-zeros F = 87 26 / 19, 468 K 35 / 31, 40 K rows, 840 K
-// non-zeros 45 / 49) and, on smaller ones still, at 33 to 64 (F = 47: 19 / 16, 22 / 24, 34 / 40).
+// Whether gathering from a copy of H on an aligned pitch beats gathering H as it lies (rows that are not 16-byte aligned:
+// one float per lane).  The copy costs 8 bytes per element, streamed, and scalar stores of Y stay; it pays where every row
+// is gathered often enough, later for wider rows (a scalar gather of a wide row is whole lines too) and, on few rows,
+// hardly where warps per piece serve scalar gathers as well.  Measured, time with the copy over time without, at rows /
+// non-zeros per row: up to 16 columns 0.75 at 3 K..10 K rows, 1.4 / 1.3 / 0.9 at 40 K / 6, 10, 40, 1.2 / 0.9 at 80 K / 4.5,
+// 10, 0.7 at 169 K; 17 to 32 0.4..0.9 throughout; 33 to 64 1.2 below 260 K non-zeros, 0.5..1.0 above; 65 to 208 1.2..1.5 on
+// 20 K rows, 0.8..0.95 on 40 K and more from 650 K non-zeros; 255 to 256 1.2 / 1.0 / 0.95 at 169 K / 4.5, 13, 20; wider
+// 0.7..1.0 on 6 K..20 K rows, and above at 6 / 10 / 13 / 20 per row 1.18 / 1.08 / 1.01 / 0.92 (F = 511, 169 K rows).
 static bool copy_pays(int64_t F, int64_t K, int64_t nnz) {
-  return F > 8 && nnz >= 4 * K && nnz >= (F <= 32 ? 1 << 16 : F <= 64 ? 1 << 18 : F <= 256 ? 5 << 17 : 1 << 17);
+  if (F <= 8 || nnz < 4 * K) return false;
+  const int64_t some = 1 << 16, many = 5 << 17;
+  if (F <= 16) return nnz >= some && (K <= 15000 || nnz >= 32 * K || (K > 75000 && nnz >= many));
+  if (F <= 32) return nnz >= some;
+  if (F <= 64) return nnz >= 4 * some;
+  const bool large = K > 30000;
+  if (F <= 256) return large && nnz >= many && (F <= 208 || nnz >= 12 * K);
+  return nnz >= 2 * some && (!large || nnz >= 12 * K);
 }
 
 // Largest such copy at a time; wider matrices take it in slabs of columns.
