@@ -112,6 +112,21 @@ int64_t padded_width(int64_t n_rows, int64_t in_dim, int64_t out_dim) {
   return (out_dim + 3) / 4 * 4;
 }
 
+// bf16 tier: whether the aggregation gathers a bf16 copy of H (half the bytes through the SM fill path, fp32 sums).  126 M
+// non-zeros, F = 256: 5.9 ms + 0.6 ms for the copy against 8.7 ms.  Sparser matrices do not repay the conversion pass, and
+// neither do small ones while fp32 has the mappings for few pieces that bf16 lacks (gc_spmm_csr_f32: up to 256 columns).
+// Measured, time of copy and product over time of the fp32 product, at 17 to 80 non-zeros per row:
+//   F = 128          2.6..1.4 to 20 K rows, 1.1..1.45 at 30 K, 0.9..1.5 at 40 K, 0.9..1.04 at 60 K, 0.8..1.05 above
+//   F = 136 to 256   2.2..1.15 to 170 K non-zeros, 1.1..1.0 at 220..330 K, 0.8..1.05 at 340..510 K, 0.7..1.03 above
+//   F = 264 to 384   1.25..1.0 to 820 K, 0.8..0.97 above
+//   F = 448 to 1024  0.6..0.97 (1.05 at worst: 640 columns on 1 K rows, 40 K rows at 17 per row)
+static bool bf16_gathers_pay(int64_t F, const Adj& a) {
+  if (F < 128 || F % 8 != 0 || a.nnz < 16 * a.K) return false;
+  if (F < 136) return a.M > 50000;
+  if (F <= 256) return a.nnz >= 3 << 17;
+  return F > 384 || a.nnz >= 13 << 16;
+}
+
 Tensor adj_matmul(Adj& a, Tensor H, int prec, const Epi& ep) {
   Tensor out = empty_f32(a.M, H.size(1), H.device());
   const int64_t F = H.size(1), ldy = std::max<int64_t>(F, 1);
@@ -129,10 +144,7 @@ Tensor adj_matmul(Adj& a, Tensor H, int prec, const Epi& ep) {
     return out;
   }
   if (H.stride(1) != 1 || (H.size(0) > 1 && H.stride(0) < F)) H = H.contiguous();
-  if (prec == GC_PREC_BF16 && F >= 128 && F % 8 == 0 && a.nnz >= 16 * H.size(0)) {
-    // bf16 tier, wide H on a graph with enough non-zeros per row: the aggregation gathers a bf16 copy (half the bytes
-    // through the SM fill path, fp32 sums).  126 M non-zeros, F = 256: 6.9 ms + 0.6 ms for the copy against 8.8 ms;
-    // narrower or sparser products do not repay the conversion pass.
+  if (prec == GC_PREC_BF16 && bf16_gathers_pay(F, a)) {
     spmm_into(a, to_bf16(H, false), out.data_ptr<float>(), ldy, ep, false, 0);
   } else {
     spmm_into(a, H, out.data_ptr<float>(), ldy, ep, false, 0);
