@@ -242,7 +242,9 @@ MPlan m_plan(int64_t M, int64_t N, int64_t K) {
   // Two CTAs per SM and not one more (299 of them for 296 places: 1433 x 16 x 2708 12.7 us, 276 10.6; 3703 x 16 x 3327
   // 26.8 and 22.3), at least 16 k-values per warp.
   int64_t s = std::min<int64_t>(std::max<int64_t>(1, 2 * gc::kNumSMs / tiles), std::max<int64_t>(1, K / 128));
-  pl.cluster = tiles == 1 && s > 1 && K <= 8192;
+  // One cluster covers the output: at most 8 CTAs, no second kernel (16 x 7, cluster / splits over more CTAs: K = 1024 3.9 /
+  // 4.8 us, 2048 4.9 / 5.2, 2708 5.9 / 5.9, 4096 6.7 / 4.9, 8192 10.3 / 5.4; 64 x 16 5.4 / 5.9 ... 15.4 / 6.5).
+  pl.cluster = tiles == 1 && s > 1 && K <= 2816;
   if (pl.cluster) s = s >= 8 ? 8 : s >= 4 ? 4 : 2;
   pl.splits = int(s);
   return pl;
@@ -291,11 +293,23 @@ int launch_k(const Args& p, cudaStream_t st) {
 
 namespace gc {
 
-// Up to 16 columns; k long enough that a warp's 32 lanes (or the splits) have work.  Tall products that are bound by
-// reading A (more rows than fill the GPU several times over) stay on the tiled kernel, which streams it.
+// Where these kernels take the place of the tiled one.  Measured as time here over time there, 2500 sizes (M 256 to 20 K, or
+// 7 to 16 K for the weight gradients, K 16 to 65 K, N 3 to 16), and as error against float64:
+//   lanes along k: 0.4..1.0 while the rows fit the GPU at once (2 CTAs of 16 rows per SM: 4736) and B is one chunk of
+//     k (1536; below K = 128 only with up to 8 columns, else up to 1.13), 1.0..1.5 at 5000 to 10,000 rows, 1.1..2.3 at
+//     12 K to 20 K and at K = 2048 and above.  B given N x K is staged 4 bytes at a time by every CTA: N <= 8 as above to
+//     K = 768, N = 16 to K = 512 and 1184 rows, 1.0..3.4 beyond.  Where the tiled kernel is the faster one its sums are the
+//     longer ones (8192 x 16 x 512: 2.1e-7 against 0.9e-7, 16,384 x 16 x 1433: 3.4e-7 against 1.1e-7): such products
+//     stay here.
+//   lanes along m: 0.67..1.1 to K = 128 (no splitting); 0.44..1.2 to 4096 rows, 1.0..1.9 above.  One tile of up to 64
+//     rows: 0.44..0.95 to K = 1536, 1.0..1.25 to 8192 except for 32 rows and 8 columns at most -- the tiled kernel is also
+//     the more exact one there (64 x 16 x 8192: 1.3e-7 against 2.2e-7) -- and 0.5..0.75 above.
 bool narrow_supported(bool ta, int64_t M, int64_t N, int64_t K) {
-  if (N > 16) return false;
-  return ta ? (M <= 8192 && K >= 64) : (M <= 16384 && K >= 128);
+  if (N > 16 || K < 16 || M > 16384) return false;
+  if (!ta) return K >= 128 || (N <= 8 && M <= 32 * kNumSMs);
+  if (K <= 128) return N <= 8 || K >= 64;
+  if (M <= 64 && (M > 32 || N > 8) && K > 1536 && K <= 8192) return false;
+  return M <= 8192;
 }
 
 size_t narrow_partial_bytes(bool ta, int64_t M, int64_t N, int64_t K) {
