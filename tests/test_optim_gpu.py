@@ -18,6 +18,21 @@ def _grads(step, device):
     return [torch.randn(*s, generator=g).to(device) for s in SHAPES]
 
 
+def _assert_close(what, got, ref, rtol, atol):
+    """allclose, with what a reader of a failure needs: where, how many, how far, and on what host the reference ran."""
+    got, ref = got.detach().cpu(), ref.detach().cpu()
+    if torch.allclose(got, ref, rtol=rtol, atol=atol):
+        return
+    over = ((got - ref).abs() - (atol + rtol * ref.abs())).flatten()
+    over[over.isnan()] = float("inf")
+    bad, i = over > 0, int(over.argmax())
+    raise AssertionError(
+        f"{what}, shape {tuple(ref.shape)}: {int(bad.sum())} of {ref.numel()} beyond rtol {rtol} atol {atol}, the first at "
+        f"{int(bad.nonzero()[0])}, the worst at {i}: {got.flatten()[i].item()!r} against {ref.flatten()[i].item()!r}; largest "
+        f"difference {(got - ref).abs().max().item():.3e}; host {torch.backends.cpu.get_cpu_capability()}, "
+        f"{torch.get_num_threads()} threads")
+
+
 @pytest.mark.parametrize("wd", [0.0, 0.05])
 def test_fused_adam_follows_torch_adam(cuda, wd):
     from graphcuda_b200 import FusedAdam
@@ -31,11 +46,12 @@ def test_fused_adam_follows_torch_adam(cuda, wd):
             q.grad = g.to(cuda)
         ref.step()
         ours.step()
+        for p, q in zip(ref_p, our_p):
+            at = f"weight decay {wd}, step {step + 1}"
+            _assert_close(f"weights, {at}", q, p, rtol=2e-6, atol=2e-7)
+            _assert_close(f"exp_avg, {at}", ours.state[q]["exp_avg"], ref.state[p]["exp_avg"], rtol=2e-6, atol=1e-6)
+            _assert_close(f"exp_avg_sq, {at}", ours.state[q]["exp_avg_sq"], ref.state[p]["exp_avg_sq"], rtol=1e-5, atol=1e-8)
     assert ours.steps_taken() == 6
-    for p, q in zip(ref_p, our_p):
-        assert torch.allclose(q.detach().cpu(), p.detach(), rtol=2e-6, atol=2e-7)
-        assert torch.allclose(ours.state[q]["exp_avg"].cpu(), ref.state[p]["exp_avg"], rtol=2e-6, atol=1e-6)
-        assert torch.allclose(ours.state[q]["exp_avg_sq"].cpu(), ref.state[p]["exp_avg_sq"], rtol=1e-5, atol=1e-8)
 
 
 def test_fused_adam_skips_parameters_without_gradient_and_many_tensors(cuda):
@@ -49,8 +65,8 @@ def test_fused_adam_skips_parameters_without_gradient_and_many_tensors(cuda):
             r.grad = torch.full((3,), 0.5 + i)
     ours.step()
     theirs.step()
-    for p, r in zip(ps, ref):
-        assert torch.allclose(p.detach().cpu(), r.detach(), rtol=2e-6, atol=1e-7)
+    for i, (p, r) in enumerate(zip(ps, ref)):
+        _assert_close(f"tensor {i} of 70, one step", p, r, rtol=2e-6, atol=1e-7)
 
 
 def test_fused_sgd_is_the_scripts_optimizer(cuda):
@@ -63,7 +79,7 @@ def test_fused_sgd_is_the_scripts_optimizer(cuda):
         ref.step()
         ours.step()
     for p, q in zip(ref_p, our_p):
-        assert torch.allclose(q.detach().cpu(), p.detach(), rtol=1e-6, atol=1e-6)
+        _assert_close("weights after 3 steps", q, p, rtol=1e-6, atol=1e-6)
 
 
 def test_rejects_cpu_parameters():
@@ -104,4 +120,4 @@ def test_graph_replay_with_fused_adam_matches_eager_torch_adam(cuda):
         opt_e.step()
     assert abs(loss_g.item() - loss_e.item()) < 1e-4 * max(1.0, abs(loss_e.item()))
     for a, b in zip(graphed.parameters(), eager.parameters()):
-        assert torch.allclose(a, b, rtol=1e-3, atol=1e-5)
+        _assert_close(f"weights after {warm} eager steps and {replays} replays", a, b, rtol=1e-3, atol=1e-5)
