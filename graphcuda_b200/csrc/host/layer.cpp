@@ -305,8 +305,13 @@ struct ConvFunction : torch::autograd::Function<ConvFunction> {
 //       bit 1 = X is the ReLU output of the layer below: gate dX by (X > 0) where it is produced
 Tensor conv(const Tensor& X, const AdjPtr& a, const Tensor& W, const OptTensor& bias, bool relu, int64_t prec,
             int64_t fuse) {
-  const bool record = c10::GradMode::is_enabled() &&
-                      (X.requires_grad() || W.requires_grad() || (bias && bias->defined() && bias->requires_grad()));
+  const bool has_bias = bias && bias->defined();
+  // A tangent goes to the autograd node too: it has no forward-mode rule and says so, where the plain call below would
+  // drop the tangent.
+  const auto dual = [](const Tensor& t) { return t._fw_grad(0).defined(); };
+  const bool record = (c10::GradMode::is_enabled() &&
+                       (X.requires_grad() || W.requires_grad() || (has_bias && bias->requires_grad()))) ||
+                      dual(X) || dual(W) || (has_bias && dual(*bias));
   if (!record) return layer_forward(X, *a, W, bias, relu, false, int(prec)).Y;
   return ConvFunction::apply(X, W, bias, a, (relu ? 1 : 0) | ((fuse & 3) << 1), prec);
 }
