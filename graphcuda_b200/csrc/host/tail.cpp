@@ -26,15 +26,16 @@ struct NllFunction : torch::autograd::Function<NllFunction> {
               labels.const_data_ptr<int64_t>(), masked ? static_cast<const uint8_t*>(mask8->data_ptr()) : nullptr, M, C,
               float(scale), loss.data_ptr<float>(), ws.data_ptr(), wsb, stream_of(dev)),
           "gc_logsoftmax_nll_forward_f32");
-    ctx->save_for_backward({Z, labels, ws, masked ? *mask8 : Tensor()});
+    ctx->save_for_backward({Z, labels, ws});
     ctx->saved_data["scale"] = scale;
+    ctx->saved_data["masked"] = masked;  // the backward pass reads the workspace's copy of the selection
     return loss;
   }
 
   static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
                                                  torch::autograd::variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &Z = saved[0], &labels = saved[1], &ws = saved[2], &mask8 = saved[3];
+    const Tensor &Z = saved[0], &labels = saved[1], &ws = saved[2];
     const int64_t M = Z.size(0), C = Z.size(1);
     const at::Device dev = Z.device();
     const c10::cuda::CUDAGuard guard(dev);
@@ -52,9 +53,11 @@ struct NllFunction : torch::autograd::Function<NllFunction> {
       dZ = empty_f32(M, C, dev);
     }
     const Tensor g = grads[0].to(at::kFloat).contiguous();
+    const uint8_t* mask = ctx->saved_data["masked"].toBool()
+                              ? static_cast<const uint8_t*>(ws.data_ptr()) + abi.gc_nll_workspace_bytes(M) - M
+                              : nullptr;
     check((lddz == C ? abi.gc_logsoftmax_nll_backward_f32 : abi.gc_logsoftmax_nll_backward_pad_f32)(
-              Z.const_data_ptr<float>(), ldz, labels.const_data_ptr<int64_t>(),
-              mask8.defined() ? static_cast<const uint8_t*>(mask8.data_ptr()) : nullptr, M, C,
+              Z.const_data_ptr<float>(), ldz, labels.const_data_ptr<int64_t>(), mask, M, C,
               float(ctx->saved_data["scale"].toDouble()), g.const_data_ptr<float>(), dZ.data_ptr<float>(), lddz,
               ws.data_ptr(), stream_of(dev)),
           "gc_logsoftmax_nll_backward_f32");

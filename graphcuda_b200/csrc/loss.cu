@@ -64,7 +64,7 @@ template <int G, int NV, bool VEC>
 __global__ void __launch_bounds__(256)
 lse_nll_forward_rows_kernel(const float* __restrict__ Z, int64_t ldz, const int64_t* __restrict__ labels,
                             const uint8_t* __restrict__ row_mask, int64_t M, int C, float* __restrict__ lse,
-                            float* __restrict__ partials) {
+                            uint8_t* __restrict__ mask_copy, float* __restrict__ partials) {
   constexpr int R = 32 / G, U = NV >= 3 ? 2 : 4;  // rows per warp pass, passes in flight
   const int lane = threadIdx.x % 32, lg = lane % G, sub = lane / G;
   const int64_t stride = int64_t(gridDim.x) * 8 * R;
@@ -72,6 +72,7 @@ lse_nll_forward_rows_kernel(const float* __restrict__ Z, int64_t ldz, const int6
   for (int64_t r0 = (int64_t(blockIdx.x) * 8 + threadIdx.x / 32) * R; r0 < M; r0 += stride * U) {  // uniform per warp
     float4 v[U][NV];
     int64_t y[U];
+    uint8_t chosen[U];
     bool counts[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -79,7 +80,8 @@ lse_nll_forward_rows_kernel(const float* __restrict__ Z, int64_t ldz, const int6
 #pragma unroll
       for (int k = 0; k < NV; ++k) v[u][k] = load_logits<VEC>(Z + r * ldz, (k * G + lg) * 4, C);
       y[u] = __ldg(labels + r);
-      counts[u] = r0 + u * stride + sub < M && (!row_mask || __ldg(row_mask + r)) && y[u] < C;
+      chosen[u] = row_mask ? __ldg(row_mask + r) : 1;
+      counts[u] = r0 + u * stride + sub < M && chosen[u] && y[u] < C;
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
@@ -92,7 +94,10 @@ lse_nll_forward_rows_kernel(const float* __restrict__ Z, int64_t ldz, const int6
         s += (expf(v[u][k].x - mx) + expf(v[u][k].y - mx)) + (expf(v[u][k].z - mx) + expf(v[u][k].w - mx));
       const float l = mx + logf(group_sum<G>(s));
       const int64_t r = r0 + u * stride + sub;
-      if (lg == 0 && r < M) lse[r] = l;
+      if (lg == 0 && r < M) {
+        lse[r] = l;
+        if (row_mask) mask_copy[r] = chosen[u];
+      }
 #pragma unroll
       for (int k = 0; k < NV; ++k) {  // the lane that holds the label's logit adds the row's loss
         const int64_t at = y[u] - (k * G + lg) * 4;
@@ -108,7 +113,7 @@ lse_nll_forward_rows_kernel(const float* __restrict__ Z, int64_t ldz, const int6
 __global__ void __launch_bounds__(256)
 lse_nll_forward_kernel(const float* __restrict__ Z, int64_t ldz, const int64_t* __restrict__ labels,
                        const uint8_t* __restrict__ row_mask, int64_t M, int C, float* __restrict__ lse,
-                       float* __restrict__ partials) {
+                       uint8_t* __restrict__ mask_copy, float* __restrict__ partials) {
   const int lane = threadIdx.x % 32;
   const int64_t stride = int64_t(gridDim.x) * 8;
   float acc = 0.f;
@@ -123,6 +128,7 @@ lse_nll_forward_kernel(const float* __restrict__ Z, int64_t ldz, const int64_t* 
     if (lane == 0) {
       const float l = mx + logf(s);
       lse[r] = l;
+      if (row_mask) mask_copy[r] = row_mask[r];
       if (!row_mask || row_mask[r]) {
         const int64_t y = labels[r];
         if (y >= 0 && y < C) acc += l - __ldg(z + y);
@@ -306,7 +312,7 @@ extern "C" {
 
 size_t gc_nll_workspace_bytes(int64_t M) {
   if (M < 0) return 0;
-  return size_t(kLossBlocks) * sizeof(float) + size_t(M) * sizeof(float);
+  return size_t(kLossBlocks) * sizeof(float) + size_t(M) * (sizeof(float) + 1);
 }
 
 int gc_logsoftmax_nll_forward_f32(const float* Z, int64_t ldz, const int64_t* labels, const uint8_t* row_mask,
@@ -321,21 +327,22 @@ int gc_logsoftmax_nll_forward_f32(const float* Z, int64_t ldz, const int64_t* la
   cudaStream_t st = gc::as_stream(stream);
   float* partials = static_cast<float*>(workspace);
   float* lse = partials + kLossBlocks;
+  uint8_t* copy = reinterpret_cast<uint8_t*>(lse + M);
   const int64_t rows_per_block = C <= 64 ? 64 : C <= 128 ? 32 : 8;
   const int blocks = int(std::max<int64_t>(1, std::min<int64_t>(gc::ceil_div(M, rows_per_block), kLossBlocks)));
   const bool vec = ldz % 4 == 0 && gc::aligned16(Z);
 #define GC_ROWS(G, NV)                                                                                            \
   (vec ? lse_nll_forward_rows_kernel<G, NV, true><<<blocks, 256, 0, st>>>(Z, ldz, labels, row_mask, M, int(C), lse, \
-                                                                         partials)                                \
+                                                                         copy, partials)                          \
        : lse_nll_forward_rows_kernel<G, NV, false><<<blocks, 256, 0, st>>>(Z, ldz, labels, row_mask, M, int(C), lse, \
-                                                                          partials))
+                                                                          copy, partials))
   if (M == 0) cudaMemsetAsync(partials, 0, sizeof(float) * size_t(blocks), st);
   else if (C <= 16) GC_ROWS(4, 1);
   else if (C <= 32) GC_ROWS(4, 2);
   else if (C <= 48) GC_ROWS(4, 3);
   else if (C <= 64) GC_ROWS(4, 4);
   else if (C <= 128) GC_ROWS(8, 4);
-  else lse_nll_forward_kernel<<<blocks, 256, 0, st>>>(Z, ldz, labels, row_mask, M, int(C), lse, partials);
+  else lse_nll_forward_kernel<<<blocks, 256, 0, st>>>(Z, ldz, labels, row_mask, M, int(C), lse, copy, partials);
 #undef GC_ROWS
   loss_reduce_kernel<<<1, 256, 0, st>>>(partials, blocks, scale, loss);
   return gc::check_launch("gc_logsoftmax_nll_forward_f32", 2);

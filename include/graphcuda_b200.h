@@ -365,7 +365,9 @@ int gc_transpose_f32(const float* in, int64_t ldin, float* out, int64_t ldout,
  * F.nll_loss on the masked rows as the reference's script computes them
  * (scale = 1 / number of selected rows gives reduction='mean').  The
  * workspace (gc_nll_workspace_bytes(M)) keeps the per-row logsumexp for the
- * backward call.  loss: one device float.
+ * backward call and, in its last M bytes, a copy of row_mask (not written when
+ * row_mask is null), so that the caller's selection may change before the
+ * backward call reads one.  loss: one device float.
  */
 size_t gc_nll_workspace_bytes(int64_t M);
 int gc_logsoftmax_nll_forward_f32(const float* Z, int64_t ldz, const int64_t* labels, const uint8_t* row_mask,
