@@ -233,12 +233,23 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     Forward f = layer_forward(X, *a, W, bias, relu, want_mask, int(prec));
     return std::make_tuple(f.Y, f.mask, f.inter);
   }, NoGil());
+  m.def("layer_backward", [](const Tensor& G, const Tensor& X, const AdjPtr& a, const Tensor& W, bool relu, const Tensor& Y,
+                             const OptTensor& inter, bool need_dX, bool need_dW, bool need_db, int64_t prec, int64_t fuse) {
+    const Grads g = layer_backward(G, X, *a, W, relu, Y, inter ? *inter : Tensor(), need_dX, need_dW, need_db, int(prec),
+                                   fuse & 1, fuse & 2);
+    return std::make_tuple(g.dX, g.dW, g.db);
+  }, NoGil());
   m.def("adj_matmul", [](const AdjPtr& a, const Tensor& H, int64_t prec) {
     require(H.dim() == 2 && H.size(0) == a->K, "A.cols must match B.rows");
     const c10::cuda::CUDAGuard guard(H.device());
     return adj_matmul(*a, H, int(prec), Epi{});
   }, NoGil());
   m.def("nll_loss", &nll_loss, NoGil());
+  m.def("nll_forward", [](const Tensor& Z, const Tensor& labels, const OptTensor& row_mask, double scale) {
+    const NllForward f = nll_forward(Z, labels, row_mask, scale);
+    return std::make_tuple(f.loss, f.Z, f.labels, f.ws, f.masked);
+  }, NoGil());
+  m.def("nll_backward", &nll_backward, NoGil());
   m.def("argmax_accuracy", &argmax_accuracy, NoGil());
   m.def("adam_step", &adam_step, NoGil());
   m.def("sgd_step", &sgd_step, NoGil());

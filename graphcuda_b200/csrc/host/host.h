@@ -163,6 +163,14 @@ void register_zero_padded(const Tensor& buf);
 OptTensor zero_padded_base(const Tensor& view, int64_t width);
 int64_t zero_padded_count();
 
+// The loss and what its backward pass needs: logits and labels as the kernels take them, and the workspace.
+struct NllForward {
+  Tensor loss, Z, labels, ws;
+  bool masked;
+};
+NllForward nll_forward(const Tensor& Z, const Tensor& labels, const OptTensor& row_mask, double scale);
+Tensor nll_backward(const Tensor& grad, const Tensor& Z, const Tensor& labels, const Tensor& ws, bool masked,
+                    double scale);
 Tensor nll_loss(const Tensor& Z, const Tensor& labels, const OptTensor& row_mask, double scale);
 std::pair<Tensor, Tensor> argmax_accuracy(const Tensor& logits, const OptTensor& labels,
                                           const std::optional<std::vector<Tensor>>& masks, bool want_pred);

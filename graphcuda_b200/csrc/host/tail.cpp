@@ -9,62 +9,6 @@
 namespace gch {
 
 namespace {
-struct NllFunction : torch::autograd::Function<NllFunction> {
-  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& Zin, const Tensor& labels_in,
-                        const OptTensor& mask8, double scale) {
-    const Tensor Z = Zin.stride(1) == 1 ? Zin : Zin.contiguous();
-    const Tensor labels = labels_in.contiguous();
-    const int64_t M = Z.size(0), C = Z.size(1);
-    const at::Device dev = Z.device();
-    const c10::cuda::CUDAGuard guard(dev);
-    const size_t wsb = std::max<size_t>(abi.gc_nll_workspace_bytes(M), 4);
-    Tensor ws = at::empty({int64_t(wsb)}, at::TensorOptions().dtype(at::kByte).device(dev));
-    Tensor loss = at::empty({}, at::TensorOptions().dtype(at::kFloat).device(dev));
-    const bool masked = mask8 && mask8->defined();
-    check(abi.gc_logsoftmax_nll_forward_f32(
-              Z.const_data_ptr<float>(), M > 1 ? Z.stride(0) : std::max<int64_t>(C, 1),
-              labels.const_data_ptr<int64_t>(), masked ? static_cast<const uint8_t*>(mask8->data_ptr()) : nullptr, M, C,
-              float(scale), loss.data_ptr<float>(), ws.data_ptr(), wsb, stream_of(dev)),
-          "gc_logsoftmax_nll_forward_f32");
-    ctx->save_for_backward({Z, labels, ws});
-    ctx->saved_data["scale"] = scale;
-    ctx->saved_data["masked"] = masked;  // the backward pass reads the workspace's copy of the selection
-    return loss;
-  }
-
-  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
-                                                 torch::autograd::variable_list grads) {
-    const auto saved = ctx->get_saved_variables();
-    const Tensor &Z = saved[0], &labels = saved[1], &ws = saved[2];
-    const int64_t M = Z.size(0), C = Z.size(1);
-    const at::Device dev = Z.device();
-    const c10::cuda::CUDAGuard guard(dev);
-    const int64_t ldz = M > 1 ? Z.stride(0) : std::max<int64_t>(C, 1);
-    int64_t lddz = std::max<int64_t>(C, 1);
-    Tensor dZ;
-    if (M > 1 && C < ldz && ldz <= C + 3 && ldz % 4 == 0 && reinterpret_cast<uintptr_t>(Z.data_ptr()) % 16 == 0) {
-      // The logits are a view of a matrix padded to 16-byte rows (an odd class count): give the gradient the same
-      // pitch with zero pad columns, so the layer below can aggregate it without re-padding a copy.
-      lddz = ldz;
-      Tensor buf = empty_f32(M, ldz, dev);
-      register_zero_padded(buf);
-      dZ = buf.narrow(1, 0, C);
-    } else {
-      dZ = empty_f32(M, C, dev);
-    }
-    const Tensor g = grads[0].to(at::kFloat).contiguous();
-    const uint8_t* mask = ctx->saved_data["masked"].toBool()
-                              ? static_cast<const uint8_t*>(ws.data_ptr()) + abi.gc_nll_workspace_bytes(M) - M
-                              : nullptr;
-    check((lddz == C ? abi.gc_logsoftmax_nll_backward_f32 : abi.gc_logsoftmax_nll_backward_pad_f32)(
-              Z.const_data_ptr<float>(), ldz, labels.const_data_ptr<int64_t>(), mask, M, C,
-              float(ctx->saved_data["scale"].toDouble()), g.const_data_ptr<float>(), dZ.data_ptr<float>(), lddz,
-              ws.data_ptr(), stream_of(dev)),
-          "gc_logsoftmax_nll_backward_f32");
-    return {dZ, Tensor(), Tensor(), Tensor()};
-  }
-};
-
 // One byte per row, non-zero where the row counts; bool and uint8 selections are used as they are.
 Tensor bytes_of(const Tensor& m) {
   if (m.scalar_type() == at::kBool || m.scalar_type() == at::kByte) return m.contiguous();
@@ -72,16 +16,86 @@ Tensor bytes_of(const Tensor& m) {
 }
 }  // namespace
 
-Tensor nll_loss(const Tensor& Z, const Tensor& labels, const OptTensor& row_mask, double scale) {
-  require(Z.dim() == 2 && Z.is_cuda() && Z.scalar_type() == at::kFloat, "logits must be a float32 CUDA matrix");
-  require(labels.is_cuda() && labels.scalar_type() == at::kLong && labels.numel() == Z.size(0),
+NllForward nll_forward(const Tensor& Zin, const Tensor& labels, const OptTensor& row_mask, double scale) {
+  require(Zin.dim() == 2 && Zin.is_cuda() && Zin.scalar_type() == at::kFloat, "logits must be a float32 CUDA matrix");
+  require(labels.is_cuda() && labels.scalar_type() == at::kLong && labels.numel() == Zin.size(0),
           "labels must be a CUDA int64 vector with one entry per row");
-  OptTensor mask8;
-  if (row_mask && row_mask->defined()) {
-    require(row_mask->is_cuda() && row_mask->numel() == Z.size(0), "row_mask must have one entry per row");
+  NllForward f;
+  f.masked = row_mask && row_mask->defined();
+  Tensor mask8;
+  if (f.masked) {
+    require(row_mask->is_cuda() && row_mask->numel() == Zin.size(0), "row_mask must have one entry per row");
     mask8 = bytes_of(*row_mask);
   }
-  return NllFunction::apply(Z, labels, mask8, scale);
+  f.Z = Zin.stride(1) == 1 ? Zin : Zin.contiguous();
+  f.labels = labels.contiguous();
+  const int64_t M = f.Z.size(0), C = f.Z.size(1);
+  const at::Device dev = f.Z.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const size_t wsb = std::max<size_t>(abi.gc_nll_workspace_bytes(M), 4);
+  f.ws = at::empty({int64_t(wsb)}, at::TensorOptions().dtype(at::kByte).device(dev));
+  f.loss = at::empty({}, at::TensorOptions().dtype(at::kFloat).device(dev));
+  check(abi.gc_logsoftmax_nll_forward_f32(
+            f.Z.const_data_ptr<float>(), M > 1 ? f.Z.stride(0) : std::max<int64_t>(C, 1),
+            f.labels.const_data_ptr<int64_t>(), f.masked ? static_cast<const uint8_t*>(mask8.data_ptr()) : nullptr, M, C,
+            float(scale), f.loss.data_ptr<float>(), f.ws.data_ptr(), wsb, stream_of(dev)),
+        "gc_logsoftmax_nll_forward_f32");
+  return f;
+}
+
+// masked: the rows are those of the forward pass's selection, of which the workspace holds a copy
+Tensor nll_backward(const Tensor& grad, const Tensor& Z, const Tensor& labels, const Tensor& ws, bool masked,
+                    double scale) {
+  const int64_t M = Z.size(0), C = Z.size(1);
+  const at::Device dev = Z.device();
+  const c10::cuda::CUDAGuard guard(dev);
+  const int64_t ldz = M > 1 ? Z.stride(0) : std::max<int64_t>(C, 1);
+  int64_t lddz = std::max<int64_t>(C, 1);
+  Tensor dZ;
+  if (M > 1 && C < ldz && ldz <= C + 3 && ldz % 4 == 0 && reinterpret_cast<uintptr_t>(Z.data_ptr()) % 16 == 0) {
+    // The logits are a view of a matrix padded to 16-byte rows (an odd class count): give the gradient the same
+    // pitch with zero pad columns, so the layer below can aggregate it without re-padding a copy.
+    lddz = ldz;
+    Tensor buf = empty_f32(M, ldz, dev);
+    register_zero_padded(buf);
+    dZ = buf.narrow(1, 0, C);
+  } else {
+    dZ = empty_f32(M, C, dev);
+  }
+  const Tensor g = grad.to(at::kFloat).contiguous();
+  const uint8_t* mask =
+      masked ? static_cast<const uint8_t*>(ws.data_ptr()) + abi.gc_nll_workspace_bytes(M) - M : nullptr;
+  check((lddz == C ? abi.gc_logsoftmax_nll_backward_f32 : abi.gc_logsoftmax_nll_backward_pad_f32)(
+            Z.const_data_ptr<float>(), ldz, labels.const_data_ptr<int64_t>(), mask, M, C, float(scale),
+            g.const_data_ptr<float>(), dZ.data_ptr<float>(), lddz, ws.data_ptr(), stream_of(dev)),
+        "gc_logsoftmax_nll_backward_f32");
+  return dZ;
+}
+
+namespace {
+struct NllFunction : torch::autograd::Function<NllFunction> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& Z, const Tensor& labels,
+                        const OptTensor& row_mask, double scale) {
+    const NllForward f = nll_forward(Z, labels, row_mask, scale);
+    ctx->save_for_backward({f.Z, f.labels, f.ws});
+    ctx->saved_data["scale"] = scale;
+    ctx->saved_data["masked"] = f.masked;
+    return f.loss;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx,
+                                                 torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    return {nll_backward(grads[0], saved[0], saved[1], saved[2], ctx->saved_data["masked"].toBool(),
+                         ctx->saved_data["scale"].toDouble()),
+            Tensor(), Tensor(), Tensor()};
+  }
+};
+
+}  // namespace
+
+Tensor nll_loss(const Tensor& Z, const Tensor& labels, const OptTensor& row_mask, double scale) {
+  return NllFunction::apply(Z, labels, row_mask, scale);
 }
 
 std::pair<Tensor, Tensor> argmax_accuracy(const Tensor& logits, const OptTensor& labels_in,

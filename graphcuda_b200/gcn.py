@@ -22,6 +22,26 @@ from .adjacency import as_adjacency, native_handle
 from .ops import _prec
 
 
+class _TracedConv(torch.autograd.Function):
+    """The layer inside torch.jit.trace: the trace records this call, where the native node would leave it the output as
+    fresh, uninitialised memory."""
+
+    @staticmethod
+    def forward(ctx, X, weights, bias, handle, relu, prec, fuse):
+        Y, _, inter = _lib.host.layer_forward(X, handle, weights, bias, relu, False, prec)
+        ctx.save_for_backward(X, weights, Y, inter)
+        ctx.call = handle, relu, prec, fuse, bias is not None
+        return Y
+
+    @staticmethod
+    def backward(ctx, grad_Y):
+        X, weights, Y, inter = ctx.saved_tensors
+        handle, relu, prec, fuse, has_bias = ctx.call
+        need = ctx.needs_input_grad
+        return _lib.host.layer_backward(grad_Y, X, handle, weights, relu, Y, inter, need[0], need[1],
+                                        has_bias and need[2], prec, fuse) + (None,) * 4
+
+
 class GCNConvFunction:
     """Y = relu((adjm @ X) @ weights [+ bias]) as one autograd node (csrc/host/layer.cpp).
 
@@ -35,6 +55,8 @@ class GCNConvFunction:
         #       bit 1 = X is the ReLU output of the layer below: gate dX by (X > 0) where it is produced
         prec = _prec(precision)
         h = native_handle(as_adjacency(adjm), prec, needs_symmetry=weights.size(1) < weights.size(0))
+        if torch.jit.is_tracing():
+            return _TracedConv.apply(X, weights, bias, h, bool(apply_relu), prec, int(fuse))
         return _lib.host.conv(X, h, weights, bias, bool(apply_relu), prec, int(fuse))
 
 

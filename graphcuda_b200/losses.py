@@ -9,6 +9,21 @@ import torch
 from . import _lib
 
 
+class _TracedLoss(torch.autograd.Function):
+    """The loss inside torch.jit.trace (see gcn._TracedConv)."""
+
+    @staticmethod
+    def forward(ctx, logits, labels, row_mask, scale):
+        loss, Z, labels, ws, masked = _lib.host.nll_forward(logits, labels, row_mask, scale)
+        ctx.save_for_backward(Z, labels, ws)
+        ctx.call = masked, scale
+        return loss
+
+    @staticmethod
+    def backward(ctx, grad_loss):
+        return _lib.host.nll_backward(grad_loss, *ctx.saved_tensors, *ctx.call), None, None, None
+
+
 def log_softmax_nll_loss(logits: torch.Tensor, labels: torch.Tensor, row_mask: Optional[torch.Tensor] = None,
                          scale: Optional[float] = None) -> torch.Tensor:
     """``F.nll_loss(torch.log_softmax(logits, 1)[row_mask], labels[row_mask])`` in one
@@ -19,6 +34,8 @@ def log_softmax_nll_loss(logits: torch.Tensor, labels: torch.Tensor, row_mask: O
     if scale is None:
         cnt = int(row_mask.sum().item()) if row_mask is not None else logits.size(0)
         scale = 1.0 / max(cnt, 1)
+    if torch.jit.is_tracing():
+        return _TracedLoss.apply(logits, labels, row_mask, scale)
     return _lib.host.nll_loss(logits, labels, row_mask, scale)
 
 
