@@ -35,6 +35,21 @@ class CSRAdjacency:
         self.perm = None  # set by normalized_adjacency(reorder=...): perm[new] = old vertex id
         self.inv_perm = None
 
+    def __getstate__(self):
+        """The arrays and what was chosen or found out; plans are built again on first use."""
+        return dict(rowptr=self.rowptr, col=self.col, val=self.val, shape=self.shape, symmetric=self._h.symmetric,
+                    use_plan=self.use_plan, segment=self.segment, perm=self.perm, inv_perm=self.inv_perm)
+
+    def __setstate__(self, s):
+        known = None if s["symmetric"] < 0 else bool(s["symmetric"])
+        self.__init__(s["rowptr"], s["col"], s["val"], s["shape"], symmetric=known, build_plan=s["use_plan"])
+        self.segment, self.perm, self.inv_perm = s["segment"], s["perm"], s["inv_perm"]
+
+    def __copy__(self):
+        other = object.__new__(type(self))  # the same native object, with its plans
+        other.__dict__.update(self.__dict__)
+        return other
+
     @property
     def use_plan(self) -> bool:
         return self._h.use_plan
@@ -143,6 +158,15 @@ class DenseAdjacency:
         self.A = A
         self.shape = tuple(A.shape)
         self.device = A.device
+
+    def __getstate__(self):
+        return dict(A=self.A, symmetric=self._h.symmetric)
+
+    def __setstate__(self, s):
+        self.__init__(s["A"], None if s["symmetric"] < 0 else bool(s["symmetric"]))
+
+    def __copy__(self):
+        return DenseAdjacency(self.A, None if self._h.symmetric < 0 else bool(self._h.symmetric))
 
     @property
     def symmetric(self) -> bool:
