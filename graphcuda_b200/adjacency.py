@@ -29,11 +29,35 @@ class CSRAdjacency:
         self.shape = (int(shape[0]), int(shape[1]))
         self._h = _lib.host.csr(rowptr, col, val, self.shape[0], self.shape[1],
                                 -1 if symmetric is None else int(bool(symmetric)), bool(build_plan))
-        self.rowptr, self.col, self.val = self._h.rowptr, self._h.col, self._h.val
         self.nnz = int(self._h.nnz)
         self.device = self.rowptr.device
         self.perm = None  # set by normalized_adjacency(reorder=...): perm[new] = old vertex id
         self.inv_perm = None
+
+    @property
+    def rowptr(self) -> torch.Tensor:
+        return self._h.rowptr
+
+    @property
+    def col(self) -> torch.Tensor:
+        return self._h.col
+
+    @property
+    def val(self) -> torch.Tensor:
+        return self._h.val
+
+    # New arrays in place of the old ones take effect at once; new values keep the plans.
+    @val.setter
+    def val(self, v: torch.Tensor) -> None:
+        self._h.set_val(v)
+
+    @rowptr.setter
+    def rowptr(self, v: torch.Tensor) -> None:
+        self.__setstate__(dict(self.__getstate__(), rowptr=v, symmetric=-1))
+
+    @col.setter
+    def col(self, v: torch.Tensor) -> None:
+        self.__setstate__(dict(self.__getstate__(), col=v, symmetric=-1))
 
     def __getstate__(self):
         """The arrays and what was chosen or found out; plans are built again on first use."""
@@ -155,9 +179,16 @@ class DenseAdjacency:
 
     def __init__(self, A: torch.Tensor, symmetric: Optional[bool] = None):
         self._h = _lib.host.dense(A, -1 if symmetric is None else int(bool(symmetric)))
-        self.A = A
         self.shape = tuple(A.shape)
         self.device = A.device
+
+    @property
+    def A(self) -> torch.Tensor:
+        return self._h.A
+
+    @A.setter
+    def A(self, A: torch.Tensor) -> None:
+        self.__init__(A)
 
     def __getstate__(self):
         return dict(A=self.A, symmetric=self._h.symmetric)

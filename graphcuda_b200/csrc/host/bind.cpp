@@ -171,6 +171,15 @@ AdjPtr make_csr(const Tensor& rowptr, const Tensor& col, const Tensor& val, int6
   return a;
 }
 
+// Other values on the same structure: the plans stay, the symmetry verdict does not.
+void set_val(Adj& a, const Tensor& val) {
+  require(!a.dense && val.is_cuda() && val.device() == a.device() && val.scalar_type() == at::kFloat &&
+              val.numel() == a.nnz,
+          "CSR values must be a float32 CUDA tensor with one entry per non-zero");
+  a.val = val.contiguous();
+  a.symmetric = -1;
+}
+
 AdjPtr make_dense(const Tensor& A, int symmetric) {
   require(A.dim() == 2 && A.is_cuda() && A.scalar_type() == at::kFloat,
           "dense adjacency must be a float32 CUDA matrix");
@@ -205,6 +214,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def_readonly("rowptr", &Adj::rowptr)
       .def_readonly("col", &Adj::col)
       .def_readonly("val", &Adj::val)
+      .def_readonly("A", &Adj::A)
+      .def("set_val", &set_val)
       .def_readonly("M", &Adj::M)
       .def_readonly("K", &Adj::K)
       .def_readonly("nnz", &Adj::nnz)
