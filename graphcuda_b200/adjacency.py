@@ -143,7 +143,8 @@ class CSRAdjacency:
         for i, b in enumerate(blocks):
             _require(b.size(0) >= min(block_rows, M - i * block_rows), "a block is shorter than its rows")
         if bias is not None:
-            _require(bias.is_cuda and bias.dtype == torch.float32 and bias.numel() == F, "bias must be float32 [F]")
+            _require(bias.device == self.device and bias.dtype == torch.float32 and bias.numel() == F,
+                     "bias must be float32 [F] on A's device")
             bias = bias.contiguous()
         if M == 0 or F == 0:
             return

@@ -27,9 +27,8 @@ py::object gemm(const Tensor& Ain, const Tensor& Bin, const OptTensor& bias_in, 
     const int64_t M = a.rows, N = b.cols, R = transposed_out ? N : M, Q = transposed_out ? M : N;
     if (out_in) {
       out = *out_in;
-      require(out.dim() == 2 && out.size(0) == R && out.size(1) == Q && out.scalar_type() == at::kFloat &&
-                  out.is_contiguous(),
-              "out has the wrong shape, dtype or layout");
+      require(f32_on(out, dev) && out.dim() == 2 && out.size(0) == R && out.size(1) == Q && out.is_contiguous(),
+              "out has the wrong shape, dtype, layout or device");
     } else {
       out = empty_f32(R, Q, dev);
     }
@@ -37,15 +36,13 @@ py::object gemm(const Tensor& Ain, const Tensor& Bin, const OptTensor& bias_in, 
     ep.relu = relu;
     Tensor bias;
     if (bias_in) {
-      require(bias_in->is_cuda() && bias_in->scalar_type() == at::kFloat && bias_in->numel() == N,
-              "bias must be float32 [N]");
+      require(f32_on(*bias_in, dev) && bias_in->numel() == N, "bias must be float32 [N] on the operands' device");
       bias = bias_in->contiguous();
       ep.bias = bias.const_data_ptr<float>();
     }
     if (gate) {
-      require(gate->is_cuda() && gate->scalar_type() == at::kFloat && gate->sizes() == out.sizes() &&
-                  gate->is_contiguous(),
-              "gate must be a contiguous float32 tensor of the result's shape");
+      require(f32_on(*gate, dev) && gate->sizes() == out.sizes() && gate->is_contiguous(),
+              "gate must be a contiguous float32 tensor of the result's shape, on its device");
       ep.gate = gate->const_data_ptr<float>();
     }
     if (want_mask) {
@@ -61,7 +58,8 @@ Tensor gemm_bf16(const Tensor& A16, const Tensor& Bt16, const OptTensor& bias_in
                  const OptTensor& gate) {
   require(A16.scalar_type() == at::kBFloat16 && Bt16.scalar_type() == at::kBFloat16 && A16.is_cuda() && Bt16.is_cuda(),
           "bf16 CUDA operands expected");
-  require(A16.size(1) == Bt16.size(1), "A16 and Bt16 must share K");
+  require(A16.dim() == 2 && Bt16.dim() == 2 && A16.size(1) == Bt16.size(1), "A16 and Bt16 must share K");
+  require(A16.device() == Bt16.device(), "Inputs must be on the same device");
   require(A16.stride(1) == 1 && Bt16.stride(1) == 1, "operands must have unit stride along K");
   const int64_t M = A16.size(0), N = Bt16.size(0);
   const at::Device dev = A16.device();
@@ -69,9 +67,8 @@ Tensor gemm_bf16(const Tensor& A16, const Tensor& Bt16, const OptTensor& bias_in
   Tensor out;
   if (out_in) {
     out = *out_in;
-    require(out.dim() == 2 && out.size(0) == M && out.size(1) == N && out.scalar_type() == at::kFloat &&
-                out.is_contiguous(),
-            "out has the wrong shape, dtype or layout");
+    require(f32_on(out, dev) && out.dim() == 2 && out.size(0) == M && out.size(1) == N && out.is_contiguous(),
+            "out has the wrong shape, dtype, layout or device");
   } else {
     out = empty_f32(M, N, dev);
   }
@@ -79,15 +76,13 @@ Tensor gemm_bf16(const Tensor& A16, const Tensor& Bt16, const OptTensor& bias_in
   ep.relu = relu;
   Tensor bias;
   if (bias_in) {
-    require(bias_in->is_cuda() && bias_in->scalar_type() == at::kFloat && bias_in->numel() == N,
-            "bias must be float32 [N]");
+    require(f32_on(*bias_in, dev) && bias_in->numel() == N, "bias must be float32 [N] on the operands' device");
     bias = bias_in->contiguous();
     ep.bias = bias.const_data_ptr<float>();
   }
   if (gate) {
-    require(gate->is_cuda() && gate->scalar_type() == at::kFloat && gate->sizes() == out.sizes() &&
-                gate->is_contiguous(),
-            "gate must be a contiguous float32 tensor of the result's shape");
+    require(f32_on(*gate, dev) && gate->sizes() == out.sizes() && gate->is_contiguous(),
+            "gate must be a contiguous float32 tensor of the result's shape, on its device");
     ep.gate = gate->const_data_ptr<float>();
   }
   gemm_bf16_into(A16, Bt16, static_cast<float*>(out.data_ptr()), N, ep, dev);
@@ -122,9 +117,9 @@ py::object spmm(const AdjPtr& adj, const Tensor& Hin, const OptTensor& bias_in, 
     else if (out_in) out = *out_in;
     else out = empty_f32(M, F, dev);
     // `out` may be a column slice of a wider row-major matrix (unit column stride)
-    require(out.dim() == 2 && out.size(0) == M && out.size(1) == F && out.scalar_type() == at::kFloat &&
-                out.stride(1) == 1 && (M <= 1 || out.stride(0) >= F),
-            "out has the wrong shape, dtype or layout");
+    require(f32_on(out, dev) && out.dim() == 2 && out.size(0) == M && out.size(1) == F && out.stride(1) == 1 &&
+                (M <= 1 || out.stride(0) >= F),
+            "out has the wrong shape, dtype, layout or device");
     const int64_t ldy = M > 1 ? out.stride(0) : std::max<int64_t>(F, 1);
     require(!want_mask || ldy == F, "a mask needs a contiguous output");
     Epi ep;
@@ -135,15 +130,13 @@ py::object spmm(const AdjPtr& adj, const Tensor& Hin, const OptTensor& bias_in, 
     }
     Tensor bias;
     if (bias_in) {
-      require(bias_in->is_cuda() && bias_in->scalar_type() == at::kFloat && bias_in->numel() == F,
-              "bias must be float32 [F]");
+      require(f32_on(*bias_in, dev) && bias_in->numel() == F, "bias must be float32 [F] on A's device");
       bias = bias_in->contiguous();
       ep.bias = bias.const_data_ptr<float>();
     }
     if (gate) {
-      require(gate->is_cuda() && gate->scalar_type() == at::kFloat && gate->sizes() == out.sizes() &&
-                  gate->is_contiguous() && ldy == F,
-              "gate must be a contiguous float32 tensor of Y's shape");
+      require(f32_on(*gate, dev) && gate->sizes() == out.sizes() && gate->is_contiguous() && ldy == F,
+              "gate must be a contiguous float32 tensor of Y's shape, on its device");
       ep.gate = gate->const_data_ptr<float>();
     }
     if (M != 0 && F != 0)
@@ -155,6 +148,7 @@ py::object spmm(const AdjPtr& adj, const Tensor& Hin, const OptTensor& bias_in, 
 AdjPtr make_csr(const Tensor& rowptr, const Tensor& col, const Tensor& val, int64_t M, int64_t K, int symmetric,
                 bool use_plan) {
   require(rowptr.is_cuda() && col.is_cuda() && val.is_cuda(), "CSR arrays must be CUDA tensors");
+  require(col.device() == rowptr.device() && val.device() == rowptr.device(), "CSR arrays must be on one device");
   require(rowptr.scalar_type() == at::kInt && col.scalar_type() == at::kInt, "rowptr/col must be int32");
   require(val.scalar_type() == at::kFloat, "CSR values must be float32");
   require(rowptr.numel() == M + 1, "rowptr must have M+1 entries");
@@ -252,6 +246,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   }, NoGil());
   m.def("adj_matmul", [](const AdjPtr& a, const Tensor& H, int64_t prec) {
     require(H.dim() == 2 && H.size(0) == a->K, "A.cols must match B.rows");
+    require(f32_on(H, a->device()), "B must be a float32 CUDA matrix on A's device");
     const c10::cuda::CUDAGuard guard(H.device());
     return adj_matmul(*a, H, int(prec), Epi{});
   }, NoGil());

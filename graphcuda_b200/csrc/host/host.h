@@ -31,6 +31,11 @@ inline void require(bool cond, const char* msg) {
   if (__builtin_expect(!cond, 0)) raise(msg);
 }
 
+// A float32 tensor whose memory a kernel on that device may be given (a host pointer would be a fault on the GPU).
+inline bool f32_on(const Tensor& t, const at::Device& dev) {
+  return t.device() == dev && t.scalar_type() == at::kFloat;
+}
+
 // ------------------------------------------------------------------ C ABI
 #define GC_HOST_FUNCTIONS(X)                                                                                        \
   X(gc_last_error) X(gc_status_string) X(gc_spmm_default_panel_cols) X(gc_spmm_segment)                     \

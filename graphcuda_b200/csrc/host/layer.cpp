@@ -162,7 +162,7 @@ Forward layer_forward(const Tensor& X, Adj& a, const Tensor& W, const OptTensor&
   ep.relu = relu;
   Tensor b;
   if (bias && bias->defined()) {
-    require(bias->is_cuda() && bias->scalar_type() == at::kFloat && bias->numel() == out_dim, "bias must be float32 [N]");
+    require(f32_on(*bias, X.device()) && bias->numel() == out_dim, "bias must be float32 [N] on the input's device");
     b = bias->contiguous();
     ep.bias = b.const_data_ptr<float>();
   }
@@ -194,7 +194,9 @@ Forward layer_forward(const Tensor& X, Adj& a, const Tensor& W, const OptTensor&
 }
 
 Tensor relu_backward(const Tensor& dYin, const Tensor& Yin) {
-  require(dYin.sizes() == Yin.sizes() && dYin.is_cuda() && Yin.is_cuda(), "relu_backward: shape/device mismatch");
+  require(dYin.dim() == 2 && dYin.sizes() == Yin.sizes() && dYin.is_cuda() && f32_on(dYin, Yin.device()) &&
+              f32_on(Yin, dYin.device()),
+          "relu_backward: two float32 CUDA matrices of one shape on one device expected");
   const Tensor dY = row_major(dYin), Y = row_major(Yin);
   const c10::cuda::CUDAGuard guard(dY.device());
   const int64_t M = dY.size(0), N = dY.size(1);
@@ -225,7 +227,9 @@ static Tensor bias_gradient(Tensor& G, const Tensor& Yin) {
 }
 
 Tensor mask_mul(const Tensor& dYin, const Tensor& maskin) {
-  require(dYin.sizes() == maskin.sizes() && dYin.is_cuda() && maskin.is_cuda(), "mask_mul: shape/device mismatch");
+  require(dYin.dim() == 2 && dYin.sizes() == maskin.sizes() && dYin.is_cuda() && f32_on(dYin, maskin.device()) &&
+              f32_on(maskin, dYin.device()),
+          "mask_mul: two float32 CUDA matrices of one shape on one device expected");
   const Tensor dY = row_major(dYin), mask = row_major(maskin);
   const c10::cuda::CUDAGuard guard(dY.device());
   const int64_t M = dY.size(0), N = dY.size(1);

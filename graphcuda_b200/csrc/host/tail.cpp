@@ -18,13 +18,14 @@ Tensor bytes_of(const Tensor& m) {
 
 NllForward nll_forward(const Tensor& Zin, const Tensor& labels, const OptTensor& row_mask, double scale) {
   require(Zin.dim() == 2 && Zin.is_cuda() && Zin.scalar_type() == at::kFloat, "logits must be a float32 CUDA matrix");
-  require(labels.is_cuda() && labels.scalar_type() == at::kLong && labels.numel() == Zin.size(0),
-          "labels must be a CUDA int64 vector with one entry per row");
+  require(labels.device() == Zin.device() && labels.scalar_type() == at::kLong && labels.numel() == Zin.size(0),
+          "labels must be a CUDA int64 vector with one entry per row, on the logits' device");
   NllForward f;
   f.masked = row_mask && row_mask->defined();
   Tensor mask8;
   if (f.masked) {
-    require(row_mask->is_cuda() && row_mask->numel() == Zin.size(0), "row_mask must have one entry per row");
+    require(row_mask->device() == Zin.device() && row_mask->numel() == Zin.size(0),
+            "row_mask must have one entry per row, on the logits' device");
     mask8 = bytes_of(*row_mask);
   }
   f.Z = Zin.stride(1) == 1 ? Zin : Zin.contiguous();
@@ -153,8 +154,9 @@ Lists lists(const std::vector<Tensor>& p, const std::vector<Tensor>& g) {
   for (size_t i = 0; i < p.size(); ++i) {
     require(p[i].is_cuda() && p[i].scalar_type() == at::kFloat && p[i].is_contiguous(),
             "fused optimizers need contiguous float32 CUDA parameters");
-    require(!g[i].is_sparse() && g[i].scalar_type() == at::kFloat && g[i].device() == p[i].device(),
+    require(!g[i].is_sparse() && f32_on(g[i], p[i].device()) && g[i].numel() == p[i].numel(),
             "fused optimizers need dense float32 gradients on the parameter's device");
+    require(p[i].device() == p[0].device(), "fused optimizers take the parameters of one device at a time");
     l.keep.push_back(g[i].contiguous());
     l.p.push_back(static_cast<float*>(p[i].data_ptr()));
     l.g.push_back(l.keep.back().const_data_ptr<float>());
@@ -168,7 +170,13 @@ void adam_step(const std::vector<Tensor>& p, const std::vector<Tensor>& g, const
                const std::vector<Tensor>& v, double lr, double b1, double b2, double eps, double wd,
                const Tensor& state) {
   Lists l = lists(p, g);
+  const auto moment = [](const Tensor& t, const Tensor& p) {
+    return f32_on(t, p.device()) && t.is_contiguous() && t.numel() == p.numel();
+  };
+  require(p.empty() || p[0].device() == state.device(), "the optimizer state must be on the parameters' device");
   for (size_t i = 0; i < p.size(); ++i) {
+    require(moment(m[i], p[i]) && moment(v[i], p[i]),
+            "FusedAdam: exp_avg and exp_avg_sq must be contiguous float32 tensors of the parameter's size on its device");
     l.m.push_back(static_cast<float*>(m[i].data_ptr()));
     l.v.push_back(static_cast<float*>(v[i].data_ptr()));
   }
