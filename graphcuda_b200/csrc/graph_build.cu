@@ -33,10 +33,16 @@ narrow_kernel(const int64_t* __restrict__ src, int32_t* __restrict__ dst, int64_
     dst[i] = int32_t(src[i]);
 }
 
+// A vertex number of an edge list; the lists come from the caller, and one that names a vertex outside the graph must not
+// be an access outside its arrays.
+__device__ __forceinline__ bool is_vertex(int64_t v, int64_t N) { return v >= 0 && v < N; }
+
 __global__ void __launch_bounds__(256)
-degree_kernel(const int64_t* __restrict__ col, int64_t E, int32_t* __restrict__ deg) {
-  for (int64_t e = int64_t(blockIdx.x) * 256 + threadIdx.x; e < E; e += int64_t(gridDim.x) * 256)
-    atomicAdd(deg + col[e], 1);  // integer counts: exact and order-independent
+degree_kernel(const int64_t* __restrict__ col, int64_t E, int64_t N, int32_t* __restrict__ deg) {
+  for (int64_t e = int64_t(blockIdx.x) * 256 + threadIdx.x; e < E; e += int64_t(gridDim.x) * 256) {
+    const int64_t c = col[e];
+    if (is_vertex(c, N)) atomicAdd(deg + c, 1);  // integer counts: exact and order-independent
+  }
 }
 
 __global__ void __launch_bounds__(256)
@@ -50,12 +56,17 @@ dinv_kernel(int32_t* __restrict__ deg_then_dinv, int64_t N) {
 }
 
 __global__ void __launch_bounds__(256)
-norm_weight_kernel(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E,
+norm_weight_kernel(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E, int64_t N,
                    const float* __restrict__ dinv, float* __restrict__ w) {
   for (int64_t e = int64_t(blockIdx.x) * 256 + threadIdx.x; e < E; e += int64_t(gridDim.x) * 256) {
+    const int64_t r = row[e], c = col[e];
+    if (!is_vertex(r, N) || !is_vertex(c, N)) {
+      w[e] = __int_as_float(0x7fffffff);
+      continue;
+    }
     // dinv[row] * 1.0f * dinv[col], left to right
-    const float a = __fmul_rn(dinv[row[e]], 1.0f);
-    w[e] = __fmul_rn(a, dinv[col[e]]);
+    const float a = __fmul_rn(dinv[r], 1.0f);
+    w[e] = __fmul_rn(a, dinv[c]);
   }
 }
 
@@ -115,12 +126,18 @@ csr_fill_kernel(const int64_t* __restrict__ row, const int64_t* __restrict__ col
 template <typename KEY>
 __global__ void __launch_bounds__(256)
 edge_key_kernel(const int64_t* __restrict__ row, const int64_t* __restrict__ col, int64_t E, int64_t N, int bits,
-                const int32_t* __restrict__ relabel, KEY* __restrict__ keys, int32_t* __restrict__ deg, int64_t total) {
+                const int32_t* __restrict__ relabel, KEY* __restrict__ keys, int32_t* __restrict__ deg,
+                int32_t* __restrict__ outside, int64_t total) {
   for (int64_t e = int64_t(blockIdx.x) * 256 + threadIdx.x; e < total; e += int64_t(gridDim.x) * 256) {
     int64_t r = e - E, c = r;  // beyond the edges: the self-loops
     if (e < E) {
       r = row[e];
       c = col[e];
+      if (!is_vertex(r, N) || !is_vertex(c, N)) {
+        *outside = 1;  // the caller discards the result
+        keys[e] = 0;
+        continue;
+      }
       if (relabel) {
         r = relabel[r];
         c = relabel[c];
@@ -253,19 +270,21 @@ int gc_gcn_norm_f32(const int64_t* row, const int64_t* col, int64_t E, int64_t N
   cudaError_t e = cudaMemsetAsync(deg_scratch, 0, size_t(N) * 4, st);
   if (e != cudaSuccess) return gc::fail(GC_ERR_CUDA, "gc_gcn_norm_f32: %s", cudaGetErrorString(e));
   int32_t* deg = reinterpret_cast<int32_t*>(deg_scratch);
-  degree_kernel<<<grid_for(E), 256, 0, st>>>(col, E, deg);
+  degree_kernel<<<grid_for(E), 256, 0, st>>>(col, E, N, deg);
   dinv_kernel<<<grid_for(N), 256, 0, st>>>(deg, N);
-  norm_weight_kernel<<<grid_for(E), 256, 0, st>>>(row, col, E, deg_scratch, w);
+  norm_weight_kernel<<<grid_for(E), 256, 0, st>>>(row, col, E, N, deg_scratch, w);
   return gc::check_launch("gc_gcn_norm_f32", 3);
 }
 
 }  // extern "C"
 
 namespace {
-// Workspace: [keys][keys, other buffer][running counts][degrees, then their -1/2 powers][temporary storage]
+// Workspace: [keys][keys, other buffer][running counts, the word for vertices outside the graph, degrees (then their -1/2
+// powers)][temporary storage].  The word lies between the last running count and the degrees: read with the one, cleared
+// with the others.
 struct EdgeWs {
   char *keys, *alt;
-  int32_t *incl, *deg;
+  int32_t *incl, *outside, *deg;
   void* cub;
   size_t cub_bytes, total;
 };
@@ -281,8 +300,11 @@ EdgeWs edge_ws(void* ws, int64_t total, int64_t N) {
   const size_t kb = (2 * id_bits(N) <= 32 ? 4 : 8) * size_t(std::max<int64_t>(total, 1));
   w.keys = take(kb);
   w.alt = take(kb);
-  w.incl = reinterpret_cast<int32_t*>(take(size_t(std::max<int64_t>(total, 1)) * 4));
-  w.deg = reinterpret_cast<int32_t*>(take(size_t(std::max<int64_t>(N, 1)) * 4));
+  w.incl = reinterpret_cast<int32_t*>(take(size_t(total + 1 + N) * 4));
+  if (p) {
+    w.outside = w.incl + total;
+    w.deg = w.outside + 1;
+  }
   w.cub_bytes = cub_bytes(total);
   w.cub = take(w.cub_bytes);
   w.total = off;
@@ -294,7 +316,7 @@ int sort_edges(const int64_t* row, const int64_t* col, int64_t E, int64_t N, int
                const EdgeWs& w, int* selector, cudaStream_t st) {
   const int bits = id_bits(N);
   KEY *k0 = reinterpret_cast<KEY*>(w.keys), *k1 = reinterpret_cast<KEY*>(w.alt);
-  edge_key_kernel<KEY><<<grid_for(total), 256, 0, st>>>(row, col, E, N, bits, relabel, k0, w.deg, total);
+  edge_key_kernel<KEY><<<grid_for(total), 256, 0, st>>>(row, col, E, N, bits, relabel, k0, w.deg, w.outside, total);
   dinv_kernel<<<grid_for(N), 256, 0, st>>>(w.deg, N);
   cub::DoubleBuffer<KEY> db(k0, k1);
   size_t need = 0;
@@ -331,7 +353,7 @@ int gc_edges_sort(const int64_t* row, const int64_t* col, int64_t E, int64_t N, 
   const EdgeWs w = edge_ws(workspace, total, N);
   if (workspace_bytes < w.total) return gc::fail(GC_ERR_WORKSPACE, "gc_edges_sort: workspace too small");
   cudaStream_t st = gc::as_stream(stream);
-  if (cudaMemsetAsync(w.deg, 0, size_t(N) * 4, st) != cudaSuccess)
+  if (cudaMemsetAsync(w.outside, 0, size_t(N + 1) * 4, st) != cudaSuccess)
     return gc::fail(GC_ERR_CUDA, "gc_edges_sort: clearing the degrees failed");
   *nnz_at = w.incl + total - 1;
   return 2 * id_bits(N) <= 32 ? sort_edges<uint32_t>(row, col, E, N, total, relabel, w, selector, st)
@@ -379,7 +401,7 @@ int gc_degree_order(const int64_t* target, int64_t E, int64_t N, int64_t* perm, 
   size_t have = cub_bytes(N), need = 0;
   if (cudaMemsetAsync(deg, 0, size_t(N) * 4, st) != cudaSuccess)
     return gc::fail(GC_ERR_CUDA, "gc_degree_order: clearing the degrees failed");
-  if (E > 0) degree_kernel<<<grid_for(E), 256, 0, st>>>(target, E, deg);
+  if (E > 0) degree_kernel<<<grid_for(E), 256, 0, st>>>(target, E, N, deg);
   degree_key_kernel<<<grid_for(N), 256, 0, st>>>(deg, dk.Current(), dv.Current(), N);
   cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, need, dk, dv, int(N), 0, 32, st);
   if (e == cudaSuccess && need > have)

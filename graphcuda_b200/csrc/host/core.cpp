@@ -376,7 +376,10 @@ std::tuple<Tensor, Tensor, Tensor> edges_to_csr(const Tensor& edge_index, int64_
         "gc_edges_sort");
   Tensor rowptr = at::empty({n + 1}, i32);
   const int64_t at = reinterpret_cast<const char*>(nnz_at) - static_cast<const char*>(ws.data_ptr());
-  const int64_t nnz = ws.narrow(0, at, 4).view(at::kInt).item<int32_t>();  // the one host read
+  const Tensor sizes = ws.narrow(0, at, 8).cpu();  // the one host read
+  const int64_t nnz = static_cast<const int32_t*>(sizes.data_ptr())[0];
+  require(static_cast<const int32_t*>(sizes.data_ptr())[1] == 0,
+          "edge_index names a vertex outside the graph (negative, or num_nodes and above)");
   Tensor c = at::empty({nnz}, i32), v = at::empty({nnz}, i32.dtype(at::kFloat));
   check(abi.gc_edges_to_csr(E, n, self_loops, selector, ws.data_ptr(), wsb, rowptr.data_ptr<int32_t>(),
                             c.data_ptr<int32_t>(), v.data_ptr<float>(), st),

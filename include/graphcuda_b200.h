@@ -443,7 +443,8 @@ int gc_narrow_i64_i32(const int64_t* src, int32_t* dst, int64_t n, void* stream)
  * (bit-identical to torch CPU pow(-0.5) and left-to-right multiplication),
  * inf -> 0 for isolated nodes.  Takes over torch_geometric's gcn_norm as
  * called at tests/gcn/graphcuda_impl.py:28.
- *   deg_scratch: N floats.  w: E floats out.
+ *   deg_scratch: N floats.  w: E floats out; NaN for an edge that names a
+ *   vertex outside [0, N), which counts towards no degree.
  */
 int gc_gcn_norm_f32(const int64_t* row, const int64_t* col, int64_t E, int64_t N,
                     float* deg_scratch, float* w, void* stream);
@@ -452,7 +453,8 @@ int gc_gcn_norm_f32(const int64_t* row, const int64_t* col, int64_t E, int64_t N
  * Edge list -> normalised CSR (tests/gcn/graphcuda_impl.py:27-38: add_self_loops, gcn_norm, coalesce) in two steps
  * around the one size that depends on the data.  gc_edges_sort sorts the edges (and the N self-loops, when asked for)
  * by (row, col) in the workspace, counts the degrees on the targets and leaves the number of distinct pairs at *nnz_at
- * (a device address inside the workspace); *selector is passed on.  relabel (or null): int32[N], vertex v becomes
+ * (a device address inside the workspace), followed by a word that is not 0 when an edge names a vertex outside [0, N):
+ * then there is no CSR to be had; *selector is passed on.  relabel (or null): int32[N], vertex v becomes
  * relabel[v].  gc_edges_to_csr then writes rowptr[N+1], col[nnz], val[nnz].  Same values, bit for bit, as
  * gc_gcn_norm_f32 on the list followed by coalescing.
  */
