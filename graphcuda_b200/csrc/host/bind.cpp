@@ -1,4 +1,5 @@
 // Python module of the native host side.
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include "host.h"
@@ -232,7 +233,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("register_zero_padded", &register_zero_padded);
   m.def("zero_padded_count", &zero_padded_count);
 
-  m.def("conv", &conv, NoGil());
+  // None while a trace is being taken: the caller then goes through an autograd function in Python, which it records.
+  m.def("conv", [](const Tensor& X, const AdjPtr& a, const Tensor& W, const OptTensor& bias, bool relu, int64_t prec,
+                   int64_t fuse) -> OptTensor {
+    if (torch::jit::tracer::isTracing()) return std::nullopt;
+    return conv(X, a, W, bias, relu, prec, fuse);
+  }, NoGil());
   m.def("layer_forward", [](const Tensor& X, const AdjPtr& a, const Tensor& W, const OptTensor& bias, bool relu,
                             bool want_mask, int64_t prec) {
     Forward f = layer_forward(X, *a, W, bias, relu, want_mask, int(prec));
@@ -250,7 +256,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     const c10::cuda::CUDAGuard guard(H.device());
     return adj_matmul(*a, H, int(prec), Epi{});
   }, NoGil());
-  m.def("nll_loss", &nll_loss, NoGil());
+  m.def("nll_loss", [](const Tensor& Z, const Tensor& labels, const OptTensor& row_mask, double scale) -> OptTensor {
+    if (torch::jit::tracer::isTracing()) return std::nullopt;
+    return nll_loss(Z, labels, row_mask, scale);
+  }, NoGil());
   m.def("nll_forward", [](const Tensor& Z, const Tensor& labels, const OptTensor& row_mask, double scale) {
     const NllForward f = nll_forward(Z, labels, row_mask, scale);
     return std::make_tuple(f.loss, f.Z, f.labels, f.ws, f.masked);

@@ -55,9 +55,8 @@ class GCNConvFunction:
         #       bit 1 = X is the ReLU output of the layer below: gate dX by (X > 0) where it is produced
         prec = _prec(precision)
         h = native_handle(as_adjacency(adjm), prec, needs_symmetry=weights.size(1) < weights.size(0))
-        if torch.jit.is_tracing():
-            return _TracedConv.apply(X, weights, bias, h, bool(apply_relu), prec, int(fuse))
-        return _lib.host.conv(X, h, weights, bias, bool(apply_relu), prec, int(fuse))
+        Y = _lib.host.conv(X, h, weights, bias, bool(apply_relu), prec, int(fuse))
+        return Y if Y is not None else _TracedConv.apply(X, weights, bias, h, bool(apply_relu), prec, int(fuse))
 
 
 class GCNConv(nn.Module):

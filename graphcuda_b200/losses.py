@@ -34,9 +34,8 @@ def log_softmax_nll_loss(logits: torch.Tensor, labels: torch.Tensor, row_mask: O
     if scale is None:
         cnt = int(row_mask.sum().item()) if row_mask is not None else logits.size(0)
         scale = 1.0 / max(cnt, 1)
-    if torch.jit.is_tracing():
-        return _TracedLoss.apply(logits, labels, row_mask, scale)
-    return _lib.host.nll_loss(logits, labels, row_mask, scale)
+    loss = _lib.host.nll_loss(logits, labels, row_mask, scale)
+    return loss if loss is not None else _TracedLoss.apply(logits, labels, row_mask, scale)
 
 
 def argmax_accuracy(logits: torch.Tensor, labels: Optional[torch.Tensor] = None, masks=None, *,
